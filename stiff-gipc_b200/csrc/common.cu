@@ -1,6 +1,8 @@
 // common.cu -- error state and the single-CTA exclusive scan used by the build stages.
 #include "common.cuh"
 
+#include <cooperative_groups.h>
+
 namespace stg
 {
 
@@ -9,16 +11,74 @@ static thread_local std::string g_error = "no error";
 void set_error(const std::string& msg) { g_error = msg; }
 const char* last_error() { return g_error.c_str(); }
 
-// Exclusive scan of n ints by one CTA of 1024 threads, 4 consecutive items per thread per
-// tile (16-byte loads are not assumed: `in` may be any offset).  n = n_host, or, when n_dev
-// is given, *n_dev (n_host >= 0) or ceil(*n_dev / -n_host) (n_host < 0: a bank count).
+// Exclusive scan.  A round scans 16 values per thread of 1,024 (16,384), read and written as
+// int4 when both arrays are 16-byte aligned.  One CTA takes 2.7 us for up to one round, then
+// about 3.6 us per round (latency of one SM: 30 us at 117,649 values); so more values than
+// SCAN_ONE go to one cluster of CL CTAs, each scanning a contiguous part: the parts' sums are
+// exchanged over distributed shared memory, and a part of one round keeps its values in
+// registers in between.
+constexpr int SCAN_PT = 16, SCAN_ROUND = SCAN_PT * 1024, SCAN_CL = 8, SCAN_ONE = SCAN_ROUND;
+
+__device__ __forceinline__ void scan_load(const int* in, int idx, int end, bool vec, int (&v)[SCAN_PT])
+{
+    if(vec && idx + SCAN_PT <= end)
+    {
+#pragma unroll
+        for(int q = 0; q < SCAN_PT / 4; q++)
+        {
+            const int4 t = reinterpret_cast<const int4*>(in + idx)[q];
+            v[4 * q] = t.x;
+            v[4 * q + 1] = t.y;
+            v[4 * q + 2] = t.z;
+            v[4 * q + 3] = t.w;
+        }
+    }
+    else
+    {
+#pragma unroll
+        for(int q = 0; q < SCAN_PT; q++) v[q] = idx + q < end ? in[idx + q] : 0;
+    }
+}
+
+// this thread's offset inside the round and the round's total (every thread gets it)
+__device__ __forceinline__ int scan_round(const int (&v)[SCAN_PT], int* warp_incl, int& total)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int local = 0;
+#pragma unroll
+    for(int q = 0; q < SCAN_PT; q++) local += v[q];
+    int x = local;
+#pragma unroll
+    for(int o = 1; o < 32; o <<= 1)
+    {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if(lane >= o) x += y;
+    }
+    if(lane == 31) warp_incl[warp] = x;
+    __syncthreads();
+    if(warp == 0)
+    {
+        int w = warp_incl[lane];
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            if(lane >= o) w += y;
+        }
+        warp_incl[lane] = w;
+    }
+    __syncthreads();
+    const int e = (warp > 0 ? warp_incl[warp - 1] : 0) + x - local;
+    total = warp_incl[31];
+    __syncthreads();
+    return e;
+}
+
+template <int CL>
 __global__ void __launch_bounds__(1024) k_scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int* total)
 {
-    // 16 values per thread per round (16,384 per round of the 1,024 threads), read and
-    // written as int4 when both arrays are 16-byte aligned
-    constexpr int PT = 16;
     __shared__ int warp_incl[32];
-    __shared__ int carry;
+    __shared__ int part_sum;
     int n = n_host;
     if(n_dev)
     {
@@ -26,79 +86,86 @@ __global__ void __launch_bounds__(1024) k_scan_exclusive(const int* in, int* out
         n = n_host < 0 ? (v + (-n_host) - 1) / (-n_host) : v;
     }
     const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if(threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for(int base = 0; base < n; base += PT * 1024)
+    // this CTA's part [b, e): a multiple of SCAN_PT values per CTA keeps the int4 alignment
+    const int len = CL == 1 ? n : ((n + CL - 1) / CL + SCAN_PT - 1) / SCAN_PT * SCAN_PT;
+    const int b = CL == 1 ? 0 : min(n, (int)blockIdx.x * len), e = CL == 1 ? n : min(n, b + len);
+    int v[SCAN_PT], off = 0, carry = 0, rt = 0;
+    if(CL > 1)
     {
-        const int idx = base + threadIdx.x * PT;
-        int v[PT];
-        if(vec && idx + PT <= n)
+        int sum = 0;
+        for(int base = b; base < e; base += SCAN_ROUND)
         {
-#pragma unroll
-            for(int q = 0; q < PT / 4; q++)
-            {
-                const int4 t = reinterpret_cast<const int4*>(in + idx)[q];
-                v[4 * q] = t.x;
-                v[4 * q + 1] = t.y;
-                v[4 * q + 2] = t.z;
-                v[4 * q + 3] = t.w;
-            }
+            scan_load(in, base + threadIdx.x * SCAN_PT, e, vec, v);
+            off = scan_round(v, warp_incl, rt);
+            sum += rt;
         }
-        else
+        if(threadIdx.x == 0) part_sum = sum;
+        auto cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        int all = 0;
+        for(int r = 0; r < CL; r++)
         {
-#pragma unroll
-            for(int q = 0; q < PT; q++) v[q] = idx + q < n ? in[idx + q] : 0;
+            const int x = *cluster.map_shared_rank(&part_sum, r);
+            if(r < (int)blockIdx.x) carry += x;
+            all += x;
         }
-        int local = 0;
-#pragma unroll
-        for(int q = 0; q < PT; q++) local += v[q];
-        int x = local;
-#pragma unroll
-        for(int o = 1; o < 32; o <<= 1)
+        cluster.sync();  // no CTA leaves while another reads its sum
+        if(blockIdx.x == 0 && threadIdx.x == 0 && total) *total = all;
+    }
+    const bool kept = CL > 1 && e - b <= SCAN_ROUND;  // values and offsets still in registers
+    for(int base = b; base < e; base += SCAN_ROUND)
+    {
+        const int idx = base + threadIdx.x * SCAN_PT;
+        if(!kept)
         {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if(lane >= o) x += y;
+            scan_load(in, idx, e, vec, v);
+            off = scan_round(v, warp_incl, rt);
         }
-        if(lane == 31) warp_incl[warp] = x;
-        __syncthreads();
-        if(warp == 0)
-        {
-            int w = warp_incl[lane];
+        int x = carry + off;
 #pragma unroll
-            for(int o = 1; o < 32; o <<= 1)
-            {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
-                if(lane >= o) w += y;
-            }
-            warp_incl[lane] = w;
-        }
-        __syncthreads();
-        int e = carry + (warp > 0 ? warp_incl[warp - 1] : 0) + x - local;
-#pragma unroll
-        for(int q = 0; q < PT; q++)
+        for(int q = 0; q < SCAN_PT; q++)
         {
             const int t = v[q];
-            v[q] = e;
-            e += t;
+            v[q] = x;
+            x += t;
         }
-        if(vec && idx + PT <= n)
+        if(vec && idx + SCAN_PT <= e)
         {
 #pragma unroll
-            for(int q = 0; q < PT / 4; q++)
+            for(int q = 0; q < SCAN_PT / 4; q++)
                 reinterpret_cast<int4*>(out + idx)[q] = make_int4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         }
         else
         {
 #pragma unroll
-            for(int q = 0; q < PT; q++)
-                if(idx + q < n) out[idx + q] = v[q];
+            for(int q = 0; q < SCAN_PT; q++)
+                if(idx + q < e) out[idx + q] = v[q];
         }
-        __syncthreads();
-        if(threadIdx.x == 0) carry += warp_incl[31];
-        __syncthreads();
+        carry += rt;
     }
-    if(threadIdx.x == 0 && total) *total = carry;
+    if(CL == 1 && threadIdx.x == 0 && total) *total = carry;
+}
+
+int scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int n_max, int* total, cudaStream_t s)
+{
+    if(n_max <= SCAN_ONE)
+    {
+        k_scan_exclusive<1><<<1, 1024, 0, s>>>(in, out, n_dev, n_host, total);
+        STG_LAUNCH_CHECK();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SCAN_CL);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = SCAN_CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    STG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_scan_exclusive<SCAN_CL>, in, out, n_dev, n_host, total));
+    return 0;
 }
 
 }  // namespace stg

@@ -174,8 +174,9 @@ __device__ __forceinline__ double block_sum(double v, double* smem /* BLOCK/32 *
     return r;
 }
 
-// Single-CTA exclusive scan of n ints (n read from n_dev if non-null, else n_host).
-// out[i] = sum in[0..i); *total = sum of all.  Launch with 1024 threads.
-__global__ void k_scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int* total);
+// Exclusive scan of n ints: out[i] = sum in[0..i), *total (when not null) = sum of all.
+// n = n_host, or, when n_dev is given, *n_dev (n_host >= 0) or ceil(*n_dev / -n_host)
+// (n_host < 0: a bank count); n <= n_max, which picks the launch.
+int scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int n_max, int* total, cudaStream_t s);
 
 }  // namespace stg

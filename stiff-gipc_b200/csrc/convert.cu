@@ -413,8 +413,7 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
     const int g = std::min(div_up(count, 256), kSMs * 16);
     k_conv_hist<<<g, 256, 0, s>>>(rows, cols, count, nrows, skip_negative, cv.row_cnt.data(), cv.scratch.data() + 2);
     STG_LAUNCH_CHECK();
-    k_scan_exclusive<<<1, 1024, 0, s>>>(cv.row_cnt.data(), cv.row_start.data(), nullptr, nrows + 1, cv.scratch.data());
-    STG_LAUNCH_CHECK();
+    STG_TRY(scan_exclusive(cv.row_cnt.data(), cv.row_start.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data(), s));
     k_conv_scatter<<<g, 256, 0, s>>>(rows, cols, count, nrows, cv.row_start.data(), cv.cursor.data(), cv.perm.data(),
                                      cv.pcol.data());
     STG_LAUNCH_CHECK();
@@ -428,8 +427,7 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
                                                         cv.long_rows.data(), cv.scratch.data() + 3);
     STG_LAUNCH_CHECK();
     STG_CUDA_TRY(cudaMemsetAsync(cv.uniq.data() + nrows, 0, sizeof(int), s));
-    k_scan_exclusive<<<1, 1024, 0, s>>>(cv.uniq.data(), row_ptr.data(), nullptr, nrows + 1, cv.scratch.data() + 1);
-    STG_LAUNCH_CHECK();
+    STG_TRY(scan_exclusive(cv.uniq.data(), row_ptr.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data() + 1, s));
     int h[2] = {0, 0};
     ConvFuse F;
     if(fuse)

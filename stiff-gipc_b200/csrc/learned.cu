@@ -223,7 +223,7 @@ int net_build_graph(cudaStream_t s, NetGraphStore& G, int n, int nnzu, const int
         STG_LAUNCH_CHECK();
         (*launches)++;
     }
-    k_scan_exclusive<<<1, 1024, 0, s>>>(G.cnt.data(), G.row.data(), nullptr, n, G.row.data() + n);
+    STG_TRY(scan_exclusive(G.cnt.data(), G.row.data(), nullptr, n, n, G.row.data() + n, s));
     STG_LAUNCH_CHECK();
     (*launches)++;
     int nnz = 0;

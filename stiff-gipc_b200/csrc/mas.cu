@@ -827,8 +827,7 @@ static int mas_build_t(Solver& S, const int* contacts, int ncp)
     }
     k_mas_l0_closure<B><<<gM, 256, 0, s>>>(m.part_map.data(), m.fine_mask.data(), m.prefix_orig.data(), M);
     STG_LAUNCH_CHECK();
-    k_scan_exclusive<<<1, 1024, 0, s>>>(m.prefix_orig.data(), m.prefix_sum_orig.data(), nullptr, m.nb0, m.scratch.data());
-    STG_LAUNCH_CHECK();
+    STG_TRY(scan_exclusive(m.prefix_orig.data(), m.prefix_sum_orig.data(), nullptr, m.nb0, m.nb0, m.scratch.data(), s));
     k_set_level1<<<1, 1, 0, s>>>(ls, m.scratch.data(), M);
     STG_LAUNCH_CHECK();
     k_mas_l1_assign<B><<<gM, 256, 0, s>>>(m.part_map.data(), m.fine_mask.data(), m.prefix_sum_orig.data(),
@@ -853,9 +852,8 @@ static int mas_build_t(Solver& S, const int* contacts, int ncp)
         k_mas_lx_closure<B><<<gN, 256, 0, s>>>(m.next_mask.data(), m.closed.data(), m.next_prefix.data(), ls, level);
         STG_LAUNCH_CHECK();
         // n = ceil(ls[2*level] / B) banks
-        k_scan_exclusive<<<1, 1024, 0, s>>>(m.next_prefix.data(), m.next_prefix_sum.data(), ls + 2 * level, -B,
-                                            ls + 2 * (level + 1));
-        STG_LAUNCH_CHECK();
+        STG_TRY(scan_exclusive(m.next_prefix.data(), m.next_prefix_sum.data(), ls + 2 * level, -B, V / B + 1,
+                               ls + 2 * (level + 1), s));
         k_mas_lx_assign<B><<<gN, 256, 0, s>>>(m.next_mask.data(), m.next_prefix_sum.data(), m.going_next.data(), ls, level);
         STG_LAUNCH_CHECK();
         k_mas_compute_next<<<gV, 256, 0, s>>>(m.coarse_tables.data(), m.next_mask.data(), level, V);

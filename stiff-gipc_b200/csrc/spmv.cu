@@ -178,8 +178,7 @@ int Solver::prepare_spmv()
     STG_CUDA_TRY(cudaMemsetAsync(bcoo.t_cnt.data(), 0, sizeof(int) * (nrows + 1), s));
     k_t_count<<<g, 256, 0, s>>>(bcoo.R(), bcoo.C(), nnzb, bcoo.t_cnt.data());
     STG_LAUNCH_CHECK();
-    k_scan_exclusive<<<1, 1024, 0, s>>>(bcoo.t_cnt.data(), bcoo.t_ptr.data(), nullptr, nrows + 1, cv.scratch.data() + 2);
-    STG_LAUNCH_CHECK();
+    STG_TRY(scan_exclusive(bcoo.t_cnt.data(), bcoo.t_ptr.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data() + 2, s));
     STG_CUDA_TRY(cudaMemsetAsync(bcoo.t_cnt.data(), 0, sizeof(int) * (nrows + 1), s));
     k_t_fill<<<g, 256, 0, s>>>(bcoo.R(), bcoo.C(), nnzb, bcoo.t_ptr.data(), bcoo.t_cnt.data(), bcoo.t_ent.data());
     STG_LAUNCH_CHECK();
@@ -372,8 +371,7 @@ int spmv_noalloc(double a, const double* blocks, const int* rows, const int* col
     STG_CUDA_TRY(cudaMemsetAsync(t_cnt, 0, sizeof(int) * (nrows + 1), s));
     k_t_count<<<g, 256, 0, s>>>(rows, cols, nnzb, t_cnt);
     STG_LAUNCH_CHECK();
-    k_scan_exclusive<<<1, 1024, 0, s>>>(t_cnt, t_ptr, nullptr, nrows + 1, counters + 1);
-    STG_LAUNCH_CHECK();
+    STG_TRY(scan_exclusive(t_cnt, t_ptr, nullptr, nrows + 1, nrows + 1, counters + 1, s));
     STG_CUDA_TRY(cudaMemsetAsync(t_cnt, 0, sizeof(int) * (nrows + 1), s));
     k_t_fill<<<g, 256, 0, s>>>(rows, cols, nnzb, t_ptr, t_cnt, t_ent);
     STG_LAUNCH_CHECK();

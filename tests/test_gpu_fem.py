@@ -48,3 +48,50 @@ def test_gpu_built_system_solves_like_cpu_built(dev):
         out.append((stt["iterations"], x.cpu().numpy()))
     assert abs(out[0][0] - out[1][0]) <= 1
     assert np.linalg.norm(out[0][1] - out[1][1]) <= 1e-6 * np.linalg.norm(out[1][1])
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 129, 300])
+def test_closed_form_projection_on_hard_tets(dev, T):
+    """The closed-form PSD projection against numpy's eigh, per tet: strongly compressed,
+    inverted, flattened, collapsed and rank-one deformations, a negative modulus, warps that are
+    not full, and one vertex shared by every tet (more incident tets than the shared-memory sort
+    holds).  Both projections are backward stable, so they agree to a few hundred eps of the
+    unprojected Hessian's norm in x (kinetic scale max d^2): 1e-12."""
+    from stgipc import fem, scenes
+    rng = np.random.default_rng(77 + T)
+    rest = rng.normal(size=(3 * T + 1, 3))
+    tets = np.stack([np.zeros(T, np.int64), 3 * np.arange(T) + 1, 3 * np.arange(T) + 2, 3 * np.arange(T) + 3], 1)
+    rest[0] = 0.0
+    Dm = np.transpose(rest[tets[:, 1:]], (0, 2, 1))
+    for t in range(T):  # well-shaped rest tets
+        q, _ = np.linalg.qr(Dm[t])
+        rest[tets[t, 1:]] = (q + 0.2 * rng.uniform(-1, 1, (3, 3))).T
+    F = np.eye(3) + rng.normal(scale=0.6, size=(T, 3, 3))
+    kind = np.arange(T) % 7
+    F[kind == 1] *= 0.05
+    F[kind == 2, :, 0] *= -1.0
+    F[kind == 3, :, 2] = F[kind == 3, :, 1]
+    F[kind == 4] = 0.0
+    F[kind == 5, :, 1:] = 2.0 * F[kind == 5, :, :1]
+    pos = rest.copy()
+    for t in range(T):
+        pos[tets[t, 1:]] = rest[tets[t, 1:]] @ F[t].T
+    E = np.exp(rng.uniform(np.log(1e3), np.log(1e6), T))
+    E[kind == 6] *= -1.0
+    st = dict(pos_rest=rest, pos=pos, vel=np.zeros_like(pos), tets=tets, E=E, nu=0.45, rho=1000.0, dt=0.01, barriers=[])
+    cpu = scenes._assemble(name="hard", **st)
+    rows, cols, blocks, b = fem.newton_system(rest, pos, st["vel"], tets, E, 0.45, 1000.0, 0.01, device=dev)
+    np.testing.assert_array_equal(rows.cpu().numpy(), cpu.rows)
+    np.testing.assert_array_equal(cols.cpu().numpy(), cpu.cols)
+    got = blocks.cpu().numpy()[:10 * T].reshape(T, 90)
+    ref = cpu.blocks[:10 * T].reshape(T, 90)
+    # scale: |H9| <= |mu| + |lam| |g|^2 + |lam (J - alpha)| |F|, times vol dt^2 |d|^2
+    Dm = np.transpose(rest[tets[:, 1:]] - rest[tets[:, :1]], (0, 2, 1))
+    Ff = np.transpose(pos[tets[:, 1:]] - pos[tets[:, :1]], (0, 2, 1)) @ np.linalg.inv(Dm)
+    mu, lam = np.abs(E) / 2.9, np.abs(E) * 0.45 / (1.45 * 0.1)
+    f = np.linalg.norm(Ff, axis=(1, 2))
+    h = mu + lam * f ** 4 + lam * (f ** 3 + 2.0) * f
+    d2 = (np.linalg.norm(np.linalg.inv(Dm), axis=(1, 2)) ** 2) * 4
+    scale = np.abs(np.linalg.det(Dm)) / 6.0 * 1e-4 * d2 * h
+    assert (np.abs(got - ref).max(axis=1) <= 1e-12 * scale).all()
+    np.testing.assert_allclose(b.cpu().numpy(), cpu.b, atol=1e-12 * T * np.abs(cpu.b).max())
