@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(256) k_mas_lx_closure(unsigned* next_mask, uns
 
 // _prefixSumLx (MASPreconditioner.cu:522-566): next-level ids; also records the level size.
 template <int B>
-__global__ void k_mas_lx_assign(unsigned* next_mask, const int* __restrict__ next_prefix_sum, int* going_next, int* ls,
-                                int level)
+__global__ void k_mas_lx_assign(unsigned* next_mask, const int* __restrict__ next_prefix_sum, int* going_next,
+                                int* lead_of, int* ls, int level)
 {
     const int number = ls[2 * level], begin = ls[2 * level + 1];
     const int rounded = (number + B - 1) / B * B;
@@ -269,6 +269,7 @@ __global__ void k_mas_lx_assign(unsigned* next_mask, const int* __restrict__ nex
     const int id = __popc(elected & lanemask_lt(lead)) + next_prefix_sum[i / B];
     next_mask[i] = (unsigned)id;
     going_next[begin + i] = id + begin + rounded;
+    if(leader) lead_of[id + begin + rounded] = begin + i;
 }
 
 // _computeNextLevel (MASPreconditioner.cu:568-579)
@@ -786,6 +787,7 @@ int Solver::mas_init(int V, int node_offset, const uint32_t* ns, const uint32_t*
     m.gn_size = pms + L * (V + B);  // >= total clusters: level l >= 1 holds <= V nodes, rounded to B
     STG_TRY(m.going_next.resize(m.gn_size));
     STG_TRY(m.closed.resize(m.gn_size));
+    STG_TRY(m.lead.resize(m.gn_size));
     STG_TRY(m.coarse_table.resize((size_t)V * std::max(L - 1, 1)));
     STG_TRY(m.level_size_d.resize(kMaxLevels + 2));
     STG_TRY(m.scratch.resize(kMaxLevels + 2));
@@ -796,6 +798,7 @@ int Solver::mas_init(int V, int node_offset, const uint32_t* ns, const uint32_t*
     STG_CUDA_TRY(cudaMemcpyAsync(m.real_map.data(), rm, sizeof(int) * V, cudaMemcpyHostToDevice, s));
     STG_CUDA_TRY(cudaMemsetAsync(m.going_next.data(), 0, sizeof(int) * m.gn_size, s));
     STG_CUDA_TRY(cudaMemsetAsync(m.closed.data(), 0, sizeof(unsigned) * m.gn_size, s));
+    STG_CUDA_TRY(cudaMemsetAsync(m.lead.data(), 0, sizeof(int) * m.gn_size, s));
     STG_CUDA_TRY(cudaStreamSynchronize(s));
     m.inited = true;
     m.built = m.assembled = false;
@@ -854,7 +857,8 @@ static int mas_build_t(Solver& S, const int* contacts, int ncp)
         // n = ceil(ls[2*level] / B) banks
         STG_TRY(scan_exclusive(m.next_prefix.data(), m.next_prefix_sum.data(), ls + 2 * level, -B, V / B + 1,
                                ls + 2 * (level + 1), s));
-        k_mas_lx_assign<B><<<gN, 256, 0, s>>>(m.next_mask.data(), m.next_prefix_sum.data(), m.going_next.data(), ls, level);
+        k_mas_lx_assign<B><<<gN, 256, 0, s>>>(m.next_mask.data(), m.next_prefix_sum.data(), m.going_next.data(),
+                                              m.lead.data(), ls, level);
         STG_LAUNCH_CHECK();
         k_mas_compute_next<<<gV, 256, 0, s>>>(m.coarse_tables.data(), m.next_mask.data(), level, V);
         STG_LAUNCH_CHECK();

@@ -42,7 +42,22 @@
 namespace stg
 {
 
-constexpr int PB = 256;  // threads per CTA in every PCG kernel
+constexpr int PB = 256;  // threads per CTA in the PCG kernels
+// phase B: 920 CTAs of 128 on the 352,947-DOF cube spread over the SMs within 13 % (460 of 256
+// threads left some SMs a third more than others)
+constexpr int PBB = 128;
+
+// Programmatic dependent launch.  The phases of an iteration are short (2 to 15 us) and form a
+// chain, so the idle time between two kernels (drain, launch, first loads) counts.  Every
+// phase is launched as a programmatic dependent of the one before it and releases its own
+// dependent at once: the next kernel's CTAs take the slots as they fall free, set up their
+// barriers and issue the loads and bulk copies of what no phase of the loop writes (matrix
+// planes, bank inverses, maps, masks).  grid_dep_wait() then returns when the phase before has
+// completed and its writes are visible; only after it may a kernel read what phases write, or
+// write anything.  Every CTA of every phase passes it, also when the solve is done, so that
+// the completion of one phase implies that of all phases before it.
+__device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 enum Site : int
 {
@@ -360,6 +375,10 @@ __device__ __forceinline__ T* zpbuf(const PcgDev& c, int parity)
 }
 // scalars are read with ld.global.cg: in the persistent kernel they change between phases
 __device__ __forceinline__ int iter_parity(const PcgDev& c) { return ((long)__ldcg(c.scal + SS_ITER)) & 1; }
+// the parity before this iteration's stop test (phases A, B) and after it (phase E): from the
+// launch when it knows it, which takes a dependent load (0.6 us) off the phase
+__device__ __forceinline__ int parity_before(const PcgDev& c) { return c.par >= 0 ? c.par : iter_parity(c); }
+__device__ __forceinline__ int parity_after(const PcgDev& c) { return c.par >= 0 ? c.par ^ 1 : iter_parity(c); }
 
 // A: q = A p_new, p_new = z + beta p_old; returns this thread's share of p_new . q
 template <typename T>
@@ -459,7 +478,7 @@ __device__ __forceinline__ void axpy_row(const PcgDev& c, const T* pn, const T* 
 
 // One level-0 slot of phase B (MAS): its row's p, q, x, r, closed mask and level-1 parent,
 // loaded before alpha is known (the loads do not depend on it), and after the upper SpMV the
-// bounds of its row's spilled products (loaded and added to q when the slot is updated)
+// bounds of its row's spilled products (added to q when the slot is updated)
 template <typename T>
 struct BSlot
 {
@@ -473,30 +492,38 @@ struct BSlot
 
 // SPILL: q may need the upper SpMV's spilled products (the persistent kernel never runs that
 // SpMV and compiles without the loop: with it, ptxas 12.9 for sm_100a aborts on that kernel)
+// b_load_maps: what the loop never writes (may run before grid_dep_wait); b_load_vecs: the rest
 template <typename T, bool SPILL = true>
-__device__ __forceinline__ void b_load(const PcgDev& c, const T* pn, const T* q, int s, BSlot<T>& L)
+__device__ __forceinline__ void b_load_maps(const PcgDev& c, int s, BSlot<T>& L)
 {
     L.v = c.identity ? (s < c.V ? s : -1) : (s < c.M ? c.part_map[s] : -1);
     if(L.v < 0) return;
-    const size_t row = (size_t)(c.fem_dof / 3) + L.v;
-    ld4(pn + 8 * row + 4, L.p[0], L.p[1], L.p[2]);
-    ld4(q + 4 * row, L.q[0], L.q[1], L.q[2]);
     if constexpr(SPILL)
     {
         if(c.spill)
         {
+            const size_t row = (size_t)(c.fem_dof / 3) + L.v;
             L.t0 = __ldg(c.t_ptr + row);
             L.t1 = __ldg(c.t_ptr + row + 1);
         }
     }
+    L.msk = c.fine_mask[L.v];
+    L.gnext = c.going_next[L.v];
+}
+
+template <typename T>
+__device__ __forceinline__ void b_load_vecs(const PcgDev& c, const T* pn, const T* q, BSlot<T>& L)
+{
+    if(L.v < 0) return;
+    const size_t row = (size_t)(c.fem_dof / 3) + L.v;
+    ld4(pn + 8 * row + 4, L.p[0], L.p[1], L.p[2]);
+    ld4(q + 4 * row, L.q[0], L.q[1], L.q[2]);
 #pragma unroll
     for(int d = 0; d < 3; d++)
     {
         L.x[d] = c.x[3 * row + d];
         L.r[d] = c.r[3 * row + d];
     }
-    L.msk = c.fine_mask[L.v];
-    L.gnext = c.going_next[L.v];
 }
 
 // x_i += alpha p_i, r_i -= alpha q_i of the slot, the level-0 residual slot and the level-0 ->
@@ -568,7 +595,7 @@ template <typename T, int B, bool SPILL = true>
 __device__ __forceinline__ double phase_b_mas(const PcgDev& c, int gt, int gn, double alpha, BSlot<T>& first,
                                               bool have_first, const T* st = nullptr, int slo = 0, int shi = 0)
 {
-    const T* pn = zpbuf<T>(c, iter_parity(c) ^ 1);
+    const T* pn = zpbuf<T>(c, parity_before(c) ^ 1);
     const T* q = reinterpret_cast<const T*>(c.q);
     double acc = 0;
     const int span = (c.M + 31) / 32 * 32;
@@ -581,7 +608,8 @@ __device__ __forceinline__ double phase_b_mas(const PcgDev& c, int gt, int gn, d
     for(; s < span; s += gn)
     {
         BSlot<T> L;
-        b_load<T, SPILL>(c, pn, q, s, L);
+        b_load_maps<T, SPILL>(c, s, L);
+        b_load_vecs<T>(c, pn, q, L);
         acc += b_update<T, B>(c, L, s, alpha);
     }
     for(int i = gt; i < c.abd_bodies * 4; i += gn)
@@ -596,7 +624,7 @@ __device__ __forceinline__ double phase_b_mas(const PcgDev& c, int gt, int gn, d
 template <typename T>
 __device__ __forceinline__ double phase_b_plain(const PcgDev& c, int gt, int gn, double alpha)
 {
-    const T* pn = zpbuf<T>(c, iter_parity(c) ^ 1);
+    const T* pn = zpbuf<T>(c, parity_before(c) ^ 1);
     const T* q = reinterpret_cast<const T*>(c.q);
     double acc = 0;
     for(int i = gt; i < c.nrows; i += gn)
@@ -860,6 +888,19 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
 // waits for phase `parity` of the mbarrier; false when the bounded wait gave up (WAIT_NS of
 // the global timer, read every 256 polls)
 __device__ __noinline__ bool mbar_wait_slow(unsigned bar, unsigned parity);
@@ -916,6 +957,8 @@ __device__ __forceinline__ void d16_issue(const PcgDev& c, char* stage, unsigned
 // Banks [b0, b1).  guarded: only on residual-replacement iterations (host loop).
 __global__ void __launch_bounds__(D_WARPS * 32) k_phase_d16(PcgDev c, int b0, int b1, int guarded)
 {
+    grid_dep_release();
+    grid_dep_wait();
     // the stop flag (and the replacement test) are loaded with the first bank's copy in
     // flight, not before it: their latency overlaps the copy's
     const int done = __ldcg(c.flags + F_DONE);
@@ -997,6 +1040,243 @@ __global__ void __launch_bounds__(D_WARPS * 32) k_phase_d16(PcgDev c, int b0, in
         bank16_join(z0, z1, z2);
         if(h == 0) st4(c.Z + ((size_t)bk * 16 + a) * 4, z0, z1, z2);
         __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// C and D in one launch (16-vertex banks): cluster 0 restricts the levels >= 2 and then solves
+// their banks, while the other clusters solve the banks of levels 0 and 1, which need only what
+// phase B left.  Separate launches put both restrictions (2.5 + 6.5 us on the 352,947-DOF
+// cube) in front of the solves; here they run beside the 98 % of the banks that do not wait
+// for them.  The restriction is a gather (one thread per coarse node, its members' loads all in
+// flight) that forms two levels at a time, so levels 2 to 5 take one cluster barrier and one
+// CTA barrier; level by level with a barrier each it took 14.8 us.  Sums, their order and the
+// bank arithmetic are those of restrict_level and k_phase_d16.  With `check`, the last cluster finishes phase
+// B's r.r and the stop test (the order of finish_reduction).
+//
+// Both stages' inverses are on their way before grid_dep_wait; the residual slots follow it.
+// F_STOP, not F_DONE, skips a finished solve: F_DONE may be written while this kernel runs, and
+// the CTAs of cluster 0 must all take the same barriers.
+// ---------------------------------------------------------------------------------------
+constexpr int CD_CL = 16;  // CTAs per cluster: 60 warps for the 87 banks of levels 2 and 3
+constexpr int CD_MAX_N1 = 16384;  // level-1 nodes one cluster restricts beside the bank solves
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A coarse node's members: its first member's bank and closed mask (never written by the loop)
+struct Members
+{
+    int bank = 0;
+    unsigned mask = 0u;
+};
+__device__ __forceinline__ Members members_of(const PcgDev& c, int node)
+{
+    Members m;
+    const int first = __ldg(c.lead + node);
+    m.bank = first & ~15;
+    m.mask = __ldg(c.closed + first);
+    return m;
+}
+
+// Residuals of the nodes of level l (threads gt, gt + gn, ...: each sums its members of level
+// l - 1 in lane order, all loads in flight) and, when there is one, of level l + 1 (a bank's
+// sums meet in its 16 lanes, as phase B forms level 1).  `mine`: the members of node gt.
+__device__ __forceinline__ void restrict_two(const PcgDev& c, int l, int gt, int gn, Members mine)
+{
+    const int number = __ldg(c.ls_dev + 2 * l), begin = __ldg(c.ls_dev + 2 * l + 1);
+    const int span = (number + 31) / 32 * 32;
+    const float4* R4 = reinterpret_cast<const float4*>(c.R);
+    for(int i = gt; i < span; i += gn)
+    {
+        const bool valid = i < number;
+        if(i != gt) mine = valid ? members_of(c, begin + i) : Members();
+        unsigned msk = 0u;
+        int g = 0;
+        if(valid && l + 1 < c.L)
+        {
+            msk = __ldg(c.closed + begin + i);
+            g = __ldg(c.going_next + begin + i);
+        }
+        float4 r[16];
+#pragma unroll
+        for(int b = 0; b < 16; b++)
+            if((mine.mask >> b) & 1u) r[b] = __ldcg(R4 + mine.bank + b);
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for(int b = 0; b < 16; b++)
+            if((mine.mask >> b) & 1u)
+            {
+                s0 += r[b].x;
+                s1 += r[b].y;
+                s2 += r[b].z;
+            }
+        if(valid) st4(c.R + 4 * (size_t)(begin + i), s0, s1, s2);
+        if(l + 1 >= c.L) continue;
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+#pragma unroll 4
+        for(int b = 0; b < 16; b++)
+        {
+            const float x0 = group_shfl<16>(s0, b), x1 = group_shfl<16>(s1, b), x2 = group_shfl<16>(s2, b);
+            if(msk & (1u << b))
+            {
+                a0 += x0;
+                a1 += x1;
+                a2 += x2;
+            }
+        }
+        if(valid && __popc(msk & lanemask_lt(i % 16)) == 0) st4(c.R + 4 * (size_t)g, a0, a1, a2);
+    }
+}
+
+// bank bk's inverse into a stage; the barrier expects it plus `extra` bytes
+__device__ __forceinline__ void cd_issue_inv(const PcgDev& c, char* stage, unsigned bar, int bk, int extra)
+{
+    mbar_expect_tx(bar, (unsigned)(D_PBYTES + extra));
+    tma_load_1d_hint(stage, c.inv + (size_t)bk * 136 * 9, D_PBYTES, bar, l2_evict_last());
+}
+__device__ __forceinline__ void cd_issue_res(const PcgDev& c, char* stage, unsigned bar, int bk)
+{
+    tma_load_1d_hint(stage + D_PBYTES, c.R + (size_t)bk * 16 * 4, D_RBYTES, bar, l2_evict_last());
+}
+
+__global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine, int check, int grid_b)
+{
+    grid_dep_release();
+    extern __shared__ __align__(128) char dsm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cl = blockIdx.x / CD_CL, rank = blockIdx.x % CD_CL;
+    const int fine_ctas = gridDim.x - CD_CL * (1 + check);
+    const bool coarse = cl == 0, checker = check && cl == (int)gridDim.x / CD_CL - 1;
+    const bool top = c.L > 4;  // levels 4 and 5: the banks of CTA 0 of the coarse cluster
+    const int bank4 = top ? c.ls[9] / 16 : c.nbanks;
+    // this warp's banks: first, stride, end
+    int bk0, step, bend;
+    if(!coarse)
+        bk0 = ((int)blockIdx.x - CD_CL) * D_WARPS + warp, step = fine_ctas * D_WARPS, bend = checker ? 0 : fine;
+    else if(top && rank == 0)
+        bk0 = bank4 + warp, step = D_WARPS, bend = c.nbanks;
+    else
+        bk0 = fine + (rank - (top ? 1 : 0)) * D_WARPS + warp, step = (CD_CL - (top ? 1 : 0)) * D_WARPS, bend = bank4;
+    const int extra = coarse ? 0 : D_RBYTES;
+    Members mem2, mem4;
+    if(coarse)
+    {
+        const int i2 = rank * D_WARPS * 32 + threadIdx.x;
+        if(i2 < c.ls[4]) mem2 = members_of(c, c.ls[5] + i2);
+        if(top && rank == 0 && (int)threadIdx.x < c.ls[8]) mem4 = members_of(c, c.ls[9] + threadIdx.x);
+    }
+    char* const base = dsm + (size_t)warp * D_WARP_BYTES;
+    const unsigned bar0 = smem_u32(base + 2 * D_BUF);
+    if(lane == 0)
+    {
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if(bk0 < bend) cd_issue_inv(c, base, bar0, bk0, extra);
+        if(bk0 + step < bend) cd_issue_inv(c, base + D_BUF, bar0 + 8, bk0 + step, extra);
+    }
+    __syncwarp();
+    const int a = lane & 15, h = lane >> 4;
+    int koff[8], rcol[8];
+    unsigned tmask = 0u;
+#pragma unroll
+    for(int j = 0; j < 8; j++)
+    {
+        const int cc = 8 * h + ((j + a) & 7);
+        const int lo = min(a, cc), hi = max(a, cc);
+        koff[j] = 9 * (lo * 16 - lo * (lo - 1) / 2 + (hi - lo));
+        rcol[j] = 4 * cc;
+        if(cc < a) tmask |= 1u << j;
+    }
+    grid_dep_wait();
+    const int stop = __ldcg(c.flags + F_STOP);
+    if(checker)
+    {
+        if(rank != 0 || stop) return;
+        static_assert(PBB == D_WARPS * 32, "the checker sums as phase B's finish_reduction does");
+        __shared__ double red[PBB / 32];
+        const double tot = block_sum<PBB>(strided_sum<PBB>(c.partials + (size_t)SITE_B * c.slots, grid_b), red);
+        if(threadIdx.x == 0 && !__ldcg(c.flags + F_DONE))
+        {
+            post_op(POST_CHECK_PQ, 0, tot, c.scal, c.flags, c.prm, __ldcg(c.scal + SS_PQ_B), __ldcg(c.scal + SS_RZ_B));
+            set_conditionals(c, POST_CHECK);
+        }
+        return;
+    }
+    if(!coarse && lane == 0)
+    {
+        if(bk0 < bend) cd_issue_res(c, base, bar0, bk0);
+        if(bk0 + step < bend) cd_issue_res(c, base + D_BUF, bar0 + 8, bk0 + step);
+    }
+    if(stop)
+    {
+        // nothing to solve: let the copies land before the warp's shared memory goes
+        if(lane == 0)
+        {
+            if(bk0 < bend) mbar_wait(bar0, 0u);
+            if(bk0 + step < bend) mbar_wait(bar0 + 8, 0u);
+        }
+        return;
+    }
+    if(coarse)
+    {
+        // levels 2 and 3 by the cluster, then 4 and 5 by its first CTA, which solves their banks
+        restrict_two(c, 2, rank * D_WARPS * 32 + threadIdx.x, CD_CL * D_WARPS * 32, mem2);
+        cluster_barrier();
+        if(top && rank == 0)
+        {
+            restrict_two(c, 4, threadIdx.x, D_WARPS * 32, mem4);
+            __syncthreads();
+        }
+    }
+    const float4* R4 = reinterpret_cast<const float4*>(c.R);
+    float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if(coarse && lane < 16 && bk0 < bend) rv = __ldcg(R4 + (size_t)bk0 * 16 + lane);
+    unsigned it = 0;
+    for(int bk = bk0; bk < bend; bk += step, it++)
+    {
+        char* const cur = base + (it & 1u) * D_BUF;
+        const unsigned bcur = bar0 + 8 * (it & 1u);
+        if(coarse)
+        {
+            // levels >= 2 were written by this kernel: read with plain loads, one bank ahead
+            if(lane < 16) reinterpret_cast<float4*>(cur + D_PBYTES)[lane] = rv;
+            if(lane < 16 && bk + step < bend) rv = __ldcg(R4 + (size_t)(bk + step) * 16 + lane);
+            __syncwarp();
+        }
+        if(!__all_sync(0xffffffffu, mbar_wait(bcur, (it >> 1) & 1u)))
+        {
+            if(lane == 0)
+            {
+                atomicExch(c.flags + F_STATUS, 6);  // STG_ERR_TIMEOUT
+                atomicExch(c.flags + F_DONE, 1);
+            }
+            // let any copy still in flight land before the CTA's shared memory is released
+            if(bk + step < bend) mbar_wait(bar0 + 8 * ((it + 1) & 1u), ((it + 1) >> 1) & 1u);
+            return;
+        }
+        const float* P = reinterpret_cast<const float*>(cur);
+        const float* rs = reinterpret_cast<const float*>(cur + D_PBYTES);
+        float z0 = 0.f, z1 = 0.f, z2 = 0.f;
+#pragma unroll
+        for(int j = 0; j < 8; j++)
+        {
+            const float4 r = *reinterpret_cast<const float4*>(rs + rcol[j]);
+            blk_fma3(P + koff[j], (tmask >> j) & 1u, r.x, r.y, r.z, z0, z1, z2);
+        }
+        bank16_join(z0, z1, z2);
+        if(h == 0) st4(c.Z + ((size_t)bk * 16 + a) * 4, z0, z1, z2);
+        __syncwarp();
+        const int nxt = bk + 2 * step;
+        if(lane == 0 && nxt < bend)
+        {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            cd_issue_inv(c, cur, bcur, nxt, extra);
+            if(!coarse) cd_issue_res(c, cur, bcur, nxt);
+        }
     }
 }
 
@@ -1083,19 +1363,6 @@ struct ATile
     static constexpr int MIN_CTAS = 2;                           // resident CTAs per SM
 };
 
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
 // shared-memory loads by 32-bit shared address
 __device__ __forceinline__ int lds_s32(unsigned a)
 {
@@ -1160,6 +1427,19 @@ __device__ __forceinline__ void ld_zp(const double* a, double& z0, double& z1, d
     (void)w1;
 }
 
+// column of stage entry f, and a zp slot's sectors on their way to L1
+template <int CAP, typename T>
+__device__ __forceinline__ int lds_col(unsigned sb, int f)
+{
+    return sizeof(T) == 4 ? lds_s32(sb + 32u * CAP + 8u * f + 4u) : lds_s32(sb + 64u * CAP + 16u * f + 8u);
+}
+template <typename T>
+__device__ __forceinline__ void prefetch_zp(const T* a)
+{
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
+    if(sizeof(T) == 8) asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 4));
+}
+
 // v_j = z_j + beta p_j gathered from the zp slots
 template <typename T>
 __device__ __forceinline__ void a_gather(int j, const T* zp, T beta, T& x0, T& x1, T& x2)
@@ -1187,9 +1467,7 @@ __global__ void __launch_bounds__(A_THREADS, ATile<T, RTT>::MIN_CTAS) k_phase_a_
     };
     const int rb = range_start(blockIdx.x), re = range_start(blockIdx.x + 1LL);
     const int mine = re > rb ? (re - rb + RT - 1) / RT : 0;
-    // the loads the start depends on are independent: issue them together
-    const int done = __ldcg(c.flags + F_DONE);
-    const double s_iter = __ldcg(c.scal + SS_ITER), rz_old = __ldcg(c.scal + SS_RZ);
+    grid_dep_release();
     int lo = 0, hi = 0;  // producer: entry bounds of the next 32 tiles, one per lane
     if(warp == A_CW && lane < mine)
     {
@@ -1235,8 +1513,8 @@ __global__ void __launch_bounds__(A_THREADS, ATile<T, RTT>::MIN_CTAS) k_phase_a_
                              (unsigned)(FP::TAIL * nc), bf, stream);
         }
     };
-    // The first STAGES tiles depend neither on beta nor on the stop flag: their copies start
-    // now and run while the r.z partials are summed.  A stopped solve drains them and returns.
+    // The first STAGES tiles depend on nothing the loop writes: their copies start before the
+    // phase before this one has ended.  A stopped solve drains them and returns.
     const int pre = min(G::STAGES, mine);
     if(warp == A_CW)
         for(int u = 0; u < pre; u++)
@@ -1244,6 +1522,25 @@ __global__ void __launch_bounds__(A_THREADS, ATile<T, RTT>::MIN_CTAS) k_phase_a_
             const int F0 = __shfl_sync(0xffffffffu, lo, u), F1 = __shfl_sync(0xffffffffu, hi, u);
             if(lane == 0) issue_tile(u, F0, F1);
         }
+    grid_dep_wait();
+    const int done = __ldcg(c.flags + F_DONE);
+    const double s_iter = __ldcg(c.scal + SS_ITER), rz_old = __ldcg(c.scal + SS_RZ);
+    // beta is not known yet, but the first tile's columns are: its operands go to L1 meanwhile
+    if(warp < A_CW && c.par >= 0 && mine > 0 && mbar_try(bar_full, 0u) && meta[1] == 0)
+    {
+        const int rl = warp * (32 / LPR) + lane / LPR;
+        if(rb + rl < min(rb + RT, re))
+        {
+            const unsigned sf = sbase + CAP * FP::ES + 4 * rl;
+            const int f0 = lds_s32(sf), f1 = lds_s32(sf + 4);
+#pragma unroll
+            for(int u = 0; u < 4; u++)
+            {
+                const int f = f0 + (lane & (LPR - 1)) + u * LPR;
+                if(f < f1) prefetch_zp(zpbuf<T>(c, c.par) + 8 * (size_t)lds_col<CAP, T>(sbase, f - meta[0]));
+            }
+        }
+    }
     // beta = rz_k / rz_(k-1): rz_k from phase E's partials, rz_(k-1) as phase B recorded it
     // (the first iteration has p_0 = 0: beta = 0)
     // flexible PCG (learned correction): beta = r_k.(z_k - z_(k-1)) / r_(k-1).z_(k-1)
@@ -1260,7 +1557,7 @@ __global__ void __launch_bounds__(A_THREADS, ATile<T, RTT>::MIN_CTAS) k_phase_a_
     }
     const double s_beta = (long)s_iter == 0 ? 0.0 : (rz_new - rz_mix) / rz_old;
 
-    const int par = ((long)s_iter) & 1;
+    const int par = c.par >= 0 ? c.par : (int)((long)s_iter & 1);
     const T* zp = zpbuf<T>(c, par);
     T* zpn = zpbuf<T>(c, par ^ 1);
     T* q = reinterpret_cast<T*>(c.q);
@@ -1508,8 +1805,7 @@ __global__ void __launch_bounds__(A_THREADS, AUpper<T>::MIN_CTAS) k_phase_a_uppe
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rb = a_range_start(blockIdx.x, gridDim.x, c.nrows), re = a_range_start(blockIdx.x + 1LL, gridDim.x, c.nrows);
     const int mine = re > rb ? (re - rb + RT - 1) / RT : 0;
-    const int done = __ldcg(c.flags + F_DONE);
-    const double s_iter = __ldcg(c.scal + SS_ITER), rz_old = __ldcg(c.scal + SS_RZ);
+    grid_dep_release();
     int lo = 0, hi = 0;  // producer: entry bounds of the next 32 tiles, one per lane
     if(warp == A_CW && lane < mine)
     {
@@ -1560,8 +1856,8 @@ __global__ void __launch_bounds__(A_THREADS, AUpper<T>::MIN_CTAS) k_phase_a_uppe
                                  (unsigned)(UP::SLOTP * nc), bf, stream);
         }
     };
-    // The first STAGES tiles depend neither on beta nor on the stop flag: their copies start
-    // now and run while the r.z partials are summed.  A stopped solve drains them and returns.
+    // The first STAGES tiles depend on nothing the loop writes: their copies start before the
+    // phase before this one has ended.  A stopped solve drains them and returns.
     const int pre = min(G::STAGES, mine);
     if(warp == A_CW)
         for(int u = 0; u < pre; u++)
@@ -1569,6 +1865,25 @@ __global__ void __launch_bounds__(A_THREADS, AUpper<T>::MIN_CTAS) k_phase_a_uppe
             const int F0 = __shfl_sync(0xffffffffu, lo, u), F1 = __shfl_sync(0xffffffffu, hi, u);
             if(lane == 0) issue_tile(u, F0, F1);
         }
+    grid_dep_wait();
+    const int done = __ldcg(c.flags + F_DONE);
+    const double s_iter = __ldcg(c.scal + SS_ITER), rz_old = __ldcg(c.scal + SS_RZ);
+    // beta is not known yet, but the first tile's columns are: its operands go to L1 meanwhile
+    if(warp < A_CW && c.par >= 0 && mine > 0 && mbar_try(bar_full, 0u) && meta[1] == 0)
+    {
+        const int rl = warp * (32 / LPR) + lane / LPR;
+        if(rb + rl < min(rb + RT, re))
+        {
+            const unsigned sf = sbase + CAP * UP::ES + 4 * rl;
+            const int f0 = lds_s32(sf), f1 = lds_s32(sf + 4);
+#pragma unroll
+            for(int u = 0; u < G::UB; u++)
+            {
+                const int f = f0 + (lane & (LPR - 1)) + u * LPR;
+                if(f < f1) prefetch_zp(zpbuf<T>(c, c.par) + 8 * (size_t)lds_col<CAP, T>(sbase, f - meta[0]));
+            }
+        }
+    }
     double rz_new, rz_mix = 0.0;
     if(c.flex && (long)s_iter > 0)
         consume_sum2<A_THREADS>(c, SITE_E, c.grid_e, SITE_F, c.grid_e, rz_new, rz_mix);
@@ -1582,7 +1897,7 @@ __global__ void __launch_bounds__(A_THREADS, AUpper<T>::MIN_CTAS) k_phase_a_uppe
     }
     const double s_beta = (long)s_iter == 0 ? 0.0 : (rz_new - rz_mix) / rz_old;
 
-    const int par = ((long)s_iter) & 1;
+    const int par = c.par >= 0 ? c.par : (int)((long)s_iter & 1);
     const T* zp = zpbuf<T>(c, par);
     T* zpn = zpbuf<T>(c, par ^ 1);
     T* q = reinterpret_cast<T*>(c.q);
@@ -2180,29 +2495,43 @@ __device__ __forceinline__ double abd_apply(const PcgDev& c, T* zp, int gt, int 
     return acc;
 }
 
-template <typename T>
-__device__ __forceinline__ double phase_e_mas(const PcgDev& c, int gt, int gn, bool skip = false)
+// level-0 slot and coarse nodes of vertex v (never written by the loop); the coarse ones beyond
+// the hierarchy stay -1
+__device__ __forceinline__ void e_load_maps(const PcgDev& c, int v, int (&node)[kMaxLevelsDev])
 {
-    T* zp = zpbuf<T>(c, iter_parity(c));
+    node[0] = c.real_map[v];
+#pragma unroll
+    for(int l = 1; l < kMaxLevelsDev; l++) node[l] = l < c.L ? c.coarse_table[(size_t)v * (c.L - 1) + l - 1] : -1;
+}
+
+// `first`: the maps of vertex gt, loaded by the caller before grid_dep_wait
+template <typename T>
+__device__ __forceinline__ double phase_e_mas(const PcgDev& c, int gt, int gn, int (&first)[kMaxLevelsDev], bool skip)
+{
+    T* zp = zpbuf<T>(c, parity_after(c));
     double acc = 0;
     const int fem_row = c.fem_dof / 3;
     for(int v = gt; v < c.V; v += gn)
     {
-        const int s = c.real_map[v];
-        float c0, c1, c2;
-        ld4(c.Z + 4 * (size_t)s, c0, c1, c2);
-        for(int l = 1; l < c.L; l++)
-        {
-            const int now = c.coarse_table[(size_t)v * (c.L - 1) + l - 1];
-            float t0, t1, t2;
-            ld4(c.Z + 4 * (size_t)now, t0, t1, t2);
-            c0 += t0;
-            c1 += t1;
-            c2 += t2;
-        }
+        if(v != gt) e_load_maps(c, v, first);
         const int row = fem_row + v;
         const double* r = c.r + 3 * (size_t)row;
-        const double rz = r[0] * (double)(T)c0 + r[1] * (double)(T)c1 + r[2] * (double)(T)c2;
+        const double r0 = r[0], r1 = r[1], r2 = r[2];
+        // all levels' loads in flight, then summed in level order
+        float t[kMaxLevelsDev][3];
+#pragma unroll
+        for(int l = 0; l < kMaxLevelsDev; l++)
+            if(l < c.L) ld4(c.Z + 4 * (size_t)first[l], t[l][0], t[l][1], t[l][2]);
+        float c0 = t[0][0], c1 = t[0][1], c2 = t[0][2];
+#pragma unroll
+        for(int l = 1; l < kMaxLevelsDev; l++)
+            if(l < c.L)
+            {
+                c0 += t[l][0];
+                c1 += t[l][1];
+                c2 += t[l][2];
+            }
+        const double rz = r0 * (double)(T)c0 + r1 * (double)(T)c1 + r2 * (double)(T)c2;
         acc += rz;
         if(skip) continue;
         st4(zp + 8 * (size_t)row, (T)c0, (T)c1, (T)c2);
@@ -2211,11 +2540,39 @@ __device__ __forceinline__ double phase_e_mas(const PcgDev& c, int gt, int gn, b
     return acc + abd_apply<T>(c, zp, gt, gn, skip);
 }
 
+// the same sums with one level in flight, for the persistent kernel (the arrays above would
+// take its second CTA per SM)
+template <typename T>
+__device__ __forceinline__ double phase_e_mas_slim(const PcgDev& c, int gt, int gn)
+{
+    T* zp = zpbuf<T>(c, iter_parity(c));
+    double acc = 0;
+    const int fem_row = c.fem_dof / 3;
+    for(int v = gt; v < c.V; v += gn)
+    {
+        float c0, c1, c2;
+        ld4(c.Z + 4 * (size_t)c.real_map[v], c0, c1, c2);
+        for(int l = 1; l < c.L; l++)
+        {
+            float t0, t1, t2;
+            ld4(c.Z + 4 * (size_t)c.coarse_table[(size_t)v * (c.L - 1) + l - 1], t0, t1, t2);
+            c0 += t0;
+            c1 += t1;
+            c2 += t2;
+        }
+        const int row = fem_row + v;
+        const double* r = c.r + 3 * (size_t)row;
+        acc += r[0] * (double)(T)c0 + r[1] * (double)(T)c1 + r[2] * (double)(T)c2;
+        st4(zp + 8 * (size_t)row, (T)c0, (T)c1, (T)c2);
+    }
+    return acc + abd_apply<T>(c, zp, gt, gn);
+}
+
 // E (global block-Jacobi / identity, then the ABD local preconditioner); share of r.z
 template <typename T>
 __device__ __forceinline__ double phase_e_plain(const PcgDev& c, int gt, int gn, bool skip = false)
 {
-    T* zp = zpbuf<T>(c, iter_parity(c));
+    T* zp = zpbuf<T>(c, parity_after(c));
     double acc = 0;
     for(int bi = c.abd_bodies * 4 + gt; bi < c.nrows; bi += gn)
     {
@@ -2273,27 +2630,30 @@ __global__ void __launch_bounds__(PB) k_phase_a(PcgDev c)
 }
 
 template <typename T, int B>
-__global__ void __launch_bounds__(PB, 4) k_phase_b(PcgDev c)
+__global__ void __launch_bounds__(PBB, 8) k_phase_b(PcgDev c, int finish)
 {
+    grid_dep_release();
+    const int gt = blockIdx.x * PBB + threadIdx.x, gn = gridDim.x * PBB;
+    BSlot<T> first;
+    if(B > 0) b_load_maps<T>(c, gt, first);
+    grid_dep_wait();
     // the first slot's loads depend neither on alpha nor on the stop flag: issue them with
     // the flag's load, before the reductions
     const int done = __ldcg(c.flags + F_DONE);
-    BSlot<T> first;
-    if(B > 0)
-        b_load<T>(c, zpbuf<T>(c, iter_parity(c) ^ 1), reinterpret_cast<const T*>(c.q), GT, first);
+    if(B > 0) b_load_vecs<T>(c, zpbuf<T>(c, parity_before(c) ^ 1), reinterpret_cast<const T*>(c.q), first);
     // the p.q and r.z partials, in flight with the slot's loads (a grid too large for the
     // registers sums them in consume_sum2 below)
-    constexpr int PK = 3;
-    const bool early = c.grid_a <= PK * PB && c.grid_e <= PK * PB;
+    constexpr int PK = 5;
+    const bool early = c.grid_a <= PK * PBB && c.grid_e <= PK * PBB;
     double pa[PK], pe[PK];
-    if(early) consume2_load<PB, PK>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pa, pe);
+    if(early) consume2_load<PBB, PK>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pa, pe);
     if(done) return;
     // After the upper SpMV, the spilled products of a warp's 32 consecutive rows (Morton
     // order: consecutive slots are consecutive rows) are one contiguous run of slots: the warp
     // copies up to SPW of them into shared memory with coalesced asynchronous copies, issued
     // before the reductions, instead of each lane reading its own run (32 lines per load).
     constexpr int SPW = 4096 / (4 * (int)sizeof(T));  // staged slots per warp (4 KB)
-    __shared__ __align__(16) T stage[B > 0 ? PB / 32 : 1][B > 0 ? 4 * SPW : 4];
+    __shared__ __align__(16) T stage[B > 0 ? PBB / 32 : 1][B > 0 ? 4 * SPW : 4];
     const int lane = threadIdx.x & 31;
     int slo = 0, shi = 0;
     if(B > 0 && c.spill && c.identity)
@@ -2317,9 +2677,9 @@ __global__ void __launch_bounds__(PB, 4) k_phase_b(PcgDev c)
     }
     double pq, rz;
     if(early)
-        consume2_finish<PB, PK>(pa, pe, pq, rz);
+        consume2_finish<PBB, PK>(pa, pe, pq, rz);
     else
-        consume_sum2<PB>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pq, rz);
+        consume_sum2<PBB>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pq, rz);
     if(B > 0 && c.spill && c.identity)
     {
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -2329,11 +2689,29 @@ __global__ void __launch_bounds__(PB, 4) k_phase_b(PcgDev c)
     if(pq > 0.0 && isfinite(pq))  // else breakdown: no update; the last CTA reports it
     {
         const double alpha = rz / pq;
-        v = B > 0 ? phase_b_mas<T, (B > 0 ? B : 16)>(c, GT, GN, alpha, first, true, shi > slo ? stage[threadIdx.x >> 5] : nullptr,
+        v = B > 0 ? phase_b_mas<T, (B > 0 ? B : 16)>(c, gt, gn, alpha, first, true, shi > slo ? stage[threadIdx.x >> 5] : nullptr,
                                                      slo, shi)
-                  : phase_b_plain<T>(c, GT, GN, alpha);
+                  : phase_b_plain<T>(c, gt, gn, alpha);
     }
-    finish_reduction(c, v, SITE_B, POST_CHECK_PQ, 0, pq, rz);
+    if(finish)
+    {
+        finish_reduction<PBB>(c, v, SITE_B, POST_CHECK_PQ, 0, pq, rz);
+        return;
+    }
+    // r.r: this CTA's partial only; k_phase_cd16 finishes the sum and the stop test beside the
+    // bank solves (finished here, the last CTA's fence, atomic and dependent loads add about
+    // 3 us to the chain)
+    __shared__ double red[PBB / 32];
+    const double bs = block_sum<PBB>(v, red);
+    if(threadIdx.x == 0)
+    {
+        c.partials[(size_t)SITE_B * c.slots + blockIdx.x] = bs;
+        if(blockIdx.x == 0)
+        {
+            c.scal[SS_PQ_B] = pq;
+            c.scal[SS_RZ_B] = rz;
+        }
+    }
 }
 
 // guarded: runs only when this iteration is a replacement iteration (host / plain graph),
@@ -2366,6 +2744,8 @@ __global__ void __launch_bounds__(PB) k_restrict01(PcgDev c, int guarded)
 template <int B>
 __global__ void __launch_bounds__(PB) k_phase_c1(PcgDev c)
 {
+    grid_dep_release();
+    grid_dep_wait();
     // the stop flag only gates the stores: its load overlaps the level's loads
     const int done = __ldcg(c.flags + F_DONE);
     if(c.L > 2) restrict_level<B>(c, c.ls[2], c.ls[3], GT, GN, done != 0);  // level 1's (count, begin)
@@ -2383,6 +2763,8 @@ constexpr int C2_SMEM_BYTES = C2_SMEM_NODES * (16 + 4 + 4);
 template <int B>
 __global__ void __launch_bounds__(1024) k_phase_c2(PcgDev c)
 {
+    grid_dep_release();
+    grid_dep_wait();
     // the stop flag only gates the stores: its load overlaps the nodes' loads
     const int done = __ldcg(c.flags + F_DONE);
     // level sizes from the parameter block (unrolled constant indices: no dependent loads)
@@ -2463,17 +2845,27 @@ __global__ void __launch_bounds__(1024) k_phase_c2(PcgDev c)
 template <int B>
 __global__ void __launch_bounds__(PB) k_phase_d(PcgDev c)
 {
+    grid_dep_release();
+    grid_dep_wait();
     if(c.flags[F_DONE]) return;
     phase_d<B>(c, blockIdx.x, c.nbanks, gridDim.x);
 }
 
 template <typename T, int B>
-__global__ void __launch_bounds__(PB, 8) k_phase_e(PcgDev c, int op)
+__global__ void __launch_bounds__(PB, 4) k_phase_e(PcgDev c, int op)
 {
+    grid_dep_release();
+    int maps[kMaxLevelsDev];
+    if(B > 0 && GT < c.V) e_load_maps(c, GT, maps);
+    grid_dep_wait();
     // the stop flag only gates the stores: its load overlaps the prolongation's loads
     const int done = __ldcg(c.flags + F_DONE);
-    const double v = B > 0 ? phase_e_mas<T>(c, GT, GN, done != 0) : phase_e_plain<T>(c, GT, GN, done != 0);
-    if(done) return;
+    const double v = B > 0 ? phase_e_mas<T>(c, GT, GN, maps, done != 0) : phase_e_plain<T>(c, GT, GN, done != 0);
+    if(done)
+    {
+        if(GT == 0) c.flags[F_STOP] = 1;
+        return;
+    }
     if(op == POST_INIT_RZ)
     {
         finish_reduction(c, v, SITE_E, POST_INIT_RZ);
@@ -2486,7 +2878,7 @@ __global__ void __launch_bounds__(PB, 8) k_phase_e(PcgDev c, int op)
     if(c.flex && (long)__ldcg(c.scal + SS_ITER) > 0)
     {
         // flexible PCG: r_(k+1).z_k with z_k still in the other zp buffer
-        const T* zo = zpbuf<T>(c, iter_parity(c) ^ 1);
+        const T* zo = zpbuf<T>(c, parity_after(c) ^ 1);
         double vo = 0;
         for(int bi = GT; bi < c.nrows; bi += GN)
         {
@@ -2521,6 +2913,8 @@ __global__ void __launch_bounds__(PB) k_seg(PcgDev c)
 {
     __shared__ double red[PB / 32];
     __shared__ bool last;
+    grid_dep_release();
+    grid_dep_wait();
     if(MODE != SEG_INIT && __ldcg(c.flags + F_DONE)) return;
     const int sc = blockIdx.x;
     const int r0 = c.seg_row_off[sc], r1 = c.seg_row_off[sc + 1];
@@ -2708,7 +3102,7 @@ __global__ void __launch_bounds__(PB) k_pcg_persistent(PcgDev c)
                 phase_d<BB>(c, blockIdx.x - 1, split, gridDim.x - 1);
             grid_barrier(c, 0.0, 0, -1, gen);
         }
-        const double ve = B > 0 ? phase_e_mas<T>(c, gt, gn) : phase_e_plain<T>(c, gt, gn);
+        const double ve = B > 0 ? phase_e_mas_slim<T>(c, gt, gn) : phase_e_plain<T>(c, gt, gn);
         grid_barrier(c, ve, SITE_E, POST_BETA, gen);
     }
 }
@@ -2971,9 +3365,39 @@ int selftest_wait(int* status, double* seconds)
 // ---------------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------------
-// MAS levels >= 2 restriction (C1 parallel, C2 one CTA) and the bank solves (D)
+// launch on the handle's stream, as a programmatic dependent of the kernel before it (dep; the
+// kernel must pass grid_dep_wait) and in clusters of `cluster` CTAs
+template <typename... P, typename... A>
+static int launch_dep(Solver& S, bool dep, int cluster, void (*kernel)(P...), int grid, int block, int smem, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = S.stream;
+    cudaLaunchAttribute at[2] = {};
+    int n = 0;
+    if(dep)
+    {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if(cluster > 1)
+    {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    STG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    S.launches++;
+    return 0;
+}
+
 // the 16-bank solves of banks [b0, b1): warp per bank, TMA-staged; one resident wave of CTAs
-static int launch_d16(Solver& S, const PcgDev& c, int b0, int b1, int guarded)
+static int launch_d16(Solver& S, const PcgDev& c, int b0, int b1, int guarded, bool dep)
 {
     if(b1 <= b0) return 0;
     const int smem = D_WARPS * D_WARP_BYTES;
@@ -2983,35 +3407,86 @@ static int launch_d16(Solver& S, const PcgDev& c, int b0, int b1, int guarded)
     int per_sm = 0;
     STG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase_d16, D_WARPS * 32, smem));
     const int grid = std::max(1, std::min(div_up(b1 - b0, D_WARPS), std::max(per_sm, 1) * kSMs));
-    k_phase_d16<<<grid, D_WARPS * 32, smem, S.stream>>>(c, b0, b1, guarded);
-    STG_LAUNCH_CHECK();
-    S.launches++;
+    STG_TRY(launch_dep(S, dep, 1, k_phase_d16, grid, D_WARPS * 32, smem, c, b0, b1, guarded));
     return 0;
 }
 
-// Restriction of the coarse levels and the bank solves of every level.
-template <int B>
-static int launch_mas_cd(Solver& S, const PcgDev& c)
+// resident clusters of k_phase_cd16 on the current device (0: it cannot run there)
+static int cd16_clusters(int* resident)
 {
-    cudaStream_t s = S.stream;
+    static thread_local unsigned long long seen = 0;
+    static thread_local int count[64];
+    int dev = 0;
+    STG_CUDA_TRY(cudaGetDevice(&dev));
+    if(first_on_device(seen))
+    {
+        const int smem = D_WARPS * D_WARP_BYTES;
+        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          cudaSharedmemCarveoutMaxShared));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(CD_CL);
+        cfg.blockDim = dim3(D_WARPS * 32);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = CD_CL;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if(cudaOccupancyMaxActiveClusters(&n, k_phase_cd16, &cfg) != cudaSuccess)
+        {
+            cudaGetLastError();
+            n = 0;
+        }
+        count[dev & 63] = n;
+    }
+    *resident = count[dev & 63];
+    return 0;
+}
+
+// The fused C + D launch: possible for 16-vertex banks with at least one coarse level to
+// restrict, level 1 within one cluster's reach (its gather of level 1 must stay short beside
+// the fine solves), clusters that fit the device, and no learned correction between D and E.
+static bool fused_cd(const Solver& S, const PcgDev& c)
+{
+    int resident = 0;
+    return S.cfg.bank_size == 16 && c.L > 2 && c.ls[2] <= CD_MAX_N1 && !c.net_mode && cd16_clusters(&resident) == 0 &&
+           resident >= 3;
+}
+
+static int launch_cd16(Solver& S, const PcgDev& c, int check, int grid_b, bool dep)
+{
+    const int smem = D_WARPS * D_WARP_BYTES, fine = c.ls[5] / 16;
+    int resident = 0;
+    STG_TRY(cd16_clusters(&resident));
+    // one resident wave: the coarse cluster, the checker's, and the fine banks' clusters
+    const int room = std::max(1, resident - 1 - check);
+    const int clusters = 1 + check + std::max(1, std::min(div_up(fine, D_WARPS * CD_CL), room));
+    return launch_dep(S, dep, CD_CL, k_phase_cd16, clusters * CD_CL, D_WARPS * 32, smem, c, fine, check, grid_b);
+}
+
+// Restriction of the coarse levels and the bank solves of every level; check: the fused launch
+// also finishes phase B's r.r over its grid_b partials.  dep: see launch_dep.
+template <int B>
+static int launch_mas_cd(Solver& S, const PcgDev& c, int check, int grid_b, bool dep)
+{
+    if(B == 16 && fused_cd(S, c)) return launch_cd16(S, c, check, grid_b, dep);
     if(c.L > 2)
     {
         const int n1 = (c.ls[2] + 31) / 32 * 32;
-        k_phase_c1<B><<<std::max(1, std::min(div_up(n1, PB), kSMs * 4)), PB, 0, s>>>(c);
-        STG_LAUNCH_CHECK();
-        S.launches++;
+        STG_TRY(launch_dep(S, dep, 1, k_phase_c1<B>, std::max(1, std::min(div_up(n1, PB), kSMs * 4)), PB, 0, c));
+        dep = true;
     }
     if(c.L > 3)
     {
-        k_phase_c2<B><<<1, 1024, C2_SMEM_BYTES, s>>>(c);
-        STG_LAUNCH_CHECK();
-        S.launches++;
+        STG_TRY(launch_dep(S, dep, 1, k_phase_c2<B>, 1, 1024, C2_SMEM_BYTES, c));
+        dep = true;
     }
-    if(B == 16) return launch_d16(S, c, 0, c.nbanks, 0);
-    k_phase_d<B><<<std::max(1, std::min(c.nbanks, kSMs * 8)), PB, 0, s>>>(c);
-    STG_LAUNCH_CHECK();
-    S.launches++;
-    return 0;
+    if(B == 16) return launch_d16(S, c, 0, c.nbanks, 0, dep);
+    return launch_dep(S, dep, 1, k_phase_d<B>, std::max(1, std::min(c.nbanks, kSMs * 8)), PB, 0, c);
 }
 
 
@@ -3089,7 +3564,7 @@ static int phase_a_grid(int nrows, int rt, int* grid, bool halo = false, bool up
 }
 
 template <typename T>
-static int launch_phase_a(const PcgDev& c, cudaStream_t s)
+static int launch_phase_a(Solver& S, const PcgDev& c, bool dep)
 {
     int grid = 0;
     STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &grid, c.halo != 0, c.upper != 0));
@@ -3098,16 +3573,11 @@ static int launch_phase_a(const PcgDev& c, cudaStream_t s)
         set_error("SpMV phase grid differs from the one phase B sums over");
         return STG_ERR_INVALID;
     }
-    if(c.upper)
-        k_phase_a_upper<T><<<grid, A_THREADS, AUpper<T>::SMEM, s>>>(c);
-    else if(c.halo)
-        k_phase_a_halo<T><<<grid, A_THREADS, AHalo<T>::SMEM, s>>>(c);
-    else if(c.a_rt == a_rt_alt<T>())
-        k_phase_a_tiled<T, a_rt_alt<T>()><<<grid, A_THREADS, ATile<T, a_rt_alt<T>()>::SMEM, s>>>(c);
-    else
-        k_phase_a_tiled<T, a_rt_default<T>()><<<grid, A_THREADS, ATile<T>::SMEM, s>>>(c);
-    STG_LAUNCH_CHECK();
-    return 0;
+    if(c.upper) return launch_dep(S, dep, 1, k_phase_a_upper<T>, grid, A_THREADS, AUpper<T>::SMEM, c);
+    if(c.halo) return launch_dep(S, false, 1, k_phase_a_halo<T>, grid, A_THREADS, AHalo<T>::SMEM, c);
+    if(c.a_rt == a_rt_alt<T>())
+        return launch_dep(S, dep, 1, k_phase_a_tiled<T, a_rt_alt<T>()>, grid, A_THREADS, ATile<T, a_rt_alt<T>()>::SMEM, c);
+    return launch_dep(S, dep, 1, k_phase_a_tiled<T, a_rt_default<T>()>, grid, A_THREADS, ATile<T>::SMEM, c);
 }
 
 // BCOO tile autotuner: every candidate of the SpMV phase launched on this system (3 untimed,
@@ -3129,10 +3599,10 @@ static int tune_phase_a(Solver& S, PcgDev c, float* us, int* out)
         c.spill = c.upper ? S.pcg.spill.data() : nullptr;
         c.a_rt = (c.halo || c.upper) ? a_rt_default<T>() : cand[v];
         STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0));
-        for(int i = 0; i < 3; i++) STG_TRY(launch_phase_a<T>(c, S.stream));
+        for(int i = 0; i < 3; i++) STG_TRY(launch_phase_a<T>(S, c, false));
         const int reps = 10;
         STG_CUDA_TRY(cudaEventRecord(S.ev[4], S.stream));
-        for(int i = 0; i < reps; i++) STG_TRY(launch_phase_a<T>(c, S.stream));
+        for(int i = 0; i < reps; i++) STG_TRY(launch_phase_a<T>(S, c, false));
         STG_CUDA_TRY(cudaEventRecord(S.ev[5], S.stream));
         STG_CUDA_TRY(cudaEventSynchronize(S.ev[5]));
         float ms = 0.f;
@@ -3174,72 +3644,70 @@ static int launch_learned(Solver& S, const PcgDev& c)
     return 0;
 }
 
+// Grids of the phases that run one thread per block row (E also one per ABD dof)
+static int row_grid(int rows) { return std::max(1, std::min(div_up(rows, PB), kSMs * 4)); }
+
+// How one iteration handles the residual replacement
+enum ReplMode : int
+{
+    REPL_NONE = 0,    // no replacement can fall on this iteration
+    REPL_GUARDED = 1, // the replacement kernels run and check the iteration themselves
+    REPL_IF = 2       // an IF node of the captured graph holds them
+};
+
+// One iteration; par: the parity of the iterations before it (-1: unknown).  dep: the first kernel follows a phase kernel directly (programmatic
+// dependent); the last kernel always is one that the next iteration may depend on that way.
 template <typename T, int B>
-static int launch_iteration(Solver& S, const PcgDev& c, int grid_vec, int grid_rows, bool in_graph_cond)
+static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep, ReplMode repl, int par)
 {
     cudaStream_t s = S.stream;
-    const bool fp32 = sizeof(T) == 4;
-    STG_TRY(launch_phase_a<T>(c, s));
-    if(c.seg_of_row)
+    PcgDev c = c0;
+    c.par = par;
+    const int grid_b = std::max(1, std::min(div_up(B > 0 ? c.M : c.nrows, PBB), kSMs * 8));
+    // phase B's stop test is finished beside the bank solves when they are fused and nothing in
+    // between depends on it
+    const bool finish = B != 16 || !fused_cd(S, c) || c.seg_of_row || repl != REPL_NONE;
+    STG_TRY(launch_phase_a<T>(S, c, dep));
+    if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_A>, c.nseg, PB, 0, c));
+    STG_TRY(launch_dep(S, true, 1, k_phase_b<T, B>, grid_b, PBB, 0, c, finish ? 1 : 0));
+    if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_B>, c.nseg, PB, 0, c));
+    if(repl == REPL_IF)
     {
-        k_seg<SEG_A><<<c.nseg, PB, 0, s>>>(c);
+        // IF node: replacement (+ re-restriction) only on replacement iterations
+        cudaStreamCaptureStatus st;
+        cudaGraph_t capg;
+        const cudaGraphNode_t* deps;
+        const cudaGraphEdgeData* edges;
+        size_t ndeps = 0;
+        STG_CUDA_TRY(cudaStreamGetCaptureInfo_v3(s, &st, nullptr, &capg, &deps, &edges, &ndeps));
+        cudaGraphNodeParams ip = {};
+        ip.type = cudaGraphNodeTypeConditional;
+        ip.conditional.handle = c.h_if;
+        ip.conditional.type = cudaGraphCondTypeIf;
+        ip.conditional.size = 1;
+        cudaGraphNode_t ifnode;
+        STG_CUDA_TRY(cudaGraphAddNode(&ifnode, capg, deps, ndeps, &ip));
+        STG_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &ifnode, 1, cudaStreamSetCaptureDependencies));
+        // the IF body is recorded by the caller (see record_if_body)
+        S.pending_if_body = ip.conditional.phGraph_out[0];
+    }
+    else if(repl == REPL_GUARDED)
+    {
+        k_replace<<<grid_rows, PB, 0, s>>>(c, 1);
         STG_LAUNCH_CHECK();
         S.launches++;
-    }
-    k_phase_b<T, B><<<B > 0 ? std::max(1, std::min(div_up(c.M, PB), kSMs * 4)) : grid_vec, PB, 0, s>>>(c);
-    STG_LAUNCH_CHECK();
-    S.launches += 2;
-    if(c.seg_of_row)
-    {
-        k_seg<SEG_B><<<c.nseg, PB, 0, s>>>(c);
-        STG_LAUNCH_CHECK();
-        S.launches++;
-    }
-    if(fp32 && c.prm.refine > 0)
-    {
-        if(in_graph_cond)
+        if(B > 0)
         {
-            // IF node: replacement (+ re-restriction) only on replacement iterations
-            cudaStreamCaptureStatus st;
-            cudaGraph_t capg;
-            const cudaGraphNode_t* deps;
-            size_t ndeps = 0;
-            STG_CUDA_TRY(cudaStreamGetCaptureInfo(s, &st, nullptr, &capg, &deps, &ndeps));
-            cudaGraphNodeParams ip = {};
-            ip.type = cudaGraphNodeTypeConditional;
-            ip.conditional.handle = c.h_if;
-            ip.conditional.type = cudaGraphCondTypeIf;
-            ip.conditional.size = 1;
-            cudaGraphNode_t ifnode;
-            STG_CUDA_TRY(cudaGraphAddNode(&ifnode, capg, deps, ndeps, &ip));
-            STG_CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &ifnode, 1, cudaStreamSetCaptureDependencies));
-            // the IF body is recorded by the caller (see record_if_body)
-            S.pending_if_body = ip.conditional.phGraph_out[0];
-        }
-        else
-        {
-            k_replace<<<grid_rows, PB, 0, s>>>(c, 1);
+            k_restrict01<(B > 0 ? B : 16)><<<row_grid(c.M), PB, 0, s>>>(c, 1);
             STG_LAUNCH_CHECK();
             S.launches++;
-            if(B > 0)
-            {
-                k_restrict01<(B > 0 ? B : 16)><<<std::max(1, std::min(div_up(c.M, PB), kSMs * 4)), PB, 0, s>>>(c, 1);
-                STG_LAUNCH_CHECK();
-                S.launches++;
-            }
         }
     }
-    if(B > 0) STG_TRY(launch_mas_cd<(B > 0 ? B : 16)>(S, c));
+    const bool after_phase = repl == REPL_NONE;
+    if(B > 0) STG_TRY(launch_mas_cd<(B > 0 ? B : 16)>(S, c, finish ? 0 : 1, grid_b, after_phase));
     if(c.net_mode) STG_TRY(launch_learned(S, c));
-    k_phase_e<T, B><<<grid_vec, PB, 0, s>>>(c, POST_BETA);
-    STG_LAUNCH_CHECK();
-    S.launches++;
-    if(c.seg_of_row)
-    {
-        k_seg<SEG_E><<<c.nseg, PB, 0, s>>>(c);
-        STG_LAUNCH_CHECK();
-        S.launches++;
-    }
+    STG_TRY(launch_dep(S, (B > 0 || after_phase) && !c.net_mode, 1, k_phase_e<T, B>, c.grid_e, PB, 0, c, (int)POST_BETA));
+    if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_E>, c.nseg, PB, 0, c));
     return 0;
 }
 
@@ -3290,7 +3758,7 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
 {
     STG_TRY((set_carveouts<T, B>()));
     STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0));
-    c.grid_e = std::max(1, std::min(div_up(c.n, PB), kSMs * 4));  // grid_vec below
+    c.grid_e = row_grid(std::max(B > 0 ? c.V : c.nrows, 12 * c.abd_bodies));
     if(c.grid_a > c.slots || c.grid_e > c.slots)
     {
         set_error("SpMV phase grid larger than the reduction slots");
@@ -3303,7 +3771,6 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
     int per_sm_a = 0;
     STG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_a, k_phase_a<T>, PB, 0));
     const int grid_rows = std::max(1, std::min(div_up(c.nrows, PB / 16), std::max(per_sm_a, 1) * kSMs));
-    const int grid_b = B > 0 ? std::max(1, std::min(div_up(c.M, PB), kSMs * 4)) : grid_vec;
     // init: r = b, x = 0, p = 0, b.b; z = M^-1 r, rz = rz0 = r.z (beta = 0 so p_new = z)
     k_init<T><<<grid_vec, PB, 0, s>>>(c);
     STG_LAUNCH_CHECK();
@@ -3311,13 +3778,13 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
     if(B > 0)
     {
         constexpr int BB = B > 0 ? B : 16;
-        k_restrict01<BB><<<grid_b, PB, 0, s>>>(c, 0);
+        k_restrict01<BB><<<row_grid(c.M), PB, 0, s>>>(c, 0);
         STG_LAUNCH_CHECK();
         S.launches++;
-        STG_TRY(launch_mas_cd<BB>(S, c));
+        STG_TRY(launch_mas_cd<BB>(S, c, 0, 0, false));
         if(c.net_mode) STG_TRY(launch_learned(S, c));
     }
-    k_phase_e<T, B><<<grid_vec, PB, 0, s>>>(c, POST_INIT_RZ);
+    k_phase_e<T, B><<<c.grid_e, PB, 0, s>>>(c, POST_INIT_RZ);
     STG_LAUNCH_CHECK();
     S.launches++;
     if(c.seg_of_row)
@@ -3337,9 +3804,10 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
     const int mode = S.cfg.loop_mode;
     if(mode == STG_LOOP_HOST)
     {
+        const ReplMode repl = sizeof(T) == 4 && c.prm.refine > 0 ? REPL_GUARDED : REPL_NONE;
         for(long it = 1; it <= max_iter; it++)
         {
-            STG_TRY((launch_iteration<T, B>(S, c, grid_vec, grid_rows, false)));
+            STG_TRY((launch_iteration<T, B>(S, c, grid_rows, false, repl, (int)(it - 1) & 1)));
             STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
             STG_CUDA_TRY(cudaStreamSynchronize(s));
             if(h_flags[F_DONE]) break;
@@ -3347,8 +3815,11 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
     }
     else if(mode == STG_LOOP_GRAPH)
     {
-        // graph: WHILE(cond) { iteration }, cond initialised to 1 (at every launch) and set by
-        // the stop test.  The captured kernels hold the parameter block by value: when it is
+        // graph: WHILE(cond) { U iterations }, cond initialised to 1 (at every launch) and set by
+        // the stop test.  A turn of the WHILE node costs about 8 us beside an iteration of 15 to
+        // 60 us, and an IF node about 4 us; the kernels of iterations past the stop return at
+        // once (about 1 us each).  U = 8 divides the default replacement interval, so that only
+        // the last iteration of a turn needs the IF node (iterations are counted from 1).  The captured kernels hold the parameter block by value: when it is
         // bytewise the one of the last capture (same buffers, sizes, scalars and kernel
         // variant), the instantiated graph is launched again instead of re-captured.
         PcgDev key = c;
@@ -3419,7 +3890,11 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
                 break;
             }
             const int l0 = S.launches;
-            rc = launch_iteration<T, B>(S, c, grid_vec, grid_rows, true);
+            int unroll = 8;
+            while(need_if && c.prm.refine % unroll != 0) unroll /= 2;
+            for(int u = 0; u < unroll && rc == 0; u++)
+                rc = launch_iteration<T, B>(S, c, grid_rows, u > 0 && !c.halo, need_if && u == unroll - 1 ? REPL_IF : REPL_NONE,
+                                            unroll > 1 ? u & 1 : -1);
             cudaGraph_t out = body;
             cudaError_t ce = cudaStreamEndCapture(S.stream, &out);
             if(rc == 0 && ce != cudaSuccess)
@@ -3429,7 +3904,7 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
             }
             if(rc == 0 && S.pending_if_body) rc = record_if_body<T, B>(S, c, grid_rows, S.pending_if_body);
             S.stream = user;
-            S.launches_per_batch = S.launches - l0;
+            S.launches_per_batch = (S.launches - l0) / unroll;
             S.launches = l0;
             if(rc) break;
             cudaError_t ie = cudaGraphInstantiate(&P.graph, g, 0);
@@ -3513,9 +3988,9 @@ int profile_spmv(Solver& S, int reps, float* avg_ms, double* bytes)
     STG_CUDA_TRY(cudaMemsetAsync(c.flags, 0, sizeof(int) * 4, s));
     auto launch = [&]() -> int {
         if(fp32)
-            STG_TRY(launch_phase_a<float>(c, s));
+            STG_TRY(launch_phase_a<float>(S, c, false));
         else
-            STG_TRY(launch_phase_a<double>(c, s));
+            STG_TRY(launch_phase_a<double>(S, c, false));
         return 0;
     };
     for(int i = 0; i < 3; i++) STG_TRY(launch());
@@ -3626,6 +4101,7 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
         c.fine_mask = mas.fine_mask.data();
         c.going_next = mas.going_next.data();
         c.closed = mas.closed.data();
+        c.lead = mas.lead.data();
         c.R = mas.R.data();
         c.Z = mas.Z.data();
         c.inv = mas.inv.data();
@@ -3653,6 +4129,7 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     c.prm.stop_rule = cfg.stop_rule;
     c.prm.refine = fp32 ? cfg.refine_interval : 0;
     c.bar = P.bar.data();
+    c.par = -1;
     // SpMV kernel: a fixed tile shape (or the halo kernel), the autotuner's choice for this
     // shape class (precision, block rows, unique blocks; one choice per class and process), or
     // the precision's default shape

@@ -54,6 +54,7 @@ struct PcgDev
     const unsigned* fine_mask;
     const int* going_next;
     const unsigned* closed;
+    const int* lead;                  // first member of every node of the levels >= 2
     float* R;
     float* Z;
     const float* inv;
@@ -81,6 +82,8 @@ struct PcgDev
     unsigned* bar;            // persistent barrier: [0] count, [1] generation
     // learned coarse correction: flexible PCG (beta from r_(k+1).(z_(k+1) - z_k), phase E's
     // r.z_old partials at SITE_F); the rest only keys the captured graph
+    int par;                  // parity of the iterations completed before this one when the
+                              // launch knows it, -1: read from the iteration counter
     int a_rt;                 // rows per tile of the SpMV phase (one of the compiled shapes)
     // independent systems (scenes) on contiguous block-row ranges, each with its own PCG
     // scalars and stop test; null seg_of_row: one system

@@ -36,14 +36,15 @@ enum : int
     F_REPL = 2,        // residual replacements performed
     F_LEARN = 3,       // nonzero: the learned coarse correction is applied
     F_LACC = 4,        // replacement checkpoints the learned correction passed
-    F_LREJ = 5         // checkpoints it failed (the correction is then switched off)
+    F_LREJ = 5,        // checkpoints it failed (the correction is then switched off)
+    F_STOP = 6         // F_DONE as phase E of the last iteration saw it (k_phase_cd16)
 };
 
 // scalar slots (mirror solver.hpp)
 enum : int
 {
     SS_RZ = 0, SS_RZ0 = 1, SS_PQ = 2, SS_ALPHA = 3, SS_BETA = 4, SS_RZNEW = 5, SS_RR = 6, SS_BB = 7, SS_ITER = 9,
-    SS_LRR = 10
+    SS_LRR = 10, SS_PQ_B = 11, SS_RZ_B = 12  // p.q and r.z as phase B used them
 };
 
 __device__ __forceinline__ void post_op(int op, int slot, double total, double* scal, int* flags, const PcgParams& p,

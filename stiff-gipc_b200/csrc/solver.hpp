@@ -96,6 +96,7 @@ struct MasState
     DBuf<int> next_prefix, next_prefix_sum;
     DBuf<int> coarse_tables;      // [L*V]
     DBuf<int> going_next;         // [L*V + M]
+    DBuf<int> lead;               // coarse node (level >= 2, global id) -> its first member's global id
     DBuf<int> coarse_table;       // [V*(L-1)]
     DBuf<int2> level_size_d;      // [kMaxLevels+1]
     DBuf<int> scratch;
