@@ -64,20 +64,16 @@ __global__ void __launch_bounds__(256) k_resid_norms(const double* __restrict__ 
     }
 }
 
-// after a pcg_solve of the same size (its scratch is sized and its counters are zero)
-static int true_residual(Solver& S, const double* b, const double* x, int n, double* rel)
+// ||b - A x||^2 and ||b||^2 into the scalars S_TRR, S_TBB (asynchronous; inside pcg_solve, whose
+// scratch it uses)
+int Solver::true_residual(const double* b, const double* x, int n)
 {
-    STG_TRY(S.pcg.q.resize(n));
-    STG_TRY(S.spmv(1.0, x, 0.0, S.pcg.q.data()));
-    double* part = S.pcg.partials.data();
-    k_resid_norms<<<std::min(RN_CTAS, div_up(n, 256)), 256, 0, S.stream>>>(b, S.pcg.q.data(), n, part,
-                                                                          S.pcg.counters.data() + 7, part + 2 * RN_CTAS);
+    STG_TRY(pcg.q.resize(n));
+    STG_TRY(spmv(1.0, x, 0.0, pcg.q.data()));
+    k_resid_norms<<<std::min(RN_CTAS, div_up(n, 256)), 256, 0, stream>>>(b, pcg.q.data(), n, pcg.partials.data(),
+                                                                        pcg.counters() + 7, pcg.scal() + S_TRR);
     STG_LAUNCH_CHECK();
-    S.launches++;
-    double h[2];
-    STG_CUDA_TRY(cudaMemcpyAsync(h, part + 2 * RN_CTAS, sizeof(h), cudaMemcpyDeviceToHost, S.stream));
-    STG_CUDA_TRY(cudaStreamSynchronize(S.stream));
-    *rel = h[1] > 0 ? std::sqrt(h[0] / h[1]) : 0.0;
+    launches++;
     return 0;
 }
 }  // namespace stg
@@ -323,9 +319,6 @@ int stg_pcg_solve(stg_handle h, const double* blocks, const int32_t* rows, const
         if(st != STG_OK && st != STG_MAX_ITER) return st;
         if(stats)
         {
-            double rel = 0;
-            STG_TRY(stg::true_residual(S, b, x, n, &rel));
-            stats->rel_residual = rel;
             stats->status = st;
             stats->nnzb = nnzb;
             stats->levels = S.mas.L;
@@ -370,14 +363,10 @@ int stg_solve_linear_system(stg_handle h, const stg_system* sys, double* x, stg_
         if(timed) STG_CUDA_TRY(cudaEventRecord(S.ev[2], s));
         S.generation++;
         if(timed) STG_CUDA_TRY(cudaEventRecord(S.ev[3], s));
-        int st = S.pcg_solve(sys->b, x, sys->n, sys->abd_bodies, sys->abd_inv, stats);
+        int st = S.pcg_solve(sys->b, x, sys->n, sys->abd_bodies, sys->abd_inv, stats, timed ? S.ev[4] : nullptr);
         if(st != STG_OK && st != STG_MAX_ITER) return st;
         if(timed)
         {
-            STG_CUDA_TRY(cudaEventRecord(S.ev[4], s));
-            double rel = 0;
-            STG_TRY(stg::true_residual(S, sys->b, x, sys->n, &rel));
-            STG_CUDA_TRY(cudaEventSynchronize(S.ev[4]));
             float t05 = 0, t51 = 0, t13 = 0, t34 = 0, t04 = 0;
             cudaEventElapsedTime(&t05, S.ev[0], S.ev[5]);
             cudaEventElapsedTime(&t51, S.ev[5], S.ev[1]);
@@ -389,7 +378,6 @@ int stg_solve_linear_system(stg_handle h, const stg_system* sys, double* x, stg_
             stats->ms_mas_assemble = t13;
             stats->ms_pcg = t34;
             stats->ms_total = t04;
-            stats->rel_residual = rel;
             stats->status = st;
             stats->nnzb = S.bcoo.nnzb;
             stats->levels = S.mas.L;

@@ -154,16 +154,8 @@ int scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int n_
         STG_LAUNCH_CHECK();
         return 0;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SCAN_CL);
-    cfg.blockDim = dim3(1024);
-    cfg.stream = s;
     cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = SCAN_CL;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = cluster_config(SCAN_CL, SCAN_CL, 1024, 0, s, &at);
     STG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_scan_exclusive<SCAN_CL>, in, out, n_dev, n_host, total));
     return 0;
 }

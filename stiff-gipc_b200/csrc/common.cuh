@@ -84,6 +84,22 @@ struct DBuf
     T* data() const { return ptr; }
 };
 
+// launch configuration of `grid` CTAs in clusters of `cluster`; `at` must outlive its use
+inline cudaLaunchConfig_t cluster_config(int grid, int cluster, int block, size_t smem, cudaStream_t s, cudaLaunchAttribute* at)
+{
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = cluster;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 inline int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
 // Kernel attributes are per device: true the first time a call site reaches it on the
@@ -114,6 +130,24 @@ template <int B>
 __device__ __forceinline__ float group_shfl(float v, int bb)
 {
     return __shfl_sync(0xffffffffu, v, ((threadIdx.x & 31) & ~(B - 1)) + bb);
+}
+
+// ascending sort of 32 register values (bitonic network, 240 exchanges)
+__device__ __forceinline__ void sort32(int (&v)[32])
+{
+#pragma unroll
+    for(int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for(int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for(int i = 0; i < 32; i++)
+            {
+                const int l = i ^ j;
+                if(l < i) continue;
+                const int x = min(v[i], v[l]), y = max(v[i], v[l]);
+                v[i] = (i & k) == 0 ? x : y;
+                v[l] = (i & k) == 0 ? y : x;
+            }
 }
 
 // 4-wide per-node vector slots {v0 v1 v2 0}: one 16-byte access (FP32) or two (FP64)

@@ -45,16 +45,16 @@ __global__ void k_conv_hist(const int* rows, const int* cols, int count, int nro
     }
 }
 
-// counting-sort scatter by row; each slot gets the triplet's index and its column, so the
-// per-row sort reads its keys contiguously
-__global__ void k_conv_scatter(const int* rows, const int* cols, int count, int nrows, const int* row_start, int* cursor,
+// counting-sort scatter by row (places in any order: the per-row sort follows); each slot gets
+// the triplet's index and its column, so the per-row sort reads its keys contiguously
+__global__ void k_conv_scatter(const int* rows, const int* cols, int count, int nrows, const int* row_start, int* row_cnt,
                                int* perm, int* pcol)
 {
     for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
     {
         const int r = rows[i], c = cols[i];
         if(r < 0 || r >= nrows || c < 0 || c >= nrows) continue;
-        const int pos = row_start[r] + atomicAdd(cursor + r, 1);
+        const int pos = row_start[r] + atomicSub(row_cnt + r, 1) - 1;  // the counts run down to zero
         perm[pos] = i;
         pcol[pos] = c;
     }
@@ -161,12 +161,13 @@ constexpr int CONV_LONG_CAP = 4096;
 
 __global__ void __launch_bounds__(CONV_LONG_THREADS) k_conv_sort_long(const int* pcol, const int* row_start,
                                                                       const int* perm_in, int* perm_out, int* scol,
-                                                                      int* uniq, const int* long_rows,
+                                                                      int* uniq, int nrows, const int* long_rows,
                                                                       const int* long_cnt)
 {
     __shared__ unsigned long long key[CONV_LONG_CAP];
     __shared__ int heads;
     const int nl = *long_cnt, t = threadIdx.x;
+    if(blockIdx.x == 0 && t == 0) uniq[nrows] = 0;  // the scan's closing value
     for(int i = blockIdx.x; i < nl; i += gridDim.x)
     {
         const int r = long_rows[i];
@@ -394,9 +395,10 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
         STG_CUDA_TRY(cudaMemsetAsync(row_ptr.data(), 0, sizeof(int) * (nrows + 1), s));
         return 0;
     }
-    STG_TRY(cv.row_cnt.resize(nrows + 1));
+    // counts, then {unique, bad, long rows}: one clear, one read-back
+    STG_TRY(cv.row_cnt.resize(nrows + 1 + 3));
+    int* const aux = cv.row_cnt.data() + nrows + 1;
     STG_TRY(cv.row_start.resize(nrows + 1));
-    STG_TRY(cv.cursor.resize(nrows + 1));
     STG_TRY(cv.perm.resize(count));
     STG_TRY(cv.perm2.resize(count));
     STG_TRY(cv.scol.resize(count));
@@ -407,33 +409,30 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
     STG_TRY(out_cols.resize(count));
     STG_TRY(out_blocks.resize((size_t)count * 9));
 
-    STG_CUDA_TRY(cudaMemsetAsync(cv.row_cnt.data(), 0, sizeof(int) * (nrows + 1), s));
-    STG_CUDA_TRY(cudaMemsetAsync(cv.cursor.data(), 0, sizeof(int) * (nrows + 1), s));
-    STG_CUDA_TRY(cudaMemsetAsync(cv.scratch.data() + 2, 0, 2 * sizeof(int), s));
+    STG_CUDA_TRY(cudaMemsetAsync(cv.row_cnt.data(), 0, sizeof(int) * (nrows + 1 + 3), s));
     const int g = std::min(div_up(count, 256), kSMs * 16);
-    k_conv_hist<<<g, 256, 0, s>>>(rows, cols, count, nrows, skip_negative, cv.row_cnt.data(), cv.scratch.data() + 2);
+    k_conv_hist<<<g, 256, 0, s>>>(rows, cols, count, nrows, skip_negative, cv.row_cnt.data(), aux + 1);
     STG_LAUNCH_CHECK();
-    STG_TRY(scan_exclusive(cv.row_cnt.data(), cv.row_start.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data(), s));
-    k_conv_scatter<<<g, 256, 0, s>>>(rows, cols, count, nrows, cv.row_start.data(), cv.cursor.data(), cv.perm.data(),
+    STG_TRY(scan_exclusive(cv.row_cnt.data(), cv.row_start.data(), nullptr, nrows + 1, nrows + 1, nullptr, s));
+    k_conv_scatter<<<g, 256, 0, s>>>(rows, cols, count, nrows, cv.row_start.data(), cv.row_cnt.data(), cv.perm.data(),
                                      cv.pcol.data());
     STG_LAUNCH_CHECK();
     const int gw = std::min(div_up((long)nrows * 32, 32 * CONV_WARPS), kSMs * 16);
     k_conv_sort_rows<<<gw, 32 * CONV_WARPS, 0, s>>>(cv.pcol.data(), cv.row_start.data(), cv.perm.data(), cv.perm2.data(),
                                                     cv.scol.data(), cv.uniq.data(), nrows, cv.long_rows.data(),
-                                                    cv.scratch.data() + 3);
+                                                    aux + 2);
     STG_LAUNCH_CHECK();
     k_conv_sort_long<<<kSMs, CONV_LONG_THREADS, 0, s>>>(cv.pcol.data(), cv.row_start.data(), cv.perm.data(),
                                                         cv.perm2.data(), cv.scol.data(), cv.uniq.data(),
-                                                        cv.long_rows.data(), cv.scratch.data() + 3);
+                                                        nrows, cv.long_rows.data(), aux + 2);
     STG_LAUNCH_CHECK();
-    STG_CUDA_TRY(cudaMemsetAsync(cv.uniq.data() + nrows, 0, sizeof(int), s));
-    STG_TRY(scan_exclusive(cv.uniq.data(), row_ptr.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data() + 1, s));
+    STG_TRY(scan_exclusive(cv.uniq.data(), row_ptr.data(), nullptr, nrows + 1, nrows + 1, aux, s));
     int h[2] = {0, 0};
     ConvFuse F;
     if(fuse)
     {
         // the fused level-0 pass needs the unique count first (its level-1 triplet arrays)
-        STG_CUDA_TRY(cudaMemcpyAsync(h, cv.scratch.data() + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        STG_CUDA_TRY(cudaMemcpyAsync(h, aux, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
         STG_CUDA_TRY(cudaStreamSynchronize(s));
         if(h[1] != 0)
         {
@@ -470,7 +469,7 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
     S.launches += 7;
     if(!fuse)
     {
-        STG_CUDA_TRY(cudaMemcpyAsync(h, cv.scratch.data() + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        STG_CUDA_TRY(cudaMemcpyAsync(h, aux, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
         STG_CUDA_TRY(cudaStreamSynchronize(s));
         if(h[1] != 0)
         {

@@ -462,24 +462,6 @@ __global__ void k_fem_fill(const int* __restrict__ tets, int T, const int* __res
         inc[start[tets[i]] + place[i]] = i;  // i = 4 t + a
 }
 
-// ascending sort of 32 register values (bitonic network, 240 exchanges)
-__device__ __forceinline__ void sort32(int (&v)[32])
-{
-#pragma unroll
-    for(int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-        for(int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-            for(int i = 0; i < 32; i++)
-            {
-                const int l = i ^ j;
-                if(l < i) continue;
-                const int x = min(v[i], v[l]), y = max(v[i], v[l]);
-                v[i] = (i & k) == 0 ? x : y;
-                v[l] = (i & k) == 0 ? y : x;
-            }
-}
-
 // Per vertex: incident (tet, slot) entries in increasing order, then the gradient and mass
 // gathered in that order (eight 32-byte shares in flight), the kinetic term, plane barriers,
 // and the vertex's diagonal triplet.  Lists of up to 32 entries (a Kuhn mesh has 24) are sorted

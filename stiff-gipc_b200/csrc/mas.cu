@@ -71,12 +71,9 @@ __global__ void k_mas_l0_mask(const int* __restrict__ part_map, const int* __res
 // (ids via real_map, OR into conn[vertex]); otherwise the previous level's coarse table
 // (OR into conn[coarse id]).
 template <int B>
-__global__ void k_mas_contacts(unsigned* conn, const int* __restrict__ coarse, const int* __restrict__ real_map,
-                               const int4* __restrict__ pairs, int ncp, int node_offset, int V)
+__device__ __forceinline__ void contact_connect(unsigned* conn, const int* coarse, const int* __restrict__ real_map,
+                                                const int4 q, int node_offset, int V)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= ncp) return;
-    const int4 q = pairs[p];
     int v[4] = {q.x, q.y, q.z, q.w};
     int cnt = 4;
     if(v[0] >= 0)
@@ -115,7 +112,7 @@ __global__ void k_mas_contacts(unsigned* conn, const int* __restrict__ coarse, c
     {
         const int id = v[i] - node_offset;
         vid[i] = (i < cnt && id >= 0 && id < V) ? id : -1;
-        cpv[i] = vid[i] >= 0 ? (coarse ? coarse[vid[i]] : real_map[vid[i]]) : -1;
+        cpv[i] = vid[i] >= 0 ? (coarse ? __ldcg(coarse + vid[i]) : real_map[vid[i]]) : -1;
     }
 #pragma unroll
     for(int i = 0; i < 4; i++)
@@ -140,6 +137,14 @@ __global__ void k_mas_contacts(unsigned* conn, const int* __restrict__ coarse, c
         else if(vid[i] >= 0 && msk[i])
             atomicOr(conn + vid[i], msk[i]);
     }
+}
+
+template <int B>
+__global__ void k_mas_contacts(unsigned* conn, const int* __restrict__ coarse, const int* __restrict__ real_map,
+                               const int4* __restrict__ pairs, int ncp, int node_offset, int V)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if(p < ncp) contact_connect<B>(conn, coarse, real_map, pairs[p], node_offset, V);
 }
 
 // Reachable set of `lane` through the bank's original masks (the visit loop of
@@ -301,6 +306,234 @@ __global__ void k_set_level1(int* ls, const int* total, int M)
 }
 
 // ---------------------------------------------------------------------------------------
+// The whole hierarchy in one launch, for meshes of up to MB_MAX_SLOTS slots: one cluster of 16
+// CTAs of 1,024 threads, the steps of the kernels above separated by cluster barriers (0.5 us)
+// instead of launches (about 4 us each, 6 a level: 122 us for 343 vertices and 152 us for 4,913,
+// of which the kernels' work was a few microseconds a level).  Larger meshes keep the separate
+// kernels, whose neighbour walks need the whole GPU.  Same integers: a component's id is the
+// number of component leaders before its own in slot order.
+// ---------------------------------------------------------------------------------------
+constexpr int MB_CL = 16, MB_T = 1024, MB_ROUNDS = 2, MB_MAX_SLOTS = MB_CL * MB_T * MB_ROUNDS;
+
+struct MasBuildArgs
+{
+    const int* part_map;
+    const int* real_map;
+    const unsigned* nstart;
+    const unsigned* nnum_init;
+    const unsigned* nlist_init;
+    unsigned* nnum;
+    unsigned* nlist;
+    unsigned* fine_mask;
+    int* prefix_orig;
+    int* coarse_tables;
+    int* going_next;
+    unsigned* closed;
+    int* lead;
+    int* coarse_table;
+    unsigned* next_mask;  // two buffers of V + B
+    int* ls;
+    const int4* pairs;
+    int ncp, node_offset, V, M, L;
+};
+
+__device__ __forceinline__ void mb_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int B>
+__global__ void __launch_bounds__(MB_T) k_mas_build_small(MasBuildArgs A)
+{
+    __shared__ unsigned orig[MB_T];
+    __shared__ int wcnt[MB_T / 32];
+    __shared__ int part;
+    const int rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gt = rank * MB_T + tid, gn = MB_CL * MB_T;
+
+    // closure of the banks over nodes [0, number) and ids in leader order: load(i, msk) gives
+    // node i's mask (false: no node), done(i, c, id, leader) stores.  Returns the id count.
+    auto level_pass = [&](int number, auto load, auto done, int* bank_count) -> int {
+        const int span = (number + 31) / 32 * 32;
+        const int chunk = ((span + MB_CL - 1) / MB_CL + 31) / 32 * 32;
+        const int lo = min(span, rank * chunk), hi = min(span, lo + chunk);
+        unsigned c[MB_ROUNDS], ball[MB_ROUNDS];
+        int base[MB_ROUNDS], carry = 0;
+        bool valid[MB_ROUNDS];
+#pragma unroll
+        for(int r = 0; r < MB_ROUNDS; r++)
+        {
+            const int i = lo + r * MB_T + tid;
+            unsigned m = 0u;
+            valid[r] = i < hi && i < number && load(i, m);
+            orig[tid] = valid[r] ? m : 0u;
+            __syncthreads();
+            c[r] = 0u;
+            bool leader = false;
+            if(valid[r])
+            {
+                const unsigned* bo = orig + (tid & ~(B - 1));
+                c[r] = bank_closure(bo, tid % B, bo[tid % B]);
+                leader = __popc(c[r] & lanemask_lt(tid % B)) == 0;
+            }
+            ball[r] = __ballot_sync(0xffffffffu, leader);
+            if(lane == 0) wcnt[warp] = __popc(ball[r]);
+            if(bank_count && i < hi && i < number && tid % B == 0)
+                bank_count[i / B] = __popc(B == 32 ? ball[r] : (ball[r] >> (lane & ~(B - 1))) & ((1u << (B & 31)) - 1u));
+            __syncthreads();
+            int x = wcnt[lane];
+#pragma unroll
+            for(int o = 1; o < 32; o <<= 1)
+            {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if(lane >= o) x += y;
+            }
+            base[r] = carry + (warp > 0 ? __shfl_sync(0xffffffffu, x, max(warp - 1, 0)) : 0);
+            carry += __shfl_sync(0xffffffffu, x, 31);
+            __syncthreads();
+        }
+        if(tid == 0) part = carry;
+        mb_barrier();
+        // lane q reads CTA q's count: one round trip for all of them
+        static_assert(MB_CL <= 32, "one lane per CTA");
+        int mine = 0;
+        if(lane < MB_CL)
+        {
+            unsigned a, v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(a)
+                         : "r"((unsigned)__cvta_generic_to_shared(&part)), "r"(lane));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+            mine = (int)v;
+        }
+        const int total = __reduce_add_sync(0xffffffffu, mine);
+        const int off = __reduce_add_sync(0xffffffffu, lane < rank ? mine : 0);
+#pragma unroll
+        for(int r = 0; r < MB_ROUNDS; r++)
+            if(valid[r])
+            {
+                const int ld = (lane & ~(B - 1)) + __ffs(c[r]) - 1;
+                done(lo + r * MB_T + tid, c[r], off + base[r] + __popc(ball[r] & lanemask_lt(ld)), ld == lane);
+            }
+        return total;
+    };
+    // neighbours eight at a time: all their loads in flight before the list is compacted
+    auto neighbours = [&](const unsigned* list, unsigned st, unsigned num, auto key, auto mine) -> unsigned {
+        unsigned nk = 0;
+        for(unsigned i0 = 0; i0 < num; i0 += 8)
+        {
+            unsigned u[8];
+            int k[8];
+#pragma unroll
+            for(int q = 0; q < 8; q++) u[q] = i0 + q < num ? __ldcg(list + st + i0 + q) : 0u;
+#pragma unroll
+            for(int q = 0; q < 8; q++) k[q] = i0 + q < num ? key(u[q]) : 0;
+#pragma unroll
+            for(int q = 0; q < 8; q++)
+                if(i0 + q < num && !mine(k[q])) A.nlist[st + nk++] = u[q];
+        }
+        return nk;
+    };
+
+    for(int i = gt; i < A.M; i += gn)
+    {
+        const int v = A.part_map[i];
+        if(v < 0) continue;
+        unsigned msk = 1u << (i % B);
+        A.nnum[v] = neighbours(
+            A.nlist_init, A.nstart[v], A.nnum_init[v], [&](unsigned u) { return A.real_map[u]; },
+            [&](int su) {
+                if(su / B != i / B) return false;
+                msk |= 1u << (su % B);
+                return true;
+            });
+        A.fine_mask[v] = msk;
+    }
+    mb_barrier();
+    if(A.ncp > 0)
+    {
+        for(int p = gt; p < A.ncp; p += gn) contact_connect<B>(A.fine_mask, nullptr, A.real_map, A.pairs[p], A.node_offset, A.V);
+        mb_barrier();
+    }
+    const bool table = A.L > 1;
+    int number = level_pass(
+        A.M,
+        [&](int i, unsigned& m) {
+            const int v = A.part_map[i];
+            if(v >= 0) m = __ldcg(A.fine_mask + v);
+            return v >= 0;
+        },
+        [&](int i, unsigned c, int id, bool) {
+            const int v = A.part_map[i];
+            A.fine_mask[v] = c;
+            A.coarse_tables[v] = id;
+            A.going_next[v] = id + A.M;
+            if(table) A.coarse_table[(size_t)v * (A.L - 1)] = id + A.M;
+        },
+        A.prefix_orig);
+    int begin = A.M;
+    if(gt == 0)
+    {
+        A.ls[0] = A.ls[1] = 0;
+        A.ls[2] = number;
+        A.ls[3] = begin;
+    }
+    for(int level = 1; level < A.L; level++)
+    {
+        unsigned* nm = A.next_mask + (size_t)(level & 1) * (A.V + B);
+        const int* prev = A.coarse_tables + (size_t)(level - 1) * A.V;
+        for(int i = gt; i < number; i += gn) nm[i] = 0u;
+        mb_barrier();
+        for(int i = gt; i < A.M; i += gn)
+        {
+            const int v = A.part_map[i];
+            if(v < 0) continue;
+            const unsigned c = (unsigned)__ldcg(prev + v);
+            unsigned msk = 0u;
+            A.nnum[v] = neighbours(
+                A.nlist, A.nstart[v], __ldcg(A.nnum + v), [&](unsigned u) { return __ldcg(prev + u); },
+                [&](int cu) {
+                    if(c / B != (unsigned)cu / B) return false;
+                    msk |= 1u << (cu % B);
+                    return true;
+                });
+            if(msk) atomicOr(nm + c, msk);
+        }
+        for(int p = gt; p < A.ncp; p += gn) contact_connect<B>(nm, prev, A.real_map, A.pairs[p], A.node_offset, A.V);
+        mb_barrier();
+        const int next = begin + (number + B - 1) / B * B;
+        const int total = level_pass(
+            number,
+            [&](int i, unsigned& m) {
+                m = (1u << (i % B)) | __ldcg(nm + i);
+                return true;
+            },
+            [&](int i, unsigned c, int id, bool leader) {
+                A.closed[begin + i] = c;
+                nm[i] = (unsigned)id;
+                A.going_next[begin + i] = id + next;
+                if(leader) A.lead[id + next] = begin + i;
+            },
+            nullptr);
+        mb_barrier();
+        for(int v = gt; v < A.V; v += gn)
+        {
+            const int id = (int)__ldcg(nm + __ldcg(prev + v));
+            A.coarse_tables[(size_t)level * A.V + v] = id;
+            if(level < A.L - 1) A.coarse_table[(size_t)v * (A.L - 1) + level] = id + next;
+        }
+        number = total;
+        begin = next;
+        if(gt == 0)
+        {
+            A.ls[2 * (level + 1)] = number;
+            A.ls[2 * (level + 1) + 1] = begin;
+        }
+    }
+    mb_barrier();  // no CTA leaves while another may read its part
+}
+
+// ---------------------------------------------------------------------------------------
 // assembly (PrepareHessian_bcoo) and inverse
 // ---------------------------------------------------------------------------------------
 // PrepareHessian_bcoo (MASPreconditioner.cu:1829-2075) accumulates, for every level l, the
@@ -386,6 +619,139 @@ __global__ void k_mas_extract(const int* __restrict__ rows, const int* __restric
         const double* H = blocks + 9 * (size_t)k;
 #pragma unroll
         for(int e = 0; e < 9; e++) D[e] = H[e];
+    }
+}
+
+// The coarse levels' aggregation in one launch, from the triplets of the first level that has
+// at most CHAIN_CAP of them: one CTA sorts a level's triplets by (row, col, index) in shared
+// memory, sums every run in that order (one thread per value), writes the level's operator and
+// bank blocks, and maps it to the next level's triplets.  As separate launches a level costs 10
+// launches and a read-back, about 55 us, for a few thousand triplets; 65 us here for
+// three levels from 2,197 triplets.
+// The sums and their order are those of convert_into.
+constexpr int CHAIN_CAP = 4096, CHAIN_T = 1024;
+constexpr int CHAIN_SMEM = CHAIN_CAP * (8 + 2) + 16;
+
+struct ChainArgs
+{
+    int* tr_rows;
+    int* tr_cols;
+    double* tr_blocks;
+    int count, level, L;      // triplets of `level`, levels
+    int begin[kMaxLevels + 1];
+    const int* going_next;
+    int* rows;                // scratch for one level's operator
+    int* cols;
+    double* blocks;
+    double* mat;
+};
+
+template <int B>
+__global__ void __launch_bounds__(CHAIN_T) k_mas_chain(ChainArgs A)
+{
+    extern __shared__ unsigned long long ckey[];
+    unsigned short* ustart = reinterpret_cast<unsigned short*>(ckey + CHAIN_CAP);  // [CHAIN_CAP + 1]
+    __shared__ int wcnt[CHAIN_T / 32];
+    __shared__ int live;
+    const int NS = nsym(B);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int n = A.count;
+    for(int level = A.level;; level++)
+    {
+        if(tid == 0) live = 0;
+        int P = 1;
+        while(P < n) P <<= 1;
+        __syncthreads();
+        int kept = 0;
+        for(int i = tid; i < P; i += CHAIN_T)
+        {
+            unsigned long long k = ~0ull;
+            const int r = i < n ? __ldcg(A.tr_rows + i) : -1;
+            if(r >= 0)
+            {
+                k = ((unsigned long long)r << 40) | ((unsigned long long)__ldcg(A.tr_cols + i) << 20) | (unsigned)i;
+                kept++;
+            }
+            ckey[i] = k;
+        }
+        if(kept) atomicAdd(&live, kept);
+        __syncthreads();
+        for(int k = 2; k <= P; k <<= 1)
+            for(int j = k >> 1; j > 0; j >>= 1)
+            {
+                for(int t = tid; t < P / 2; t += CHAIN_T)
+                {
+                    const int a = 2 * t - (t & (j - 1)), b = a + j;  // pairs (a, a ^ j), a & j == 0
+                    const unsigned long long x = ckey[a], y = ckey[b];
+                    if((x > y) == ((a & k) == 0)) ckey[a] = y, ckey[b] = x;
+                }
+                __syncthreads();
+            }
+        // run starts: each thread owns a stretch of PT keys, a block scan numbers the runs
+        const int m = live, PT = (m + CHAIN_T - 1) / CHAIN_T, i0 = min(m, tid * PT), i1 = min(m, i0 + PT);
+        int heads = 0;
+        for(int i = i0; i < i1; i++) heads += i == 0 || (ckey[i] >> 20) != (ckey[i - 1] >> 20);
+        int x = heads;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= o) x += y;
+        }
+        if(lane == 31) wcnt[warp] = x;
+        __syncthreads();
+        int w = wcnt[lane];
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            if(lane >= o) w += y;
+        }
+        const int runs = __shfl_sync(0xffffffffu, w, 31);
+        int u = x - heads + (warp > 0 ? __shfl_sync(0xffffffffu, w, max(warp - 1, 0)) : 0);
+        for(int i = i0; i < i1; i++)
+            if(i == 0 || (ckey[i] >> 20) != (ckey[i - 1] >> 20))
+            {
+                ustart[u] = (unsigned short)i;
+                A.rows[u] = (int)(ckey[i] >> 40);
+                A.cols[u] = (int)(ckey[i] >> 20) & 0xfffff;
+                u++;
+            }
+        __syncthreads();
+        const int begin = A.begin[level];
+        for(int t = tid; t < 9 * runs; t += CHAIN_T)
+        {
+            const int q = t / 9, e = t - 9 * q;
+            const int s0 = ustart[q], s1 = q + 1 < runs ? ustart[q + 1] : m;
+            double acc = __ldcg(A.tr_blocks + 9 * (size_t)((unsigned)ckey[s0] & 0xfffffu) + e);
+            for(int i = s0 + 1; i < s1; i += 16)  // a diagonal block's run holds up to about 100
+            {
+                double v[16];
+#pragma unroll
+                for(int z = 0; z < 16; z++)
+                    if(i + z < s1) v[z] = __ldcg(A.tr_blocks + 9 * (size_t)((unsigned)ckey[i + z] & 0xfffffu) + e);
+#pragma unroll
+                for(int z = 0; z < 16; z++)
+                    if(i + z < s1) acc += v[z];
+            }
+            A.blocks[t] = acc;
+            const int ga = begin + (int)(ckey[s0] >> 40), gb = begin + ((int)(ckey[s0] >> 20) & 0xfffff);
+            if(ga / B == gb / B) A.mat[((size_t)(ga / B) * NS + upper_index(B, ga % B, gb % B)) * 9 + e] = acc;
+        }
+        if(level + 1 >= A.L || runs == 0) return;
+        __syncthreads();
+        const int next = A.begin[level + 1];
+        for(int i = tid; i < runs; i += CHAIN_T)
+        {
+            const int r = __ldcg(A.rows + i), c = __ldcg(A.cols + i);
+            double H[9];
+#pragma unroll
+            for(int e = 0; e < 9; e++) H[e] = __ldcg(A.blocks + 9 * (size_t)i + e);
+            coarse_triplet(r, c, A.going_next[begin + r] - next, A.going_next[begin + c] - next, H, A.tr_rows + i,
+                           A.tr_cols + i, A.tr_blocks + 9 * (size_t)i);
+        }
+        n = runs;
+        __syncthreads();
     }
 }
 
@@ -778,7 +1144,7 @@ int Solver::mas_init(int V, int node_offset, const uint32_t* ns, const uint32_t*
     STG_TRY(m.part_map.resize(pms));
     STG_TRY(m.real_map.resize(V));
     STG_TRY(m.fine_mask.resize(V));
-    STG_TRY(m.next_mask.resize(V + B));
+    STG_TRY(m.next_mask.resize(2 * (size_t)(V + B)));
     STG_TRY(m.prefix_orig.resize(m.nb0 + 1));
     STG_TRY(m.prefix_sum_orig.resize(m.nb0 + 1));
     STG_TRY(m.next_prefix.resize(V / B + 2));
@@ -805,6 +1171,45 @@ int Solver::mas_init(int V, int node_offset, const uint32_t* ns, const uint32_t*
     return 0;
 }
 
+// one cluster's launch configuration; false where such clusters do not fit the device
+template <int B>
+static int build_small_fits(bool* fits)
+{
+    static thread_local unsigned long long seen = 0;
+    static thread_local bool ok[64];
+    int dev = 0;
+    STG_CUDA_TRY(cudaGetDevice(&dev));
+    if(first_on_device(seen))
+    {
+        cudaLaunchAttribute at = {};
+        const cudaLaunchConfig_t cfg = cluster_config(MB_CL, MB_CL, MB_T, 0, nullptr, &at);
+        int n = 0;
+        STG_CUDA_TRY(cudaFuncSetAttribute(k_mas_build_small<B>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        ok[dev & 63] = cudaOccupancyMaxActiveClusters(&n, k_mas_build_small<B>, &cfg) == cudaSuccess && n > 0;
+        cudaGetLastError();
+    }
+    *fits = ok[dev & 63];
+    return 0;
+}
+
+// reads the level sizes back and derives the bank counts
+static int mas_sizes(Solver& S, int B)
+{
+    MasState& m = S.mas;
+    STG_CUDA_TRY(cudaMemcpyAsync(m.level_size, m.level_size_d.data(), sizeof(int) * 2 * (m.L + 1), cudaMemcpyDeviceToHost,
+                                 S.stream));
+    STG_CUDA_TRY(cudaStreamSynchronize(S.stream));
+    m.total_clusters = m.level_size[2 * m.L + 1];
+    m.nbanks = m.total_clusters / B;
+    if(m.total_clusters > m.gn_size || m.total_clusters % B != 0)
+    {
+        set_error("MAS build produced an inconsistent cluster count");
+        return STG_ERR_INVALID;
+    }
+    m.built = true;
+    return 0;
+}
+
 template <int B>
 static int mas_build_t(Solver& S, const int* contacts, int ncp)
 {
@@ -812,6 +1217,20 @@ static int mas_build_t(Solver& S, const int* contacts, int ncp)
     cudaStream_t s = S.stream;
     const int V = m.V, M = m.M, L = m.L;
     int* ls = reinterpret_cast<int*>(m.level_size_d.data());
+    bool small = M <= MB_MAX_SLOTS;
+    if(small) STG_TRY(build_small_fits<B>(&small));
+    if(small)
+    {
+        MasBuildArgs A{m.part_map.data(), m.real_map.data(), m.nstart.data(), m.nnum_init.data(), m.nlist_init.data(),
+                       m.nnum.data(), m.nlist.data(), m.fine_mask.data(), m.prefix_orig.data(), m.coarse_tables.data(),
+                       m.going_next.data(), m.closed.data(), m.lead.data(), m.coarse_table.data(), m.next_mask.data(),
+                       ls, reinterpret_cast<const int4*>(contacts), ncp, m.node_offset, V, M, L};
+        cudaLaunchAttribute at = {};
+        const cudaLaunchConfig_t cfg = cluster_config(MB_CL, MB_CL, MB_T, 0, s, &at);
+        STG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_mas_build_small<B>, A));
+        S.launches++;
+        return mas_sizes(S, B);
+    }
     STG_CUDA_TRY(cudaMemcpyAsync(m.nlist.data(), m.nlist_init.data(), sizeof(unsigned) * std::max(m.nlist_size, 1),
                                  cudaMemcpyDeviceToDevice, s));
     STG_CUDA_TRY(cudaMemcpyAsync(m.nnum.data(), m.nnum_init.data(), sizeof(unsigned) * V, cudaMemcpyDeviceToDevice, s));
@@ -870,17 +1289,7 @@ static int mas_build_t(Solver& S, const int* contacts, int ncp)
         STG_LAUNCH_CHECK();
         S.launches++;
     }
-    STG_CUDA_TRY(cudaMemcpyAsync(m.level_size, ls, sizeof(int) * 2 * (L + 1), cudaMemcpyDeviceToHost, s));
-    STG_CUDA_TRY(cudaStreamSynchronize(s));
-    m.total_clusters = m.level_size[2 * L + 1];
-    m.nbanks = m.total_clusters / B;
-    if(m.total_clusters > m.gn_size || m.total_clusters % B != 0)
-    {
-        set_error("MAS build produced an inconsistent cluster count");
-        return STG_ERR_INVALID;
-    }
-    m.built = true;
-    return 0;
+    return mas_sizes(S, B);
 }
 
 int Solver::mas_build(const int* contacts, int ncp)
@@ -941,10 +1350,32 @@ static int mas_assemble_t(Solver& S, int offset)
             STG_LAUNCH_CHECK();
             S.launches++;
         }
+        // a level with few enough triplets and nodes (20-bit keys) ends the levels in one launch;
+        // the learned level's operator is read back level by level
+        auto chain = [&](int level, int count) -> bool {
+            return count <= CHAIN_CAP && m.level_size[2 * level] < (1 << 20) && S.learned.level == 0;
+        };
+        auto run_chain = [&](int level, int count) -> int {
+            STG_TRY(m.ga_rows.resize(std::max<size_t>(m.ga_rows.size, count)));
+            STG_TRY(m.ga_cols.resize(std::max<size_t>(m.ga_cols.size, count)));
+            STG_TRY(m.ga_blocks.resize(std::max<size_t>(m.ga_blocks.size, 9 * (size_t)count)));
+            ChainArgs A{m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(), count, level, m.L, {}, m.going_next.data(),
+                        m.ga_rows.data(), m.ga_cols.data(), m.ga_blocks.data(), m.mat.data()};
+            for(int l = 0; l <= m.L; l++) A.begin[l] = m.level_size[2 * l + 1];
+            static thread_local unsigned long long seen = 0;
+            if(first_on_device(seen))
+                STG_CUDA_TRY(cudaFuncSetAttribute(k_mas_chain<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SMEM));
+            k_mas_chain<B><<<1, CHAIN_T, CHAIN_SMEM, s>>>(A);
+            STG_LAUNCH_CHECK();
+            S.launches++;
+            return 0;
+        };
         int nnz = 0;
-        STG_TRY(convert_into(S, m.gcv, nnzb, m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(), m.level_size[2],
+        const bool all = chain(1, nnzb);
+        if(all) STG_TRY(run_chain(1, nnzb));
+        if(!all) STG_TRY(convert_into(S, m.gcv, nnzb, m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(), m.level_size[2],
                              true, m.ga_rows, m.ga_cols, m.ga_blocks, m.g_rowptr, &nnz));
-        for(int level = 1;; level++)
+        for(int level = 1; !all; level++)
         {
             const int begin = m.level_size[2 * level + 1];
             if(level == S.learned.level && nnz > 0)
@@ -978,6 +1409,11 @@ static int mas_assemble_t(Solver& S, int offset)
                 m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data());
             STG_LAUNCH_CHECK();
             S.launches++;
+            if(chain(level + 1, nnz))
+            {
+                STG_TRY(run_chain(level + 1, nnz));
+                break;
+            }
             int nnz2 = 0;
             STG_TRY(convert_into(S, m.gcv, nnz, m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(),
                                  m.level_size[2 * (level + 1)], false, m.gb_rows, m.gb_cols, m.gb_blocks, m.g_rowptr,

@@ -3140,7 +3140,7 @@ __global__ void k_pack_blocks(const double* __restrict__ src, int nnzb, float* d
 template <typename T>
 __global__ void k_build_full(const int* __restrict__ row_ptr, const int* __restrict__ cols,
                              const int* __restrict__ t_ptr, const int2* __restrict__ t_ent,
-                             const double* __restrict__ blocks, int nrows, size_t S, unsigned char* fent)
+                             const double* __restrict__ blocks, int nrows, size_t S, unsigned char* fent, int* frow)
 {
     const int gt = blockIdx.x * blockDim.x + threadIdx.x, sub = gt & 15;
     for(int i = gt >> 4; i < nrows; i += (gridDim.x * blockDim.x) >> 4)
@@ -3148,6 +3148,8 @@ __global__ void k_build_full(const int* __restrict__ row_ptr, const int* __restr
         const int u0 = row_ptr[i], nu = row_ptr[i + 1] - u0;
         const int t0 = t_ptr[i], nt = t_ptr[i + 1] - t0;
         const size_t f0 = (size_t)u0 + t0;
+        if(sub == 0) frow[i] = (int)f0;
+        if(sub == 1 && i == nrows - 1) frow[nrows] = (int)f0 + nt + nu;
         for(int e = sub; e < nt + nu; e += 16)
         {
             T h[9];
@@ -3176,15 +3178,6 @@ __global__ void k_build_full(const int* __restrict__ row_ptr, const int* __restr
 }
 
 // first full-copy entry of every row: frow[i] = row_ptr[i] + t_ptr[i], i <= nrows
-__global__ void k_frow(const int* __restrict__ row_ptr, const int* __restrict__ t_ptr, int nrows, int* frow)
-{
-    for(int i = blockIdx.x * blockDim.x + threadIdx.x; i <= nrows; i += gridDim.x * blockDim.x)
-        frow[i] = row_ptr[i] + t_ptr[i];
-}
-
-// Builds the upper copy (UpperPlanes) used by the upper SpMV phase: entry k is upper block k
-// in the iteration precision with its column and slot -1; k_upper_slots then gives every
-// block of a transpose list its place t in that list.
 template <typename T>
 __global__ void k_build_upper(const int* __restrict__ cols, const double* __restrict__ blocks, int nnzb, size_t S,
                               unsigned char* uent)
@@ -3228,11 +3221,15 @@ int pack_blocks(Solver& S)
     const int nnzb = A.nnzb;
     A.upper_built = false;
     if(nnzb < 1) return 0;
-    STG_TRY(A.blk64p.resize((size_t)nnzb * 10));
     const bool fp32 = S.cfg.precision == STG_PREC_FP32;
-    k_pack_blocks<<<std::max(1, std::min(div_up(nnzb, 256), kSMs * 16)), 256, 0, S.stream>>>(A.B(), nnzb, nullptr,
-                                                                                           A.blk64p.data());
-    STG_LAUNCH_CHECK();
+    if(fp32 && S.cfg.refine_interval > 0)  // read by the residual replacement only
+    {
+        STG_TRY(A.blk64p.resize((size_t)nnzb * 10));
+        k_pack_blocks<<<std::max(1, std::min(div_up(nnzb, 256), kSMs * 16)), 256, 0, S.stream>>>(A.B(), nnzb, nullptr,
+                                                                                               A.blk64p.data());
+        STG_LAUNCH_CHECK();
+        S.launches++;
+    }
     // the autotuner times every kernel: both copies; otherwise the copy the chosen kernel reads
     const bool tuning = S.spmv_tune && S.spmv_rt == 0 && S.cfg.loop_mode != STG_LOOP_PERSISTENT;
     const bool need_upper = tuning || upper_spmv_selected(S);
@@ -3276,25 +3273,21 @@ int pack_blocks(Solver& S)
     // so that every even-aligned entry range of the 8-byte tail plane is a 16-byte multiple
     A.fstride = ((size_t)2 * nnzb + 2) & ~(size_t)1;
     STG_TRY(A.frow.resize((size_t)A.nrows + 1 + 72));  // tiles copy frow[r0 .. r0 + RT + 4)
-    k_frow<<<std::max(1, std::min(div_up(A.nrows + 1, 256), kSMs * 8)), 256, 0, S.stream>>>(
-        A.row_ptr.data(), A.t_ptr.data(), A.nrows, A.frow.data());
-    STG_LAUNCH_CHECK();
-    S.launches++;
     const int g = std::max(1, std::min(div_up(A.nrows, 16), kSMs * 16));
     if(fp32)
     {
         STG_TRY(A.fent.resize(A.fstride * FullPlanes<float>::ES));
         k_build_full<float><<<g, 256, 0, S.stream>>>(A.row_ptr.data(), A.C(), A.t_ptr.data(), A.t_ent.data(), A.B(),
-                                                     A.nrows, A.fstride, A.fent.data());
+                                                     A.nrows, A.fstride, A.fent.data(), A.frow.data());
     }
     else
     {
         STG_TRY(A.fent.resize(A.fstride * FullPlanes<double>::ES));
         k_build_full<double><<<g, 256, 0, S.stream>>>(A.row_ptr.data(), A.C(), A.t_ptr.data(), A.t_ent.data(), A.B(),
-                                                      A.nrows, A.fstride, A.fent.data());
+                                                      A.nrows, A.fstride, A.fent.data(), A.frow.data());
     }
     STG_LAUNCH_CHECK();
-    S.launches += 2;
+    S.launches++;
     // operand windows of the halo SpMV phase (one CTA per tile), when that kernel may run
     A.halo_ok = false;
     if(S.spmv_rt == SPMV_HALO || S.spmv_tune)
@@ -3425,16 +3418,8 @@ static int cd16_clusters(int* resident)
         STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributePreferredSharedMemoryCarveout,
                                           cudaSharedmemCarveoutMaxShared));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(CD_CL);
-        cfg.blockDim = dim3(D_WARPS * 32);
-        cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute at = {};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = CD_CL;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
+        const cudaLaunchConfig_t cfg = cluster_config(CD_CL, CD_CL, D_WARPS * 32, smem, nullptr, &at);
         int n = 0;
         if(cudaOccupancyMaxActiveClusters(&n, k_phase_cd16, &cfg) != cudaSuccess)
         {
@@ -3754,7 +3739,7 @@ static int set_carveouts()
 }
 
 template <typename T, int B>
-static int pcg_run(Solver& S, PcgDev& c, int& h_done)
+static int pcg_run(Solver& S, PcgDev& c)
 {
     STG_TRY((set_carveouts<T, B>()));
     STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0));
@@ -3794,21 +3779,17 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
         S.launches++;
     }
 
-    int h_flags[4] = {0, 0, 0, 0};
     const long max_iter = c.prm.max_iter;
-    if(max_iter <= 1)
-    {
-        h_done = 1;
-        return 0;
-    }
+    if(max_iter <= 1) return 0;
     const int mode = S.cfg.loop_mode;
     if(mode == STG_LOOP_HOST)
     {
+        int h_flags[4] = {0, 0, 0, 0};
         const ReplMode repl = sizeof(T) == 4 && c.prm.refine > 0 ? REPL_GUARDED : REPL_NONE;
         for(long it = 1; it <= max_iter; it++)
         {
             STG_TRY((launch_iteration<T, B>(S, c, grid_rows, false, repl, (int)(it - 1) & 1)));
-            STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
+            STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
             STG_CUDA_TRY(cudaStreamSynchronize(s));
             if(h_flags[F_DONE]) break;
         }
@@ -3833,10 +3814,7 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
             c.h_if = P.graph_dev.h_if;
             c.use_cond = P.graph_dev.use_cond;
             STG_CUDA_TRY(cudaGraphLaunch(P.graph, s));
-            STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
-            STG_CUDA_TRY(cudaStreamSynchronize(s));
             c.use_cond = 0;
-            h_done = h_flags[F_DONE];
             return 0;
         }
         if(P.graph)
@@ -3920,8 +3898,6 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
         P.graph_dev = c;
         P.graph_variant = variant;
         STG_CUDA_TRY(cudaGraphLaunch(P.graph, s));
-        STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
-        STG_CUDA_TRY(cudaStreamSynchronize(s));
         c.use_cond = 0;
     }
     else
@@ -3942,10 +3918,7 @@ static int pcg_run(Solver& S, PcgDev& c, int& h_done)
         void* args[] = {&c};
         STG_CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_pcg_persistent<T, B>, grid, PB, args, 0, s));
         S.launches++;
-        STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 4, cudaMemcpyDeviceToHost, s));
-        STG_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    h_done = h_flags[F_DONE];
     return 0;
 }
 
@@ -4017,7 +3990,8 @@ int profile_spmv(Solver& S, int reps, float* avg_ms, double* bytes)
     return 0;
 }
 
-int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const double* abd_inv, stg_stats* st)
+int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const double* abd_inv, stg_stats* st,
+                      cudaEvent_t done_ev)
 {
     cudaStream_t s = stream;
     const bool fp32 = cfg.precision == STG_PREC_FP32;
@@ -4060,13 +4034,9 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     STG_TRY(pack_blocks(*this));
     const int slots = kSMs * 8;
     STG_TRY(P.partials.resize((size_t)slots * 8));
-    STG_TRY(P.scal.resize(S_COUNT));
-    STG_TRY(P.counters.resize(8));
-    STG_TRY(P.flags.resize(8));
+    STG_TRY(P.ctl.resize(PcgState::CTL_BYTES));
     STG_TRY(P.bar.resize(2));
-    STG_CUDA_TRY(cudaMemsetAsync(P.counters.data(), 0, sizeof(unsigned) * 8, s));
-    STG_CUDA_TRY(cudaMemsetAsync(P.flags.data(), 0, sizeof(int) * 8, s));
-    STG_CUDA_TRY(cudaMemsetAsync(P.scal.data(), 0, sizeof(double) * S_COUNT, s));
+    STG_CUDA_TRY(cudaMemsetAsync(P.ctl.data(), 0, PcgState::CTL_BYTES, s));
 
     // zeroed bytewise (padding included): the graph loop compares parameter blocks with memcmp
     PcgDev c;
@@ -4120,9 +4090,9 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     c.abd_bodies = abd_bodies;
     c.abd_inv = abd_inv;
     c.partials = P.partials.data();
-    c.counters = P.counters.data();
-    c.scal = P.scal.data();
-    c.flags = P.flags.data();
+    c.counters = P.counters();
+    c.scal = P.scal();
+    c.flags = P.flags();
     c.slots = slots;
     c.prm.tol = cfg.tol;
     c.prm.max_iter = (long)(cfg.max_iter_ratio * (double)n);
@@ -4226,38 +4196,45 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
         if(net_apply)
         {
             const int on = 1;
-            STG_CUDA_TRY(cudaMemcpyAsync(P.flags.data() + F_LEARN, &on, sizeof(int), cudaMemcpyHostToDevice, s));
+            STG_CUDA_TRY(cudaMemcpyAsync(P.flags() + F_LEARN, &on, sizeof(int), cudaMemcpyHostToDevice, s));
         }
         if(net_rec) STG_CUDA_TRY(cudaMemsetAsync(learned.rec_count.data(), 0, sizeof(int), s));
     }
 
-    int done = 0;
     if(fp32)
     {
         if(!use_mas)
-            STG_TRY((pcg_run<float, 0>(*this, c, done)));
+            STG_TRY((pcg_run<float, 0>(*this, c)));
         else if(cfg.bank_size == 32)
-            STG_TRY((pcg_run<float, 32>(*this, c, done)));
+            STG_TRY((pcg_run<float, 32>(*this, c)));
         else
-            STG_TRY((pcg_run<float, 16>(*this, c, done)));
+            STG_TRY((pcg_run<float, 16>(*this, c)));
     }
     else
     {
         if(!use_mas)
-            STG_TRY((pcg_run<double, 0>(*this, c, done)));
+            STG_TRY((pcg_run<double, 0>(*this, c)));
         else if(cfg.bank_size == 32)
-            STG_TRY((pcg_run<double, 32>(*this, c, done)));
+            STG_TRY((pcg_run<double, 32>(*this, c)));
         else
-            STG_TRY((pcg_run<double, 16>(*this, c, done)));
+            STG_TRY((pcg_run<double, 16>(*this, c)));
     }
     pcg_dev = c;
     pcg_ready = true;
 
-    double h_scal[S_COUNT];
-    int h_flags[8];
-    STG_CUDA_TRY(cudaMemcpyAsync(h_scal, P.scal.data(), sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, s));
-    STG_CUDA_TRY(cudaMemcpyAsync(h_flags, P.flags.data(), sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+    if(done_ev) STG_CUDA_TRY(cudaEventRecord(done_ev, s));
+    // the residual of the final x, so that one read-back brings it with the loop's scalars
+    if(st) STG_TRY(true_residual(b, x, n));
+    struct
+    {
+        double scal[S_COUNT];
+        int flags[8];
+    } h;
+    static_assert(sizeof(double) * S_COUNT == PcgState::CTL_FLAGS, "flags follow the scalars");
+    STG_CUDA_TRY(cudaMemcpyAsync(&h, P.ctl.data(), sizeof(h), cudaMemcpyDeviceToHost, s));
     STG_CUDA_TRY(cudaStreamSynchronize(s));
+    const double* h_scal = h.scal;
+    const int* h_flags = h.flags;
     const long max_iter = c.prm.max_iter;
     int status = h_flags[F_DONE] ? h_flags[F_STATUS] : STG_MAX_ITER;
     if(status == STG_ERR_TIMEOUT) set_error("persistent PCG: a grid barrier wait gave up");
@@ -4271,6 +4248,7 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     if(st)
     {
         st->iterations = (int)iters;
+        st->rel_residual = h_scal[S_TBB] > 0 ? std::sqrt(h_scal[S_TRR] / h_scal[S_TBB]) : 0.0;
         st->rz0 = h_scal[S_RZ0];
         st->rz_final = h_scal[S_RZ];
         st->rel_residual_recursive = h_scal[S_BB] > 0 ? std::sqrt(h_scal[S_RR] / h_scal[S_BB]) : 0.0;

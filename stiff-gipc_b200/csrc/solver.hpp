@@ -75,7 +75,7 @@ struct ConvFuse
 
 struct ConvertScratch
 {
-    DBuf<int> row_cnt, row_start, cursor, perm, perm2, pcol, scol, uniq, scratch, long_rows;
+    DBuf<int> row_cnt, row_start, perm, perm2, pcol, scol, uniq, scratch, long_rows;
 };
 
 struct MasState
@@ -115,9 +115,11 @@ struct PcgState
     DBuf<double> vbuf;             // zp0, zp1, q slots in the iteration precision
     DBuf<double> q;                // scratch for the true residual
     DBuf<double> partials;         // per-block partial sums, 6 sites
-    DBuf<double> scal;             // device scalars, see enum below
-    DBuf<unsigned> counters;       // last-block counters
-    DBuf<int> flags;               // [0] done, [1] status, [2] replacements
+    DBuf<unsigned char> ctl;       // scalars, flags, counters: one clear, one read-back
+    double* scal() const { return reinterpret_cast<double*>(ctl.data()); }            // see enum below
+    int* flags() const { return reinterpret_cast<int*>(ctl.data() + CTL_FLAGS); }     // F_* of reduce.cuh
+    unsigned* counters() const { return reinterpret_cast<unsigned*>(ctl.data() + CTL_COUNTERS); }  // last-CTA counters
+    static constexpr int CTL_FLAGS = 128, CTL_COUNTERS = 256, CTL_BYTES = 384;  // a 128-byte line each
     DBuf<unsigned> bar;            // persistent grid barrier
     DBuf<unsigned char> flush;     // 256 MiB written between timed SpMV launches (L2 flush)
     DBuf<double> abd_inv;          // ABD 12x12 block-Jacobi built from the BCOO [bodies * 144]
@@ -142,6 +144,8 @@ enum : int
     S_TOL = 8,     // stop threshold
     S_ITER = 9,    // completed iterations (as double)
     S_LRR = 10,    // true r.r at the last residual replacement (learned correction judge)
+    S_TRR = 13,    // ||b - A x||^2 and ||b||^2 of the final x
+    S_TBB = 14,
     S_COUNT = 16
 };
 
@@ -215,7 +219,10 @@ struct Solver
     int mas_build(const int* contacts, int ncp);
     int mas_assemble(int fem_block_offset);
     int mas_apply(const double* r, double* z);
-    int pcg_solve(const double* b, double* x, int n, int abd_bodies, const double* abd_inv, stg_stats* st);
+    // st: also the true residual of x; done_ev: recorded when the loop has ended (both may be null)
+    int pcg_solve(const double* b, double* x, int n, int abd_bodies, const double* abd_inv, stg_stats* st,
+                  cudaEvent_t done_ev = nullptr);
+    int true_residual(const double* b, const double* x, int n);
 };
 
 // ABD block-Jacobi (abd.cu): inverses of the bodies' diagonal 12x12 tiles of a sorted BCOO

@@ -85,26 +85,35 @@ __global__ void k_t_count(const int* rows, const int* cols, int nnzb, int* t_cnt
     }
 }
 
-__global__ void k_t_fill(const int* rows, const int* cols, int nnzb, const int* t_ptr, int* cursor, int2* t_ent)
+// the places of a list in any order (k_t_sort follows): the counts run down to zero
+__global__ void k_t_fill(const int* rows, const int* cols, int nnzb, const int* t_ptr, int* t_cnt, int2* t_ent)
 {
     for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnzb; k += gridDim.x * blockDim.x)
     {
         int i = rows[k], j = cols[k];
-        if(i != j)
-        {
-            int pos = t_ptr[j] + atomicAdd(cursor + j, 1);
-            t_ent[pos] = make_int2(k, i);
-        }
+        if(i != j) t_ent[t_ptr[j] + atomicSub(t_cnt + j, 1) - 1] = make_int2(k, i);
     }
 }
 
-// sort each transpose list by block index (insertion sort; lists are short) so that the
-// summation order does not depend on atomic arrival order
-__global__ void k_t_sort(const int* t_ptr, int2* t_ent, int nrows)
+// Sort each transpose list by block index, so that the summation order does not depend on
+// atomic arrival order: up to 32 entries in registers (the row of a block is read again from
+// the BCOO), longer lists in place by insertion.
+__global__ void __launch_bounds__(64) k_t_sort(const int* t_ptr, int2* t_ent, const int* __restrict__ rows, int nrows)
 {
     for(int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
     {
-        int s = t_ptr[r], e = t_ptr[r + 1];
+        const int s = t_ptr[r], e = t_ptr[r + 1], n = e - s;
+        if(n <= 32)
+        {
+            int k[32];
+#pragma unroll
+            for(int u = 0; u < 32; u++) k[u] = u < n ? t_ent[s + u].x : 0x7fffffff;
+            sort32(k);
+#pragma unroll
+            for(int u = 0; u < 32; u++)
+                if(u < n) t_ent[s + u] = make_int2(k[u], rows[k[u]]);
+            continue;
+        }
         for(int a = s + 1; a < e; a++)
         {
             int2 v = t_ent[a];
@@ -117,12 +126,6 @@ __global__ void k_t_sort(const int* t_ptr, int2* t_ent, int nrows)
             t_ent[b + 1] = v;
         }
     }
-}
-
-__global__ void k_to_f32(const double* in, float* out, size_t count)
-{
-    for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = (float)in[i];
 }
 
 // 3x3 inverse of every diagonal block (DiagPreconditioner::assemble,
@@ -179,10 +182,10 @@ int Solver::prepare_spmv()
     k_t_count<<<g, 256, 0, s>>>(bcoo.R(), bcoo.C(), nnzb, bcoo.t_cnt.data());
     STG_LAUNCH_CHECK();
     STG_TRY(scan_exclusive(bcoo.t_cnt.data(), bcoo.t_ptr.data(), nullptr, nrows + 1, nrows + 1, cv.scratch.data() + 2, s));
-    STG_CUDA_TRY(cudaMemsetAsync(bcoo.t_cnt.data(), 0, sizeof(int) * (nrows + 1), s));
     k_t_fill<<<g, 256, 0, s>>>(bcoo.R(), bcoo.C(), nnzb, bcoo.t_ptr.data(), bcoo.t_cnt.data(), bcoo.t_ent.data());
     STG_LAUNCH_CHECK();
-    k_t_sort<<<std::max(1, std::min(div_up(nrows, 256), kSMs * 16)), 256, 0, s>>>(bcoo.t_ptr.data(), bcoo.t_ent.data(), nrows);
+    k_t_sort<<<std::max(1, std::min(div_up(nrows, 64), kSMs * 64)), 64, 0, s>>>(bcoo.t_ptr.data(), bcoo.t_ent.data(),
+                                                                              bcoo.R(), nrows);
     STG_LAUNCH_CHECK();
     launches += 4;
     if(cfg.preconditioner == STG_PRECOND_DIAG)
@@ -372,10 +375,9 @@ int spmv_noalloc(double a, const double* blocks, const int* rows, const int* col
     k_t_count<<<g, 256, 0, s>>>(rows, cols, nnzb, t_cnt);
     STG_LAUNCH_CHECK();
     STG_TRY(scan_exclusive(t_cnt, t_ptr, nullptr, nrows + 1, nrows + 1, counters + 1, s));
-    STG_CUDA_TRY(cudaMemsetAsync(t_cnt, 0, sizeof(int) * (nrows + 1), s));
     k_t_fill<<<g, 256, 0, s>>>(rows, cols, nnzb, t_ptr, t_cnt, t_ent);
     STG_LAUNCH_CHECK();
-    k_t_sort<<<std::max(1, std::min(div_up(nrows, 256), kSMs * 16)), 256, 0, s>>>(t_ptr, t_ent, nrows);
+    k_t_sort<<<std::max(1, std::min(div_up(nrows, 64), kSMs * 64)), 64, 0, s>>>(t_ptr, t_ent, rows, nrows);
     STG_LAUNCH_CHECK();
     const int grid = std::max(1, std::min(div_up(nrows, 256 / 16), kSMs * 8));
     k_spmv_sym<double, 16><<<grid, 256, 0, s>>>(row_ptr, cols, blocks, t_ptr, t_ent, x, y, a, b, nrows);
