@@ -1051,8 +1051,8 @@ __global__ void __launch_bounds__(D_WARPS * 32) k_phase_d16(PcgDev c, int b0, in
 // for them.  The restriction is a gather (one thread per coarse node, its members' loads all in
 // flight) that forms two levels at a time, so levels 2 to 5 take one cluster barrier and one
 // CTA barrier; level by level with a barrier each it took 14.8 us.  Sums, their order and the
-// bank arithmetic are those of restrict_level and k_phase_d16.  With `check`, the last cluster finishes phase
-// B's r.r and the stop test (the order of finish_reduction).
+// bank arithmetic are those of restrict_level and k_phase_d16.  With `checkers`, the last clusters
+// finish phase B's r.r and the stop test (cd_check).
 //
 // Both stages' inverses are on their way before grid_dep_wait; the residual slots follow it.
 // F_STOP, not F_DONE, skips a finished solve: F_DONE may be written while this kernel runs, and
@@ -1072,18 +1072,20 @@ struct Members
     int bank = 0;
     unsigned mask = 0u;
 };
+template <int B>
 __device__ __forceinline__ Members members_of(const PcgDev& c, int node)
 {
     Members m;
     const int first = __ldg(c.lead + node);
-    m.bank = first & ~15;
+    m.bank = first & ~(B - 1);
     m.mask = __ldg(c.closed + first);
     return m;
 }
 
 // Residuals of the nodes of level l (threads gt, gt + gn, ...: each sums its members of level
-// l - 1 in lane order, all loads in flight) and, when there is one, of level l + 1 (a bank's
-// sums meet in its 16 lanes, as phase B forms level 1).  `mine`: the members of node gt.
+// l - 1 in lane order, 16 loads in flight) and, when there is one, of level l + 1 (a bank's
+// sums meet in its lanes, as phase B forms level 1).  `mine`: the members of node gt.
+template <int B>
 __device__ __forceinline__ void restrict_two(const PcgDev& c, int l, int gt, int gn, Members mine)
 {
     const int number = __ldg(c.ls_dev + 2 * l), begin = __ldg(c.ls_dev + 2 * l + 1);
@@ -1092,7 +1094,7 @@ __device__ __forceinline__ void restrict_two(const PcgDev& c, int l, int gt, int
     for(int i = gt; i < span; i += gn)
     {
         const bool valid = i < number;
-        if(i != gt) mine = valid ? members_of(c, begin + i) : Members();
+        if(i != gt) mine = valid ? members_of<B>(c, begin + i) : Members();
         unsigned msk = 0u;
         int g = 0;
         if(valid && l + 1 < c.L)
@@ -1100,26 +1102,30 @@ __device__ __forceinline__ void restrict_two(const PcgDev& c, int l, int gt, int
             msk = __ldg(c.closed + begin + i);
             g = __ldg(c.going_next + begin + i);
         }
-        float4 r[16];
-#pragma unroll
-        for(int b = 0; b < 16; b++)
-            if((mine.mask >> b) & 1u) r[b] = __ldcg(R4 + mine.bank + b);
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll
-        for(int b = 0; b < 16; b++)
-            if((mine.mask >> b) & 1u)
-            {
-                s0 += r[b].x;
-                s1 += r[b].y;
-                s2 += r[b].z;
-            }
+        for(int h = 0; h < B; h += 16)
+        {
+            float4 r[16];
+#pragma unroll
+            for(int b = 0; b < 16; b++)
+                if((mine.mask >> (h + b)) & 1u) r[b] = __ldcg(R4 + mine.bank + h + b);
+#pragma unroll
+            for(int b = 0; b < 16; b++)
+                if((mine.mask >> (h + b)) & 1u)
+                {
+                    s0 += r[b].x;
+                    s1 += r[b].y;
+                    s2 += r[b].z;
+                }
+        }
         if(valid) st4(c.R + 4 * (size_t)(begin + i), s0, s1, s2);
         if(l + 1 >= c.L) continue;
         float a0 = 0.f, a1 = 0.f, a2 = 0.f;
 #pragma unroll 4
-        for(int b = 0; b < 16; b++)
+        for(int b = 0; b < B; b++)
         {
-            const float x0 = group_shfl<16>(s0, b), x1 = group_shfl<16>(s1, b), x2 = group_shfl<16>(s2, b);
+            const float x0 = group_shfl<B>(s0, b), x1 = group_shfl<B>(s1, b), x2 = group_shfl<B>(s2, b);
             if(msk & (1u << b))
             {
                 a0 += x0;
@@ -1127,8 +1133,121 @@ __device__ __forceinline__ void restrict_two(const PcgDev& c, int l, int gt, int
                 a2 += x2;
             }
         }
-        if(valid && __popc(msk & lanemask_lt(i % 16)) == 0) st4(c.R + 4 * (size_t)g, a0, a1, a2);
+        if(valid && __popc(msk & lanemask_lt(i % B)) == 0) st4(c.R + 4 * (size_t)g, a0, a1, a2);
     }
+}
+
+// The banks of one worker (a warp with 16-vertex banks, a CTA with 32-vertex ones; CD_CL * W
+// workers per cluster): the fine clusters share banks [0, fine), the coarse cluster the rest,
+// the banks of levels 4 and 5 going to its first CTA, which restricts those levels.
+struct CdBanks
+{
+    int first, step, end;
+};
+template <int B, int W>
+__device__ __forceinline__ CdBanks cd_banks(const PcgDev& c, int fine, int checkers, int worker)
+{
+    const int cl = blockIdx.x / CD_CL, rank = blockIdx.x % CD_CL, clusters = gridDim.x / CD_CL;
+    const bool top = c.L > 4;
+    const int bank4 = top ? c.ls[9] / B : c.nbanks;
+    if(cl >= clusters - checkers) return {0, 1, 0};
+    if(cl > 0) return {((int)blockIdx.x - CD_CL) * W + worker, (clusters - 1 - checkers) * CD_CL * W, fine};
+    if(top && rank == 0) return {bank4 + worker, W, c.nbanks};
+    const int skip = top ? 1 : 0;
+    return {fine + (rank - skip) * W + worker, (CD_CL - skip) * W, bank4};
+}
+
+// The coarse cluster's restriction: levels 2 and 3 by the cluster, then 4 and 5 by its first
+// CTA.  The first members are loaded by cd_members, before grid_dep_wait.
+template <int B>
+__device__ __forceinline__ void cd_members(const PcgDev& c, int rank, Members& m2, Members& m4)
+{
+    const int i2 = rank * D_WARPS * 32 + threadIdx.x;
+    if(i2 < c.ls[4]) m2 = members_of<B>(c, c.ls[5] + i2);
+    if(c.L > 4 && rank == 0 && (int)threadIdx.x < c.ls[8]) m4 = members_of<B>(c, c.ls[9] + threadIdx.x);
+}
+template <int B>
+__device__ __forceinline__ void cd_restrict(const PcgDev& c, int rank, const Members& m2, const Members& m4)
+{
+    restrict_two<B>(c, 2, rank * D_WARPS * 32 + threadIdx.x, CD_CL * D_WARPS * 32, m2);
+    cluster_barrier();
+    if(c.L > 4 && rank == 0)
+    {
+        restrict_two<B>(c, 4, threadIdx.x, D_WARPS * 32, m4);
+        __syncthreads();
+    }
+}
+
+// Phase B's r.r and the stop test, by one CTA of the last cluster (128 threads, in the order of
+// phase B's finish_reduction); with scenes, one CTA per scene (the last `checkers` clusters)
+// first runs the scene's test as k_seg<SEG_B> does, and the last of them to finish goes on.
+__device__ __forceinline__ void cd_check(const PcgDev& c, int grid_b, int checkers)
+{
+    static_assert(PBB == D_WARPS * 32, "the checker sums as phase B's finish_reduction does");
+    __shared__ double red[8];
+    __shared__ bool last;
+    const int id = (int)blockIdx.x - ((int)gridDim.x - checkers * CD_CL);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if(!c.seg_of_row)
+    {
+        if(id != 0) return;
+    }
+    else
+    {
+        if(id >= c.nseg) return;
+        const int r0 = c.seg_row_off[id], r1 = c.seg_row_off[id + 1];
+        const double* src = c.seg_row + (size_t)c.nrows;
+        double v0 = 0, v1 = 0;  // threads t and t + 128 of k_seg's 256
+        for(int i = r0 + (int)threadIdx.x; i < r1; i += PB) v0 += __ldcg(src + i);
+        for(int i = r0 + (int)threadIdx.x + PB / 2; i < r1; i += PB) v1 += __ldcg(src + i);
+        v0 = warp_sum(v0);
+        v1 = warp_sum(v1);
+        if(lane == 0)
+        {
+            red[warp] = v0;
+            red[warp + 4] = v1;
+        }
+        __syncthreads();
+        const double v = warp == 0 ? warp_sum(lane < 8 ? red[lane] : 0.0) : 0.0;
+        if(threadIdx.x == 0)
+        {
+            // the iteration that just ended; at the iteration limit the loop ends before the
+            // scenes' test, as with the separate launches
+            const long k = (long)__ldcg(c.scal + SS_ITER) + 1;
+            double* S = c.seg + SEG_N * (size_t)id;
+            if(k + 1 < c.prm.max_iter)
+            {
+                S[SG_RR] = v;
+                if(S[SG_DONE] == 0.0 && v <= c.seg_tol2 * S[SG_BB])
+                {
+                    S[SG_DONE] = 1.0;
+                    S[SG_ITER] = (double)k;
+                }
+            }
+            __threadfence();
+            last = atomicAdd(c.counters + CNT_SEG, 1u) == (unsigned)(c.nseg - 1);
+        }
+        __syncthreads();
+        if(!last) return;
+        __threadfence();
+    }
+    const double tot = block_sum<PBB>(strided_sum<PBB>(c.partials + (size_t)SITE_B * c.slots, grid_b), red);
+    double open = 0;
+    if(c.seg_of_row)
+    {
+        for(int q = threadIdx.x; q < c.nseg; q += PBB) open += __ldcg(c.seg + SEG_N * (size_t)q + SG_DONE) == 0.0 ? 1.0 : 0.0;
+        open = block_sum<PBB>(open, red);
+    }
+    if(threadIdx.x != 0) return;
+    if(c.seg_of_row) c.counters[CNT_SEG] = 0u;
+    if(__ldcg(c.flags + F_DONE)) return;
+    post_op(POST_CHECK_PQ, 0, tot, c.scal, c.flags, c.prm, __ldcg(c.scal + SS_PQ_B), __ldcg(c.scal + SS_RZ_B));
+    if(c.seg_of_row && open == 0.0 && !c.flags[F_DONE])
+    {
+        c.flags[F_DONE] = 1;
+        c.flags[F_STATUS] = 0;
+    }
+    set_conditionals(c, POST_CHECK);
 }
 
 // bank bk's inverse into a stage; the barrier expects it plus `extra` bytes
@@ -1142,32 +1261,18 @@ __device__ __forceinline__ void cd_issue_res(const PcgDev& c, char* stage, unsig
     tma_load_1d_hint(stage + D_PBYTES, c.R + (size_t)bk * 16 * 4, D_RBYTES, bar, l2_evict_last());
 }
 
-__global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine, int check, int grid_b)
+__global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine, int checkers, int grid_b)
 {
     grid_dep_release();
     extern __shared__ __align__(128) char dsm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cl = blockIdx.x / CD_CL, rank = blockIdx.x % CD_CL;
-    const int fine_ctas = gridDim.x - CD_CL * (1 + check);
-    const bool coarse = cl == 0, checker = check && cl == (int)gridDim.x / CD_CL - 1;
-    const bool top = c.L > 4;  // levels 4 and 5: the banks of CTA 0 of the coarse cluster
-    const int bank4 = top ? c.ls[9] / 16 : c.nbanks;
-    // this warp's banks: first, stride, end
-    int bk0, step, bend;
-    if(!coarse)
-        bk0 = ((int)blockIdx.x - CD_CL) * D_WARPS + warp, step = fine_ctas * D_WARPS, bend = checker ? 0 : fine;
-    else if(top && rank == 0)
-        bk0 = bank4 + warp, step = D_WARPS, bend = c.nbanks;
-    else
-        bk0 = fine + (rank - (top ? 1 : 0)) * D_WARPS + warp, step = (CD_CL - (top ? 1 : 0)) * D_WARPS, bend = bank4;
+    const int rank = blockIdx.x % CD_CL;
+    const bool coarse = blockIdx.x < CD_CL, checker = (int)blockIdx.x >= (int)gridDim.x - checkers * CD_CL;
+    const CdBanks mine = cd_banks<16, D_WARPS>(c, fine, checkers, warp);
+    const int bk0 = mine.first, step = mine.step, bend = mine.end;
     const int extra = coarse ? 0 : D_RBYTES;
     Members mem2, mem4;
-    if(coarse)
-    {
-        const int i2 = rank * D_WARPS * 32 + threadIdx.x;
-        if(i2 < c.ls[4]) mem2 = members_of(c, c.ls[5] + i2);
-        if(top && rank == 0 && (int)threadIdx.x < c.ls[8]) mem4 = members_of(c, c.ls[9] + threadIdx.x);
-    }
+    if(coarse) cd_members<16>(c, rank, mem2, mem4);
     char* const base = dsm + (size_t)warp * D_WARP_BYTES;
     const unsigned bar0 = smem_u32(base + 2 * D_BUF);
     if(lane == 0)
@@ -1195,15 +1300,7 @@ __global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine,
     const int stop = __ldcg(c.flags + F_STOP);
     if(checker)
     {
-        if(rank != 0 || stop) return;
-        static_assert(PBB == D_WARPS * 32, "the checker sums as phase B's finish_reduction does");
-        __shared__ double red[PBB / 32];
-        const double tot = block_sum<PBB>(strided_sum<PBB>(c.partials + (size_t)SITE_B * c.slots, grid_b), red);
-        if(threadIdx.x == 0 && !__ldcg(c.flags + F_DONE))
-        {
-            post_op(POST_CHECK_PQ, 0, tot, c.scal, c.flags, c.prm, __ldcg(c.scal + SS_PQ_B), __ldcg(c.scal + SS_RZ_B));
-            set_conditionals(c, POST_CHECK);
-        }
+        if(!stop) cd_check(c, grid_b, checkers);
         return;
     }
     if(!coarse && lane == 0)
@@ -1221,17 +1318,7 @@ __global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine,
         }
         return;
     }
-    if(coarse)
-    {
-        // levels 2 and 3 by the cluster, then 4 and 5 by its first CTA, which solves their banks
-        restrict_two(c, 2, rank * D_WARPS * 32 + threadIdx.x, CD_CL * D_WARPS * 32, mem2);
-        cluster_barrier();
-        if(top && rank == 0)
-        {
-            restrict_two(c, 4, threadIdx.x, D_WARPS * 32, mem4);
-            __syncthreads();
-        }
-    }
+    if(coarse) cd_restrict<16>(c, rank, mem2, mem4);
     const float4* R4 = reinterpret_cast<const float4*>(c.R);
     float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
     if(coarse && lane < 16 && bk0 < bend) rv = __ldcg(R4 + (size_t)bk0 * 16 + lane);
@@ -1276,6 +1363,110 @@ __global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd16(PcgDev c, int fine,
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             cd_issue_inv(c, cur, bcur, nxt, extra);
             if(!coarse) cd_issue_res(c, cur, bcur, nxt);
+        }
+    }
+}
+
+// The same for 32-vertex banks: one CTA per bank (its packed inverse, 19,008 B, and 32 residual
+// slots, two stages), warp w forming block rows 8 w .. 8 w + 7 with the arithmetic of phase_d<32>
+// (lane c: column block c, then the xor butterfly).  Without the staging ring and beside the
+// restriction the 32-bank iteration takes the same chain as the 16-bank one.
+constexpr int D32_PBYTES = 528 * 9 * 4, D32_RBYTES = 32 * 16, D32_BUF = D32_PBYTES + D32_RBYTES;
+constexpr int D32_SMEM = 2 * D32_BUF + 16;
+
+__global__ void __launch_bounds__(D_WARPS * 32) k_phase_cd32(PcgDev c, int fine, int checkers, int grid_b)
+{
+    grid_dep_release();
+    extern __shared__ __align__(128) char dsm[];
+    constexpr int B = 32, ROWS = B / D_WARPS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % CD_CL;
+    const bool coarse = blockIdx.x < CD_CL, checker = (int)blockIdx.x >= (int)gridDim.x - checkers * CD_CL;
+    const CdBanks mine = cd_banks<B, 1>(c, fine, checkers, 0);
+    const int bk0 = mine.first, step = mine.step, bend = mine.end;
+    const int extra = coarse ? 0 : D32_RBYTES;
+    const unsigned bar0 = smem_u32(dsm + 2 * D32_BUF);
+    auto issue_inv = [&](int s, int bk) {
+        mbar_expect_tx(bar0 + 8 * s, (unsigned)(D32_PBYTES + extra));
+        tma_load_1d_hint(dsm + s * D32_BUF, c.inv + (size_t)bk * 528 * 9, D32_PBYTES, bar0 + 8 * s, l2_evict_last());
+    };
+    auto issue_res = [&](int s, int bk) {
+        tma_load_1d_hint(dsm + s * D32_BUF + D32_PBYTES, c.R + (size_t)bk * B * 4, D32_RBYTES, bar0 + 8 * s,
+                         l2_evict_last());
+    };
+    Members mem2, mem4;
+    if(coarse) cd_members<B>(c, rank, mem2, mem4);
+    if(threadIdx.x == 0)
+    {
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if(bk0 < bend) issue_inv(0, bk0);
+        if(bk0 + step < bend) issue_inv(1, bk0 + step);
+    }
+    __syncthreads();
+    grid_dep_wait();
+    const int stop = __ldcg(c.flags + F_STOP);
+    if(checker)
+    {
+        if(!stop) cd_check(c, grid_b, checkers);
+        return;
+    }
+    if(!coarse && threadIdx.x == 0)
+    {
+        if(bk0 < bend) issue_res(0, bk0);
+        if(bk0 + step < bend) issue_res(1, bk0 + step);
+    }
+    if(stop)
+    {
+        if(threadIdx.x == 0)
+        {
+            if(bk0 < bend) mbar_wait(bar0, 0u);
+            if(bk0 + step < bend) mbar_wait(bar0 + 8, 0u);
+        }
+        return;
+    }
+    if(coarse) cd_restrict<B>(c, rank, mem2, mem4);
+    unsigned it = 0;
+    for(int bk = bk0; bk < bend; bk += step, it++)
+    {
+        const int s = it & 1u;
+        char* const cur = dsm + s * D32_BUF;
+        // levels >= 2 were written by this kernel: read with plain loads
+        if(coarse && threadIdx.x < B)
+            reinterpret_cast<float4*>(cur + D32_PBYTES)[lane] =
+                __ldcg(reinterpret_cast<const float4*>(c.R) + (size_t)bk * B + lane);
+        const bool ok = mbar_wait(bar0 + 8 * s, (it >> 1) & 1u);
+        if(!__syncthreads_and(ok))
+        {
+            if(threadIdx.x == 0)
+            {
+                atomicExch(c.flags + F_STATUS, 6);  // STG_ERR_TIMEOUT
+                atomicExch(c.flags + F_DONE, 1);
+                // let any copy still in flight land before the CTA's shared memory is released
+                if(bk + step < bend) mbar_wait(bar0 + 8 * (s ^ 1), ((it + 1) >> 1) & 1u);
+            }
+            __syncthreads();
+            return;
+        }
+        const float* P = reinterpret_cast<const float*>(cur);
+        const float4 x = reinterpret_cast<const float4*>(cur + D32_PBYTES)[lane];
+#pragma unroll 2
+        for(int r = 0; r < ROWS; r++)
+        {
+            const int a = warp * ROWS + r, lo = min(a, lane), hi = max(a, lane);
+            float z0, z1, z2;
+            blk_mul3(P + (B * lo - lo * (lo + 1) / 2 + hi) * 9, lane < a, x.x, x.y, x.z, z0, z1, z2);
+            warp_butterfly3(z0, z1, z2);
+            if(lane == 0) st4(c.Z + ((size_t)bk * B + a) * 4, z0, z1, z2);
+        }
+        __syncthreads();
+        const int nxt = bk + 2 * step;
+        if(threadIdx.x == 0 && nxt < bend)
+        {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue_inv(s, nxt);
+            if(!coarse) issue_res(s, nxt);
         }
     }
 }
@@ -3404,8 +3595,9 @@ static int launch_d16(Solver& S, const PcgDev& c, int b0, int b1, int guarded, b
     return 0;
 }
 
-// resident clusters of k_phase_cd16 on the current device (0: it cannot run there)
-static int cd16_clusters(int* resident)
+// resident clusters of k_phase_cd16 / k_phase_cd32 on the current device (0: it cannot run there)
+template <int B>
+static int cd_clusters(int* resident)
 {
     static thread_local unsigned long long seen = 0;
     static thread_local int count[64];
@@ -3413,15 +3605,16 @@ static int cd16_clusters(int* resident)
     STG_CUDA_TRY(cudaGetDevice(&dev));
     if(first_on_device(seen))
     {
-        const int smem = D_WARPS * D_WARP_BYTES;
-        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        STG_CUDA_TRY(cudaFuncSetAttribute(k_phase_cd16, cudaFuncAttributePreferredSharedMemoryCarveout,
+        const auto kernel = B == 16 ? k_phase_cd16 : k_phase_cd32;
+        const int smem = B == 16 ? D_WARPS * D_WARP_BYTES : D32_SMEM;
+        STG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        STG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        STG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                           cudaSharedmemCarveoutMaxShared));
         cudaLaunchAttribute at = {};
         const cudaLaunchConfig_t cfg = cluster_config(CD_CL, CD_CL, D_WARPS * 32, smem, nullptr, &at);
         int n = 0;
-        if(cudaOccupancyMaxActiveClusters(&n, k_phase_cd16, &cfg) != cudaSuccess)
+        if(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)
         {
             cudaGetLastError();
             n = 0;
@@ -3432,33 +3625,44 @@ static int cd16_clusters(int* resident)
     return 0;
 }
 
-// The fused C + D launch: possible for 16-vertex banks with at least one coarse level to
-// restrict, level 1 within one cluster's reach (its gather of level 1 must stay short beside
-// the fine solves), clusters that fit the device, and no learned correction between D and E.
-static bool fused_cd(const Solver& S, const PcgDev& c)
+// clusters of CTAs that run the stop test: one CTA, or one per scene
+static int cd_checkers(const PcgDev& c) { return c.seg_of_row ? div_up(c.nseg, CD_CL) : 1; }
+
+// The fused C + D launch: possible with at least one coarse level to restrict, level 1 within
+// one cluster's reach (its gather of level 1 must stay short beside the fine solves), clusters
+// that fit the device, no learned correction between D and E, and scenes few enough that their
+// test CTAs leave most of the resident clusters to the banks.
+template <int B>
+static bool fused_cd(const PcgDev& c)
 {
-    int resident = 0;
-    return S.cfg.bank_size == 16 && c.L > 2 && c.ls[2] <= CD_MAX_N1 && !c.net_mode && cd16_clusters(&resident) == 0 &&
-           resident >= 3;
+    if constexpr(B == 16 || B == 32)
+    {
+        int resident = 0;
+        return c.L > 2 && c.ls[2] <= CD_MAX_N1 && !c.net_mode && cd_clusters<B>(&resident) == 0 && resident >= 3 &&
+               4 * cd_checkers(c) <= std::max(resident, 4);
+    }
+    return false;
 }
 
-static int launch_cd16(Solver& S, const PcgDev& c, int check, int grid_b, bool dep)
+template <int B>
+static int launch_cd(Solver& S, const PcgDev& c, bool check, int grid_b, bool dep)
 {
-    const int smem = D_WARPS * D_WARP_BYTES, fine = c.ls[5] / 16;
+    const int fine = c.ls[5] / B, checkers = check ? cd_checkers(c) : 0;
     int resident = 0;
-    STG_TRY(cd16_clusters(&resident));
-    // one resident wave: the coarse cluster, the checker's, and the fine banks' clusters
-    const int room = std::max(1, resident - 1 - check);
-    const int clusters = 1 + check + std::max(1, std::min(div_up(fine, D_WARPS * CD_CL), room));
-    return launch_dep(S, dep, CD_CL, k_phase_cd16, clusters * CD_CL, D_WARPS * 32, smem, c, fine, check, grid_b);
+    STG_TRY(cd_clusters<B>(&resident));
+    // one resident wave: the coarse cluster, the checkers', and the fine banks' clusters
+    const int room = std::max(1, resident - 1 - checkers), per = B == 16 ? D_WARPS * CD_CL : CD_CL;
+    const int clusters = 1 + checkers + std::max(1, std::min(div_up(fine, per), room));
+    return launch_dep(S, dep, CD_CL, B == 16 ? k_phase_cd16 : k_phase_cd32, clusters * CD_CL, D_WARPS * 32,
+                      B == 16 ? D_WARPS * D_WARP_BYTES : D32_SMEM, c, fine, checkers, grid_b);
 }
 
 // Restriction of the coarse levels and the bank solves of every level; check: the fused launch
 // also finishes phase B's r.r over its grid_b partials.  dep: see launch_dep.
 template <int B>
-static int launch_mas_cd(Solver& S, const PcgDev& c, int check, int grid_b, bool dep)
+static int launch_mas_cd(Solver& S, const PcgDev& c, bool check, int grid_b, bool dep)
 {
-    if(B == 16 && fused_cd(S, c)) return launch_cd16(S, c, check, grid_b, dep);
+    if(fused_cd<B>(c)) return launch_cd<B>(S, c, check, grid_b, dep);
     if(c.L > 2)
     {
         const int n1 = (c.ls[2] + 31) / 32 * 32;
@@ -3651,11 +3855,11 @@ static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep
     const int grid_b = std::max(1, std::min(div_up(B > 0 ? c.M : c.nrows, PBB), kSMs * 8));
     // phase B's stop test is finished beside the bank solves when they are fused and nothing in
     // between depends on it
-    const bool finish = B != 16 || !fused_cd(S, c) || c.seg_of_row || repl != REPL_NONE;
+    const bool finish = !fused_cd<B>(c) || repl != REPL_NONE;
     STG_TRY(launch_phase_a<T>(S, c, dep));
     if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_A>, c.nseg, PB, 0, c));
     STG_TRY(launch_dep(S, true, 1, k_phase_b<T, B>, grid_b, PBB, 0, c, finish ? 1 : 0));
-    if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_B>, c.nseg, PB, 0, c));
+    if(c.seg_of_row && finish) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_B>, c.nseg, PB, 0, c));
     if(repl == REPL_IF)
     {
         // IF node: replacement (+ re-restriction) only on replacement iterations
@@ -3689,7 +3893,7 @@ static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep
         }
     }
     const bool after_phase = repl == REPL_NONE;
-    if(B > 0) STG_TRY(launch_mas_cd<(B > 0 ? B : 16)>(S, c, finish ? 0 : 1, grid_b, after_phase));
+    if(B > 0) STG_TRY(launch_mas_cd<(B > 0 ? B : 16)>(S, c, !finish, grid_b, after_phase));
     if(c.net_mode) STG_TRY(launch_learned(S, c));
     STG_TRY(launch_dep(S, (B > 0 || after_phase) && !c.net_mode, 1, k_phase_e<T, B>, c.grid_e, PB, 0, c, (int)POST_BETA));
     if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_E>, c.nseg, PB, 0, c));
@@ -3766,7 +3970,7 @@ static int pcg_run(Solver& S, PcgDev& c)
         k_restrict01<BB><<<row_grid(c.M), PB, 0, s>>>(c, 0);
         STG_LAUNCH_CHECK();
         S.launches++;
-        STG_TRY(launch_mas_cd<BB>(S, c, 0, 0, false));
+        STG_TRY(launch_mas_cd<BB>(S, c, false, 0, false));
         if(c.net_mode) STG_TRY(launch_learned(S, c));
     }
     k_phase_e<T, B><<<c.grid_e, PB, 0, s>>>(c, POST_INIT_RZ);

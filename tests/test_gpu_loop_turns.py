@@ -44,3 +44,30 @@ def test_turns_match_single_iterations(dev, n, bank, precision, refine):
     assert sg["status"] == 0
     r = s.b - orc.spmv(rows, cols, blocks, xg)
     assert np.linalg.norm(r) <= 1.01e-9 * np.linalg.norm(s.b) + 1e-13 * np.linalg.norm(s.b) * dof
+
+
+@pytest.mark.parametrize("precision,refine", [("fp64", 32), ("fp32", 32), ("fp32", 5)])
+@pytest.mark.parametrize("count", [1, 17, 40])
+def test_scene_turns_match_single_iterations(dev, count, precision, refine):
+    """Scenes with their own stop tests (one CTA each beside the bank solves; more than one
+    cluster of them at 17 and 40): graph and host loop end every scene at the same iteration
+    with the same bits, at convergence and when the iteration limit ends the loop first."""
+    import torch
+    from stgipc import PCGSolverConfig, scenes
+    from stgipc.batch import ConcatenatedBatch
+    sysl = scenes.make_batched_cubes(count=count, seed=4300, n_lo=3, n_hi=7)
+    dof = sum(s.n for s in sysl)
+    for ratio in (0.3, 9.5 / dof):
+        got = []
+        for loop in ("graph", "host"):
+            cb = ConcatenatedBatch(sysl, PCGSolverConfig(precision=precision, refine_interval=refine, loop=loop,
+                                                         max_iter_ratio=ratio), device=dev, spmv_tiles=-1)
+            st = cb.solve()
+            torch.cuda.synchronize()
+            it, rel = cb.scene_stats()
+            got.append((st["status"], st["iterations"], it.tolist(), rel.tolist(), cb.x.cpu().numpy()))
+            cb.close()
+        assert got[0][:4] == got[1][:4]
+        np.testing.assert_array_equal(got[0][4], got[1][4])
+        if ratio == 0.3:
+            assert got[0][0] == 0 and max(got[0][3]) <= 1e-4
