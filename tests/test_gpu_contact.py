@@ -117,3 +117,21 @@ def test_energy_matches_oracle(dev):
     # near s = 1 the energy goes as (1 - s^2)^4, so a pair's relative error grows there: the
     # bound is relative to the largest energy of the set
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("P", [1, 31, 32, 33, 63, 65, 200])
+def test_ragged_pair_counts(dev, P):
+    """Pair counts around the warp's 32 staged pairs, every encoding with invalid, repeated and
+    inactive vertices among them, against the oracle (the bars of _compare)."""
+    rng = np.random.default_rng(500 + P)
+    V = 4 * P + 4
+    x = rng.uniform(0, 1, size=(V, 3))
+    pairs = random_contacts(V, P, seed=600 + P, local=8)
+    for q in pairs[: (3 * P) // 4 + 1]:
+        ids = [(-i - 1) if i < 0 else i for i in q]
+        x[ids[1:]] = x[ids[0]] + rng.normal(scale=0.01, size=(3, 3))
+    for k in range(0, P, 9):
+        pairs[k, 1] = V + 5          # out of range
+    for k in range(4, P, 11):
+        pairs[k, 1] = pairs[k, 2] if pairs[k, 2] >= 0 else pairs[k, 1]
+    _compare(pairs, x, 4e-4, 1e5, dev, offset=3)
