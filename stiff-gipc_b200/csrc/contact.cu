@@ -132,9 +132,11 @@ __device__ __forceinline__ void barrier_derivs(double s, double dhat, double kap
          Ic;
 }
 
-// Squared distance and its gradient in closed form.  A cross product's derivative is a triple
-// product, e.g. d(w . (u x v)) = dw . (u x v) + du . (v x w) + dv . (w x u); the first or second
-// vertex takes the negative sum of the others (a translation changes nothing).
+// Squared distance and its gradient: the forward derivative of the formulas of squared_distance
+// with its zeros left out.  A vertex moves the difference vectors u, v, w by su, sv, sw (0 or
+// +-1) times a unit vector e_k, so of n = u x v only the two components beside k change.  Every
+// term and sum is the one that differentiating with all 12 partials forms, in its order, with
+// p2 for the derivative of a square (x' x + x x').
 __device__ __forceinline__ void v_cross(const double* a, const double* b, double* r)
 {
     r[0] = a[1] * b[2] - a[2] * b[1];
@@ -142,44 +144,55 @@ __device__ __forceinline__ void v_cross(const double* a, const double* b, double
     r[2] = a[0] * b[1] - a[1] * b[0];
 }
 __device__ __forceinline__ double v_dot(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+__device__ __forceinline__ double p2(double dx, double x) { return fma(dx, x, dx * x); }
+
+// derivative of the components k + 1 and k + 2 of u x v
+__device__ __forceinline__ void d_cross(const double* u, const double* v, int k, double su, double sv, double& d1, double& d2)
+{
+    const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+    d1 = sv * u[k2] - su * v[k2];
+    d2 = su * v[k1] - sv * u[k1];
+}
 
 __device__ __forceinline__ double distance2_gradient(int type, const double (&x)[4][3], double (&g)[4][3])
 {
     if(type == 0)
     {
-        double d2 = 0.0;
+        double d[3];
 #pragma unroll
         for(int k = 0; k < 3; k++)
         {
-            const double d = x[0][k] - x[1][k];
-            d2 += d * d;
-            g[0][k] = 2.0 * d;
-            g[1][k] = -2.0 * d;
+            d[k] = x[0][k] - x[1][k];
+            g[0][k] = 2.0 * d[k];
+            g[1][k] = -2.0 * d[k];
         }
-        return d2;
+        return v_dot(d, d);
     }
     if(type == 1)
     {
         // |u x v|^2 / |e|^2, u = x1 - x0, v = x2 - x0, e = x2 - x1
-        double u[3], v[3], e[3], n[3], gu[3], gv[3];
+        double u[3], v[3], e[3], n[3];
 #pragma unroll
         for(int k = 0; k < 3; k++) u[k] = x[1][k] - x[0][k], v[k] = x[2][k] - x[0][k], e[k] = x[2][k] - x[1][k];
         v_cross(u, v, n);
-        v_cross(v, n, gu);
-        v_cross(n, u, gv);
-        const double den = v_dot(e, e), d2 = v_dot(n, n) / den, s = 2.0 / den;
+        const double den = v_dot(e, e), q = v_dot(n, n) / den, ib = 1.0 / den;
 #pragma unroll
-        for(int k = 0; k < 3; k++)
-        {
-            g[0][k] = -s * (gu[k] + gv[k]);
-            g[1][k] = s * (gu[k] + d2 * e[k]);
-            g[2][k] = s * (gv[k] - d2 * e[k]);
-        }
-        return d2;
+        for(int m = 0; m < 3; m++)
+#pragma unroll
+            for(int k = 0; k < 3; k++)
+            {
+                const double su = m == 0 ? -1.0 : (m == 1 ? 1.0 : 0.0), sv = m == 0 ? -1.0 : (m == 2 ? 1.0 : 0.0);
+                const double se = m == 1 ? -1.0 : (m == 2 ? 1.0 : 0.0);
+                double d1, d2;
+                d_cross(u, v, k, su, sv, d1, d2);
+                const double dn = p2(d1, n[(k + 1) % 3]) + p2(d2, n[(k + 2) % 3]);
+                g[m][k] = fma(-q, 2.0 * se * e[k], dn) * ib;
+            }
+        return q;
     }
     // (w . n)^2 / |n|^2 with n = u x v: point-triangle u = x2 - x1, v = x3 - x1, w = x0 - x1;
     // edge-edge u = x1 - x0, v = x3 - x2, w = x2 - x0
-    double u[3], v[3], w[3], n[3], vw[3], wu[3], vn[3], nu[3];
+    double u[3], v[3], w[3], n[3];
 #pragma unroll
     for(int k = 0; k < 3; k++)
     {
@@ -188,38 +201,35 @@ __device__ __forceinline__ double distance2_gradient(int type, const double (&x)
         w[k] = type == 2 ? x[0][k] - x[1][k] : x[2][k] - x[0][k];
     }
     v_cross(u, v, n);
-    v_cross(v, w, vw);
-    v_cross(w, u, wu);
-    v_cross(v, n, vn);
-    v_cross(n, u, nu);
-    const double a = v_dot(w, n), den = v_dot(n, n), d2 = a * a / den, s = 2.0 / den;
+    const double a = v_dot(w, n), den = v_dot(n, n), q = a * a / den, ib = 1.0 / den;
 #pragma unroll
-    for(int k = 0; k < 3; k++)
+    for(int m = 0; m < 4; m++)
     {
-        const double gw = s * (a * n[k]), gu = s * (a * vw[k] - d2 * vn[k]), gv = s * (a * wu[k] - d2 * nu[k]);
-        if(type == 2)
+        const double su = type == 2 ? (m == 1 ? -1.0 : (m == 2 ? 1.0 : 0.0)) : (m == 0 ? -1.0 : (m == 1 ? 1.0 : 0.0));
+        const double sv = type == 2 ? (m == 1 ? -1.0 : (m == 3 ? 1.0 : 0.0)) : (m == 2 ? -1.0 : (m == 3 ? 1.0 : 0.0));
+        const double sw = type == 2 ? (m == 0 ? 1.0 : (m == 1 ? -1.0 : 0.0)) : (m == 0 ? -1.0 : (m == 2 ? 1.0 : 0.0));
+#pragma unroll
+        for(int k = 0; k < 3; k++)
         {
-            g[0][k] = gw;
-            g[1][k] = -(gw + gu + gv);
-            g[2][k] = gu;
-            g[3][k] = gv;
-        }
-        else
-        {
-            g[0][k] = -(gw + gu);
-            g[1][k] = gu;
-            g[2][k] = gw - gv;
-            g[3][k] = gv;
+            const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+            double d1, d2, t[3];
+            d_cross(u, v, k, su, sv, d1, d2);
+            t[k] = sw * n[k];
+            t[k1] = __dmul_rn(w[k1], d1);
+            t[k2] = __dmul_rn(w[k2], d2);
+            const double da = t[0] + t[1] + t[2];
+            const double dn = p2(d1, n[k1]) + p2(d2, n[k2]);
+            g[m][k] = fma(-q, dn, p2(da, a)) * ib;
         }
     }
-    return d2;
+    return q;
 }
 
 // One thread per pair.  A warp's 32 pairs' outputs are contiguous (720, 96 and 40 bytes a pair)
 // and pass through shared memory, the blocks five at a time (45 doubles a pair: an odd stride),
 // so that they leave in long runs; written by each thread in place, every store instruction
-// touched 32 sectors for 8 bytes each.  The gradient is closed form: forward differentiation
-// with 13 doubles per intermediate took 122 registers and most of 24.6 us for 30,001 pairs.
+// touched 32 sectors for 8 bytes each.  30,001 pairs (27 MB out) took 24.6 us that way, with a
+// gradient that carried all 12 partials through every operation (122 registers).
 constexpr int CT = 64, CT_ROW = 45;
 
 __global__ void __launch_bounds__(CT) k_contact_barrier(int ncp, const int4* __restrict__ pairs,
@@ -279,9 +289,9 @@ __global__ void __launch_bounds__(CT) k_contact_barrier(int ncp, const int4* __r
             if(s < 1.0 && s > 0.0)
             {
                 barrier_derivs(s, dhat, kappa, e1, lam);
-                const double f = 0.5 / d * rs;  // ds/dx = f dd2/dx
+                const double f = 0.5 / d;  // dd/dx = f dd2/dx
 #pragma unroll
-                for(int k = 0; k < 12; k++) h[k] = f * g[k / 3][k % 3];
+                for(int k = 0; k < 12; k++) h[k] = g[k / 3][k % 3] * f * rs;
             }
         }
         else if(skipped)
