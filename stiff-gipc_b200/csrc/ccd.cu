@@ -8,7 +8,8 @@
 // by the factor eta, or the step reaches 1; the bound is alpha = 1 / max over pairs of 1 / toc.
 // One thread per pair, 50,000 advancement steps at most (the reference's cap).  The largest
 // 1 / toc is taken with an integer atomicMax on its bit pattern (every value is >= 1, and
-// positive doubles order like their bits), so the result does not depend on launch order.
+// positive doubles order like their bits), so the result does not depend on launch order; nor
+// does it with the early stop of accd, which leaves out only steps that cannot raise it.
 // This file is compiled without FMA contraction (build.py): with the operand order of the
 // reference's vector helpers kept, every toc equals the oracle's bit for bit.
 #include "solver.hpp"
@@ -37,29 +38,38 @@ __device__ inline double det_cols(V3 a, V3 b, V3 c)
     return a.x * b.y * c.z + a.y * b.z * c.x + a.z * b.x * c.y - a.z * b.y * c.x - a.x * c.y * b.z - b.x * a.y * c.z;
 }
 
-// parameters of p against edge (a, b) of a triangle with normal n: (along, outward)
-__device__ inline void edge_param(V3 p, V3 a, V3 b, V3 n, double& px, double& py)
+// Parameters of p against edge (a, b) of a triangle with normal n: along = A / D, outward = O / D,
+// with D > 0.  Only their order against 0 and 1 matters, and for D > 0 a rounded quotient is
+// ordered as its operands are (A / D < 1 exactly when A < D: the closest smaller A gives a
+// quotient of at most 1 - 2^-53), so the six divisions of a classification are left out.  A
+// degenerate edge or triangle (D zero, infinite or not a number) divides: along and outward with
+// D = 1.
+struct EdgeParam
+{
+    double A, O, D;
+};
+__device__ inline EdgeParam edge_param(V3 p, V3 a, V3 b, V3 n)
 {
     const V3 b0 = vsub(b, a), b1 = vcross(b0, n), b2 = vsub(p, a);
-    const double D = det_cols(b0, b1, n);
-    px = det_cols(b2, b1, n) / D;
-    py = det_cols(b0, b2, n) / D;
+    const double D = det_cols(b0, b1, n), A = det_cols(b2, b1, n), O = det_cols(b0, b2, n);
+    if(D > 0.0 && D < 1e300) return {A, O, D};
+    if(D < 0.0 && D > -1e300) return {-A, -O, -D};
+    return {A / D, O / D, 1.0};
 }
 
 // closest feature of triangle (t0, t1, t2) to p: 0..2 vertex, 3..5 edge, 6 interior
 __device__ int pt_type(V3 p, V3 t0, V3 t1, V3 t2)
 {
     const V3 n = vcross(vsub(t1, t0), vsub(t2, t0));
-    double x0, y0, x1, y1, x2, y2;
-    edge_param(p, t0, t1, n, x0, y0);
-    if(x0 > 0 && x0 < 1 && y0 >= 0) return 3;
-    edge_param(p, t1, t2, n, x1, y1);
-    if(x1 > 0.0 && x1 < 1.0 && y1 >= 0.0) return 4;
-    edge_param(p, t2, t0, n, x2, y2);
-    if(x2 > 0.0 && x2 < 1.0 && y2 >= 0.0) return 5;
-    if(x0 <= 0.0 && x2 >= 1.0) return 0;
-    if(x1 <= 0.0 && x0 >= 1.0) return 1;
-    if(x2 <= 0.0 && x1 >= 1.0) return 2;
+    const EdgeParam e0 = edge_param(p, t0, t1, n);
+    if(e0.A > 0 && e0.A < e0.D && e0.O >= 0) return 3;
+    const EdgeParam e1 = edge_param(p, t1, t2, n);
+    if(e1.A > 0 && e1.A < e1.D && e1.O >= 0) return 4;
+    const EdgeParam e2 = edge_param(p, t2, t0, n);
+    if(e2.A > 0 && e2.A < e2.D && e2.O >= 0) return 5;
+    if(e0.A <= 0 && e2.A >= e2.D) return 0;
+    if(e1.A <= 0 && e0.A >= e0.D) return 1;
+    if(e2.A <= 0 && e1.A >= e1.D) return 2;
     return 6;
 }
 
@@ -143,8 +153,12 @@ __device__ inline double ee_floor(V3 a0, V3 a1, V3 b0, V3 b1)
     return fmin(fmin(s0, s1), fmin(s2, s3));
 }
 
-// time of impact along d: type 0 point-triangle (v = p, t0, t1, t2), 1 edge-edge
-__device__ double accd(int type, V3* v, V3* d, double eta, double thickness)
+// Time of impact along d: type 0 point-triangle (v = p, t0, t1, t2), 1 edge-edge.
+// bound (may be null): the largest 1 / toc of the pairs so far.  After the first step toc never
+// falls (a step that would shrink it fails the gap test first, as gap > 0), so a pair whose toc
+// has passed 1 / bound cannot change the bound and stops there; its own toc is then not the time
+// of impact, and bound is null when the caller wants those.
+__device__ double accd(int type, V3* v, V3* d, double eta, double thickness, const unsigned long long* bound)
 {
     const double th2 = thickness * thickness;
     V3 mov;
@@ -177,6 +191,9 @@ __device__ double accd(int type, V3* v, V3* d, double eta, double thickness)
     for(int count = 1;; count++)
     {
         if(count > 50000) return toc;
+        // read with the step's arithmetic in flight
+        unsigned long long best = 0ull;
+        if(bound) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(best) : "l"(bound));
         const double lb = (1 - eta) * dF / ((dist + thickness) * mdm);
         for(int i = 0; i < 4; i++) v[i] = vadd(v[i], vmul(d[i], lb));
         if(type == 1)
@@ -191,6 +208,7 @@ __device__ double accd(int type, V3* v, V3* d, double eta, double thickness)
         if(toc != 0.0 && (dF / (dist + thickness) < gap)) break;
         toc += lb;
         if(toc > 1.0) return 1.0;
+        if(gap > 0.0 && toc * __longlong_as_double((long long)best) > 1.0 + 1e-15) return 1.0;
     }
     return toc;
 }
@@ -205,27 +223,37 @@ __global__ void k_ccd_pairs(int np, const int4* __restrict__ pairs, const double
                             unsigned long long* mx, double* toc_out, int* bad)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= np) return;
-    const int4 q = pairs[p];
-    const int id[4] = {q.x < 0 ? -q.x - 1 : q.x, q.y, q.z, q.w};
-    bool ok = true;
-    for(int i = 0; i < 4; i++) ok = ok && id[i] >= 0 && id[i] < nv;
     double toc = 1.0;
-    if(ok)
+    if(p < np)
     {
-        V3 v[4], d[4];
-        for(int i = 0; i < 4; i++)
+        const int4 q = pairs[p];
+        const int id[4] = {q.x < 0 ? -q.x - 1 : q.x, q.y, q.z, q.w};
+        bool ok = true;
+        for(int i = 0; i < 4; i++) ok = ok && id[i] >= 0 && id[i] < nv;
+        if(ok)
         {
-            const size_t o = 3 * (size_t)id[i];
-            v[i] = v3(x[o], x[o + 1], x[o + 2]);
-            d[i] = v3(dx[o], dx[o + 1], dx[o + 2]);
+            V3 v[4], d[4];
+            for(int i = 0; i < 4; i++)
+            {
+                const size_t o = 3 * (size_t)id[i];
+                v[i] = v3(x[o], x[o + 1], x[o + 2]);
+                d[i] = v3(dx[o], dx[o + 1], dx[o + 2]);
+            }
+            toc = accd(q.x < 0 ? 0 : 1, v, d, eta, thickness, toc_out ? nullptr : mx);
         }
-        toc = accd(q.x < 0 ? 0 : 1, v, d, eta, thickness);
-        atomicMax(mx, (unsigned long long)__double_as_longlong(1.0 / toc));
+        else if(bad)
+            atomicAdd(bad, 1);
+        if(toc_out) toc_out[p] = toc;
     }
-    else if(bad)
-        atomicAdd(bad, 1);
-    if(toc_out) toc_out[p] = toc;
+    // one atomic per warp, and only where it can raise the bound: one per pair queued 100,003
+    // atomics on one address
+    unsigned long long m = (unsigned long long)__double_as_longlong(1.0 / toc);
+    for(int o = 16; o > 0; o >>= 1)
+    {
+        const unsigned long long y = __shfl_xor_sync(0xffffffffu, m, o);
+        m = m < y ? y : m;
+    }
+    if((threadIdx.x & 31) == 0 && m > (unsigned long long)__double_as_longlong(1.0)) atomicMax(mx, m);
 }
 
 __global__ void k_ccd_final(const unsigned long long* mx, double* alpha)

@@ -67,3 +67,47 @@ def test_stacked_cubes_pushed_together(dev):
         ids = [(-q[0] - 1) if q[0] < 0 else q[0], q[1], q[2], q[3]]
         d2, _ = orc.contact_d2(2 if q[0] < 0 else 3, moved[ids])
         assert d2 > 0
+
+
+@pytest.mark.parametrize("P", [1, 31, 33, 129, 6000])
+@pytest.mark.parametrize("speed", [0.05, 3.0])
+def test_bound_without_per_pair_times(dev, P, speed):
+    """The bound alone stops pairs that cannot lower it: it equals the bound of the full run and
+    the oracle's, bit for bit, with degenerate pairs (a zero-length edge, a flat triangle, a
+    pair at rest) among them."""
+    from oracle import oracle as orc
+    from stgipc import ccd
+    rng = np.random.default_rng(900 + P)
+    V = 4 * P
+    x = rng.normal(size=(V, 3))
+    dx = rng.normal(size=(V, 3)) * speed
+    v = rng.permutation(V).reshape(P, 4)
+    pairs = np.where((np.arange(P) % 2 == 0)[:, None], np.stack([-v[:, 0] - 1, v[:, 1], v[:, 2], v[:, 3]], 1), v).astype(np.int32)
+    for k in range(5, P, 17):
+        x[v[k, 3]] = 0.5 * (x[v[k, 1]] + x[v[k, 2]])  # collinear triangle / nearby edge
+    for k in range(7, P, 19):
+        dx[v[k]] = 0.0
+    a0 = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev))
+    a1, _ = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev), per_pair=True)
+    want = orc.ccd_step_size(pairs, x, dx, 0.8)
+    # a degenerate pair's time may be no number: the bound then is none either, in both modes
+    np.testing.assert_array_equal(float(a0.item()), float(a1.item()))
+    if np.isfinite(float(a1.item())):
+        assert float(a0.item()) == want
+
+
+@pytest.mark.parametrize("P", [33, 6000])
+def test_bound_of_regular_pairs_without_per_pair_times(dev, P):
+    """As above without degenerate pairs: the bound is a number, set by one pair among many that
+    stop early."""
+    from oracle import oracle as orc
+    from stgipc import ccd
+    rng = np.random.default_rng(950 + P)
+    V = 4 * P
+    x = rng.normal(size=(V, 3))
+    dx = rng.normal(size=(V, 3)) * 0.4
+    v = rng.permutation(V).reshape(P, 4)
+    pairs = np.where((np.arange(P) % 2 == 0)[:, None], np.stack([-v[:, 0] - 1, v[:, 1], v[:, 2], v[:, 3]], 1), v).astype(np.int32)
+    a0 = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev))
+    want = orc.ccd_step_size(pairs, x, dx, 0.8)
+    assert want < 1.0 and float(a0.item()) == want
