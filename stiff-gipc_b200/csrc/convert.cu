@@ -62,7 +62,8 @@ __global__ void k_conv_scatter(const int* rows, const int* cols, int count, int 
 
 // One warp per row: order every entry by (col, original index), write the sorted permutation
 // and sorted cols, and count distinct cols.  Rows of up to 128 entries are sorted by a
-// bitonic network on 64-bit keys (col << 32 | index; 4 keys per lane, position 4 * lane + h);
+// bitonic network on 64-bit keys (col << 32 | index) of 32, 64 or 128 places (a tet mesh's
+// interior rows have about 60 triplets: 42 exchange steps instead of the 128 places' 112);
 // longer rows are listed for k_conv_sort_long, which sorts each with a whole CTA.  The keys
 // are unique, so every path gives the same permutation.
 constexpr int CONV_WARPS = 8;
@@ -72,6 +73,64 @@ __device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v,
     const unsigned lo = __shfl_xor_sync(0xffffffffu, (unsigned)v, m);
     const unsigned hi = __shfl_xor_sync(0xffffffffu, (unsigned)(v >> 32), m);
     return ((unsigned long long)hi << 32) | lo;
+}
+
+// one row of n <= 32 K entries at s: K keys per lane, position K * lane + h
+template <int K>
+__device__ __forceinline__ void sort_row(const int* pcol, const int* perm_in, int* perm_out, int* scol, int s, int n,
+                                         int lane)
+{
+    unsigned long long k[K];
+#pragma unroll
+    for(int h = 0; h < K; h++)
+    {
+        const int p = K * lane + h;
+        k[h] = ~0ull;
+        if(p < n) k[h] = ((unsigned long long)(unsigned)pcol[s + p] << 32) | (unsigned)perm_in[s + p];
+    }
+#pragma unroll
+    for(int kk = 2; kk <= 32 * K; kk <<= 1)
+    {
+#pragma unroll
+        for(int d = kk >> 1; d >= 1; d >>= 1)
+        {
+            if(d >= K)
+            {
+#pragma unroll
+                for(int h = 0; h < K; h++)
+                {
+                    const int p = K * lane + h;
+                    const unsigned long long o = shfl_xor_u64(k[h], d / K);
+                    const bool up = (p & kk) == 0, lower = (p & d) == 0;
+                    k[h] = (up == lower) ? (k[h] < o ? k[h] : o) : (k[h] < o ? o : k[h]);
+                }
+            }
+            else
+            {
+#pragma unroll
+                for(int h = 0; h < K; h++)
+                {
+                    if(h & d) continue;
+                    const int p = K * lane + h;
+                    const bool up = (p & kk) == 0;
+                    const unsigned long long x = k[h], y = k[(h + d) & (K - 1)];
+                    const bool sw = up ? (x > y) : (x < y);
+                    k[h] = sw ? y : x;
+                    k[(h + d) & (K - 1)] = sw ? x : y;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for(int h = 0; h < K; h++)
+    {
+        const int p = K * lane + h;
+        if(p < n)
+        {
+            perm_out[s + p] = (int)(unsigned)k[h];
+            scol[s + p] = (int)(k[h] >> 32);
+        }
+    }
 }
 
 __global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_sort_rows(const int* pcol, const int* row_start,
@@ -84,60 +143,12 @@ __global__ void __launch_bounds__(32 * CONV_WARPS) k_conv_sort_rows(const int* p
     for(int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps)
     {
         const int s = row_start[r], e = row_start[r + 1], n = e - s;
-        if(n <= 128)
-        {
-            unsigned long long k[4];
-#pragma unroll
-            for(int h = 0; h < 4; h++)
-            {
-                const int p = 4 * lane + h;
-                k[h] = ~0ull;
-                if(p < n) k[h] = ((unsigned long long)(unsigned)pcol[s + p] << 32) | (unsigned)perm_in[s + p];
-            }
-#pragma unroll
-            for(int kk = 2; kk <= 128; kk <<= 1)
-            {
-#pragma unroll
-                for(int d = kk >> 1; d >= 1; d >>= 1)
-                {
-                    if(d >= 4)
-                    {
-#pragma unroll
-                        for(int h = 0; h < 4; h++)
-                        {
-                            const int p = 4 * lane + h;
-                            const unsigned long long o = shfl_xor_u64(k[h], d >> 2);
-                            const bool up = (p & kk) == 0, lower = (p & d) == 0;
-                            k[h] = (up == lower) ? (k[h] < o ? k[h] : o) : (k[h] < o ? o : k[h]);
-                        }
-                    }
-                    else
-                    {
-#pragma unroll
-                        for(int h = 0; h < 4; h++)
-                        {
-                            if(h & d) continue;
-                            const int p = 4 * lane + h;
-                            const bool up = (p & kk) == 0;
-                            const unsigned long long x = k[h], y = k[h + d];
-                            const bool sw = up ? (x > y) : (x < y);
-                            k[h] = sw ? y : x;
-                            k[h + d] = sw ? x : y;
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for(int h = 0; h < 4; h++)
-            {
-                const int p = 4 * lane + h;
-                if(p < n)
-                {
-                    perm_out[s + p] = (int)(unsigned)k[h];
-                    scol[s + p] = (int)(k[h] >> 32);
-                }
-            }
-        }
+        if(n <= 32)
+            sort_row<1>(pcol, perm_in, perm_out, scol, s, n, lane);
+        else if(n <= 64)
+            sort_row<2>(pcol, perm_in, perm_out, scol, s, n, lane);
+        else if(n <= 128)
+            sort_row<4>(pcol, perm_in, perm_out, scol, s, n, lane);
         else
         {
             if(lane == 0) long_rows[atomicAdd(long_cnt, 1)] = r;
@@ -228,43 +239,61 @@ __global__ void __launch_bounds__(CONV_LONG_THREADS) k_conv_sort_long(const int*
     }
 }
 
-// One warp per row: each lane owns a run of equal cols (a unique block) and sums it in
-// sorted (= original) order.  Rows of up to CONV_EMIT_CAP entries first stage their blocks
-// (in sorted order) in shared memory with independent loads, so the sequential sums read
-// shared memory; longer rows sum from global memory.  The sums are the same either way.
+// One warp per row: the sum of each run of equal cols (a unique block) in sorted (= original)
+// order.  A row of up to CONV_EMIT_CAP entries stages its blocks in sorted order in shared
+// memory, 32 consecutive values per load instruction (about four 72-byte blocks; a block per
+// lane touched 32 lines per instruction, and those lookups took most of 450 us for 6.75 M
+// triplets), then one lane per value of the unique blocks sums its run and stores it: the
+// row's sums leave contiguously.  Longer rows sum from global memory.  The sums are the same
+// either way.
 constexpr int CONV_EMIT_WARPS = 4;
 constexpr int CONV_EMIT_CAP = 128;
+constexpr int CONV_EMIT_WARP_BYTES = CONV_EMIT_CAP * 72 + 4 * (3 * CONV_EMIT_CAP + 4);
 
-// the fused level-0 pass for unique block o = (r, c) with sum acc (ConvFuse)
-__device__ __forceinline__ void fuse_block(const ConvFuse& F, int r, int c, const double* acc, int o)
+// The fused level-0 pass (ConvFuse) for unique block o = (r, c): its block index in the level-0
+// matrices (-1: not stored there), its level-1 triplet's place written, and how the triplet's
+// block follows from it (coarse_triplet): 0 as is, 1 transposed, 2 plus its transpose, -1 none.
+__device__ __forceinline__ void fuse_place(const ConvFuse& F, int r, int c, int o, int& dst, int& kind)
 {
     const int rr = r - F.offset, cc = c - F.offset;
     const bool in = rr >= 0 && rr < F.V && cc >= 0 && cc < F.V;
     bool lower_in_bank = false;
+    dst = kind = -1;
     if(in)
     {
         const int sc = F.real_map[cc], sr = F.real_map[rr];
         if(sc / F.B == sr / F.B)
         {
             if(sc >= sr)
-            {
-                double* D = F.mat + ((size_t)(sc / F.B) * F.NS + upper_index(F.B, sr % F.B, sc % F.B)) * 9;
-#pragma unroll
-                for(int e = 0; e < 9; e++) D[e] = acc[e];
-            }
+                dst = (sc / F.B) * F.NS + upper_index(F.B, sr % F.B, sc % F.B);
             else
                 lower_in_bank = true;
         }
     }
-    if(F.c1)
+    if(!F.c1) return;
+    if(!in || lower_in_bank)
     {
-        if(!in || lower_in_bank)
-        {
-            F.trow[o] = -1;
-            F.tcol[o] = 0;
-        }
-        else
-            coarse_triplet(rr, cc, F.c1[rr], F.c1[cc], acc, F.trow + o, F.tcol + o, F.tblk + 9 * (size_t)o);
+        F.trow[o] = -1;
+        F.tcol[o] = 0;
+        return;
+    }
+    const int a = F.c1[rr], b = F.c1[cc];
+    kind = a < b || (a == b && rr == cc) ? 0 : (a > b ? 1 : 2);
+    F.trow[o] = min(a, b);
+    F.tcol[o] = max(a, b);
+}
+
+// the same for a whole block held by one lane
+__device__ __forceinline__ void fuse_block(const ConvFuse& F, int r, int c, const double* acc, int o)
+{
+    int dst, kind;
+    fuse_place(F, r, c, o, dst, kind);
+#pragma unroll
+    for(int t = 0; t < 9; t++)
+    {
+        const int tt = (t % 3) * 3 + t / 3;
+        if(dst >= 0) F.mat[9 * (size_t)dst + t] = acc[t];
+        if(kind >= 0) F.tblk[9 * (size_t)o + t] = kind == 0 ? acc[t] : (kind == 1 ? acc[tt] : acc[t] + acc[tt]);
     }
 }
 
@@ -273,24 +302,17 @@ __global__ void __launch_bounds__(32 * CONV_EMIT_WARPS) k_conv_emit(const double
                                                                     const int* ustart, int* out_rows, int* out_cols,
                                                                     double* out_blocks, int nrows, ConvFuse F)
 {
-    extern __shared__ double ebuf[];  // [CONV_EMIT_WARPS][CONV_EMIT_CAP * 9]
+    extern __shared__ __align__(16) unsigned char ebuf[];  // per warp: values, places, cols, run starts
     const int warps = (gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double* sb = ebuf + (size_t)w * CONV_EMIT_CAP * 9;
+    double* sb = reinterpret_cast<double*>(ebuf + (size_t)w * CONV_EMIT_WARP_BYTES);
+    int* sp = reinterpret_cast<int*>(sb + CONV_EMIT_CAP * 9);
+    int* sc = sp + CONV_EMIT_CAP;
+    int* run = sc + CONV_EMIT_CAP;  // [unique + 1]
     for(int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps)
     {
         const int s = row_start[r], e = row_start[r + 1], n = e - s;
         const bool staged = n <= CONV_EMIT_CAP;
-        if(staged)
-        {
-            for(int a = lane; a < n; a += 32)
-            {
-                const double* b0 = blocks + 9 * (size_t)perm[s + a];
-#pragma unroll
-                for(int t = 0; t < 9; t++) sb[9 * a + t] = b0[t];
-            }
-            __syncwarp();
-        }
         if(!staged)
         {
             // a long row: the warp loads 32 entries at a time and every lane accumulates the
@@ -349,32 +371,86 @@ __global__ void __launch_bounds__(32 * CONV_EMIT_WARPS) k_conv_emit(const double
             __syncwarp();
             continue;
         }
-        int base = 0;
+        for(int a = lane; a < n; a += 32)
+        {
+            sp[a] = perm[s + a];
+            sc[a] = scol[s + a];
+        }
+        __syncwarp();
+        for(int i0 = lane; i0 < 9 * n; i0 += 8 * 32)
+        {
+            double v[8];
+#pragma unroll
+            for(int u = 0; u < 8; u++)
+            {
+                const int i = i0 + 32 * u, a = i / 9;
+                if(i < 9 * n) v[u] = blocks[9 * (size_t)sp[a] + (i - 9 * a)];
+            }
+#pragma unroll
+            for(int u = 0; u < 8; u++)
+                if(i0 + 32 * u < 9 * n) sb[i0 + 32 * u] = v[u];
+        }
+        int nu = 0;
         for(int a0 = 0; a0 < n; a0 += 32)
         {
             const int a = a0 + lane;
-            const bool head = a < n && (a == 0 || scol[s + a] != scol[s + a - 1]);
+            const bool head = a < n && (a == 0 || sc[a] != sc[a - 1]);
             const unsigned hm = __ballot_sync(0xffffffffu, head);
-            if(head)
-            {
-                const int o = ustart[r] + base + __popc(hm & lanemask_lt(lane));
-                double acc[9];
-#pragma unroll
-                for(int t = 0; t < 9; t++) acc[t] = sb[9 * a + t];
-                for(int c = a + 1; c < n && scol[s + c] == scol[s + a]; c++)
-                {
-#pragma unroll
-                    for(int t = 0; t < 9; t++) acc[t] += sb[9 * c + t];
-                }
-                out_rows[o] = r;
-                out_cols[o] = scol[s + a];
-#pragma unroll
-                for(int t = 0; t < 9; t++) out_blocks[9 * (size_t)o + t] = acc[t];
-                if(F.B) fuse_block(F, r, scol[s + a], acc, o);
-            }
-            base += __popc(hm);
+            if(head) run[nu + __popc(hm & lanemask_lt(lane))] = a;
+            nu += __popc(hm);
+        }
+        if(lane == 0) run[nu] = n;
+        __syncwarp();
+        const int o0 = n > 0 ? ustart[r] : 0;
+        for(int i = lane; i < 9 * nu; i += 32)
+        {
+            const int q = i / 9, t = i - 9 * q, a0 = run[q], a1 = run[q + 1];
+            double acc = sb[9 * a0 + t];
+            for(int c = a0 + 1; c < a1; c++) acc += sb[9 * c + t];
+            out_blocks[9 * (size_t)o0 + i] = acc;
+            sb[9 * a0 + t] = acc;  // read again by the fused pass
+        }
+        for(int q = lane; q < nu; q += 32)
+        {
+            out_rows[o0 + q] = r;
+            out_cols[o0 + q] = sc[run[q]];
         }
         __syncwarp();
+        if(F.B)
+        {
+            // the fused level-0 pass, a lane per unique block for the places (kept over the
+            // row's staging indices), then a lane per value
+            int* dst = sp;   // level-0 matrix block, or -1
+            int* kind = sc;  // level-1 triplet: 0 as is, 1 transposed, 2 plus its transpose, -1 none
+            for(int q0 = 0; q0 < nu; q0 += 32)
+            {
+                const int q = q0 + lane;
+                int c = 0, a = 0;
+                if(q < nu)
+                {
+                    a = run[q];
+                    c = sc[a];
+                }
+                __syncwarp();  // dst[q] and kind[q] overwrite entries that later q still read: q <= run[q]
+                if(q < nu)
+                {
+                    int d, kd;
+                    fuse_place(F, r, c, o0 + q, d, kd);
+                    dst[q] = d;
+                    kind[q] = kd;
+                }
+                __syncwarp();
+            }
+            for(int i = lane; i < 9 * nu; i += 32)
+            {
+                const int q = i / 9, t = i - 9 * q, tt = (t % 3) * 3 + t / 3;
+                const double* H = sb + 9 * run[q];
+                if(dst[q] >= 0) F.mat[9 * (size_t)dst[q] + t] = H[t];
+                if(kind[q] >= 0)
+                    F.tblk[9 * (size_t)o0 + i] = kind[q] == 0 ? H[t] : (kind[q] == 1 ? H[tt] : H[t] + H[tt]);
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -462,7 +538,7 @@ int convert_into(Solver& S, ConvertScratch& cv, int count, const int* rows, cons
         }
     }
     const int ge = std::min(div_up((long)nrows * 32, 32 * CONV_EMIT_WARPS), kSMs * 32);
-    k_conv_emit<<<ge, 32 * CONV_EMIT_WARPS, sizeof(double) * CONV_EMIT_WARPS * CONV_EMIT_CAP * 9, s>>>(
+    k_conv_emit<<<ge, 32 * CONV_EMIT_WARPS, CONV_EMIT_WARPS * CONV_EMIT_WARP_BYTES, s>>>(
         blocks, cv.row_start.data(), cv.perm2.data(), cv.scol.data(), row_ptr.data(), out_rows.data(), out_cols.data(),
         out_blocks.data(), nrows, F);
     STG_LAUNCH_CHECK();

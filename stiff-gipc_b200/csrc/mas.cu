@@ -814,107 +814,114 @@ __global__ void __launch_bounds__(3 * B) k_mas_invert(const double* __restrict__
     }
 }
 
-// The same Gauss-Jordan for 16-banks, one CTA of 256 threads per bank, thread (bi, bj) owning
-// the 3x3 tile at block row bi, block column bj in registers.  Pivot j: the tiles of block
-// column j / 3 publish column j; those of block row j / 3 scale row j by the reciprocal of
-// the pivot (one FP64 division per thread and pivot: divisions on the pivot's critical path
-// made a per-element division three times slower) and publish it; then every tile updates
-// itself with fma(-colm[k], A[j][i], A[k][i]) as k_mas_invert does.  The broadcasts are
-// double-buffered (two barriers per pivot).  Scaling by the reciprocal instead of dividing
-// changes the last bit of some FP64 entries against the reference's per-element division;
-// k_mas_invert scales the same way, and the CPU oracle (ORC_ORDER_FIXED) restates it.
-__global__ void __launch_bounds__(256) k_mas_invert16(const double* __restrict__ mat, float* inv, int nbanks)
+// The same Gauss-Jordan for 16-banks, one warp per bank: lane (bi, bj) of a 4 x 8 grid holds
+// rows 12 bi .. 12 bi + 11, columns 6 bj .. 6 bj + 5 in registers (72 doubles).  Pivot j: the
+// lanes of its column publish column j, those of its row scale row j by the reciprocal of the
+// pivot and publish it; then every lane updates its tile with fma(-colm[k], A[j][i], A[k][i])
+// as k_mas_invert does: 18 shared-memory reads for 72 FMAs and warp barriers only.  (A CTA of
+// 256 threads per bank with 3x3 tiles read 6 values for 9 FMAs and took two CTA barriers a
+// pivot: 456 us for 8,163 banks, against 50 us of FP64 FMAs.)  Scaling by the reciprocal
+// instead of dividing changes the last bit of some FP64 entries against the reference's
+// per-element division; k_mas_invert scales the same way, and the CPU oracle
+// (ORC_ORDER_FIXED) restates it.
+constexpr int INV_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * INV_WARPS, 2) k_mas_invert16(const double* __restrict__ mat, float* inv, int nbanks)
 {
-    constexpr int B = 16;
+    constexpr int B = 16, TR = 12, TC = 6;
     const int NS = nsym(B);
-    __shared__ double rowj[2][3 * B], colj[2][3 * B];
-    const int bk = blockIdx.x;
-    const int bi = threadIdx.x / B, bj = threadIdx.x % B;
+    __shared__ double rowj[INV_WARPS][2][3 * B], colj[INV_WARPS][2][3 * B];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bk = blockIdx.x * INV_WARPS + w;
+    if(bk >= nbanks) return;
+    const int bi = lane >> 3, bj = lane & 7;
     const double* Mb = mat + (size_t)bk * NS * 9;
-    double a[3][3];
-    if(bj >= bi)
-    {
-        const double* H = Mb + upper_index(B, bi, bj) * 9;  // column-major
+    double a[TR][TC];
 #pragma unroll
-        for(int r = 0; r < 3; r++)
+    for(int p = 0; p < TR / 3; p++)
 #pragma unroll
-            for(int cc = 0; cc < 3; cc++) a[r][cc] = H[cc * 3 + r];
-    }
-    else
-    {
-        const double* H = Mb + upper_index(B, bj, bi) * 9;  // the mirror block, transposed
-#pragma unroll
-        for(int r = 0; r < 3; r++)
-#pragma unroll
-            for(int cc = 0; cc < 3; cc++) a[r][cc] = H[r * 3 + cc];
-    }
-    if(bi == bj)
-    {
-#pragma unroll
-        for(int r = 0; r < 3; r++)
-            if(a[r][r] == 0.0) a[r][r] = 1.0;
-    }
-    for(int j = 0; j < 3 * B; j++)
-    {
-        const int pb = j / 3, pr = j % 3, buf = j & 1;
-        // 1: block column pb publishes the old column j
-        if(bj == pb)
+        for(int q = 0; q < TC / 3; q++)
         {
+            const int rb = 4 * bi + p, cb = 2 * bj + q;
+            const bool up = cb >= rb;  // else the mirror block, transposed
+            const double* H = Mb + upper_index(B, min(rb, cb), max(rb, cb)) * 9;  // column-major
 #pragma unroll
-            for(int r = 0; r < 3; r++) colj[buf][3 * bi + r] = pr == 0 ? a[r][0] : (pr == 1 ? a[r][1] : a[r][2]);
+            for(int r = 0; r < 3; r++)
+#pragma unroll
+                for(int cc = 0; cc < 3; cc++)
+                {
+                    double v = up ? H[cc * 3 + r] : H[r * 3 + cc];
+                    if(r == cc && rb == cb && v == 0.0) v = 1.0;
+                    a[3 * p + r][3 * q + cc] = v;
+                }
         }
-        __syncthreads();
-        // 2: block row pb forms row j after the column replacement (e_j) and the division by
-        // the pivot, keeps it and publishes it
-        if(bi == pb)
-        {
-            const double rinv = 1.0 / colj[buf][j];
+    for(int pb = 0; pb < 4; pb++)
+    {
 #pragma unroll
-            for(int cc = 0; cc < 3; cc++)
+        for(int pr = 0; pr < TR; pr++)
+        {
+            const int j = TR * pb + pr;
+            double* cj = colj[w][pr & 1];
+            double* rj = rowj[w][pr & 1];
+            const bool my_col = bj == 2 * pb + pr / TC, my_row = bi == pb;
+            // 1: the old column j
+            if(my_col)
             {
-                const int col = 3 * bj + cc;
-                const double x = col == j ? 1.0 : (pr == 0 ? a[0][cc] : (pr == 1 ? a[1][cc] : a[2][cc]));
-                const double v = __dmul_rn(x, rinv);
-                rowj[buf][col] = v;
-                if(pr == 0)
-                    a[0][cc] = v;
-                else if(pr == 1)
-                    a[1][cc] = v;
-                else
-                    a[2][cc] = v;
+#pragma unroll
+                for(int k = 0; k < TR; k++) cj[TR * bi + k] = a[k][pr % TC];
             }
-        }
-        __syncthreads();
-        // 3: every other row: A[k][i] = fma(-colm[k], A[j][i], A[k][i]) (column j replaced by e_j)
-#pragma unroll
-        for(int r = 0; r < 3; r++)
-        {
-            const int row = 3 * bi + r;
-            if(row == j) continue;
-            const double cm = colj[buf][row];
-#pragma unroll
-            for(int cc = 0; cc < 3; cc++)
+            __syncwarp();
+            // 2: row j after the column replacement (e_j) and the scaling by the pivot's reciprocal
+            if(my_row)
             {
-                const double old = (3 * bj + cc == j) ? 0.0 : a[r][cc];
-                a[r][cc] = fma(-cm, rowj[buf][3 * bj + cc], old);
+                const double rinv = 1.0 / cj[j];
+#pragma unroll
+                for(int cc = 0; cc < TC; cc++)
+                {
+                    const double x = my_col && cc == pr % TC ? 1.0 : a[pr][cc];
+                    a[pr][cc] = __dmul_rn(x, rinv);
+                    rj[TC * bj + cc] = a[pr][cc];
+                }
             }
+            __syncwarp();
+            // 3: every other row (column j replaced by e_j)
+            double rv[TC];
+#pragma unroll
+            for(int cc = 0; cc < TC; cc++) rv[cc] = rj[TC * bj + cc];
+#pragma unroll
+            for(int k = 0; k < TR; k++)
+            {
+                if(k == pr && my_row) continue;
+                const double cm = cj[TR * bi + k];
+#pragma unroll
+                for(int cc = 0; cc < TC; cc++)
+                {
+                    const double old = my_col && cc == pr % TC ? 0.0 : a[k][cc];
+                    a[k][cc] = fma(-cm, rv[cc], old);
+                }
+            }
+            // the next pivot writes the other buffers; this pivot's are reused two pivots later,
+            // after two more barriers
         }
-        // the next pivot writes the other buffers; this pivot's are reused two pivots later,
-        // after two more barriers
     }
-    if(bj < bi) return;
-    if(bi == bj)
-    {
-        // lower triangle of the diagonal 3x3 block mirrored from the upper one
-        a[1][0] = a[0][1];
-        a[2][1] = a[1][2];
-        a[2][0] = a[0][2];
-    }
-    float* P = inv + ((size_t)bk * NS + upper_index(B, bi, bj)) * 9;
+    float* P = inv + (size_t)bk * NS * 9;
 #pragma unroll
-    for(int r = 0; r < 3; r++)
+    for(int p = 0; p < TR / 3; p++)
 #pragma unroll
-        for(int cc = 0; cc < 3; cc++) P[cc * 3 + r] = (float)a[r][cc];
+        for(int q = 0; q < TC / 3; q++)
+        {
+            const int rb = 4 * bi + p, cb = 2 * bj + q;
+            if(cb < rb) continue;
+            float* D = P + upper_index(B, rb, cb) * 9;
+#pragma unroll
+            for(int r = 0; r < 3; r++)
+#pragma unroll
+                for(int cc = 0; cc < 3; cc++)
+                {
+                    // lower triangle of a diagonal 3x3 block mirrored from the upper one
+                    D[cc * 3 + r] = (float)(rb == cb && r > cc ? a[3 * p + cc][3 * q + r] : a[3 * p + r][3 * q + cc]);
+                }
+        }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1429,7 +1436,7 @@ static int mas_assemble_t(Solver& S, int offset)
     }
     if(B == 16)
     {
-        k_mas_invert16<<<m.nbanks, 256, 0, s>>>(m.mat.data(), m.inv.data(), m.nbanks);
+        k_mas_invert16<<<div_up(m.nbanks, INV_WARPS), 32 * INV_WARPS, 0, s>>>(m.mat.data(), m.inv.data(), m.nbanks);
         STG_LAUNCH_CHECK();
     }
     else

@@ -179,49 +179,57 @@ __device__ __forceinline__ void consume_sum2(const PcgDev& c, int site_a, int co
     rb = tot[1];
 }
 
-// consume_sum2 in two steps, so that the partials' loads can be issued early and other
-// work done while they are in flight: consume2_load fetches this thread's partials (at most
-// K per site; the caller checks K * BLOCK against the counts), consume2_finish sums them in
-// consume_sum2's order (bitwise its result).
-template <int BLOCK, int K>
+// consume_sum2<PB> in two steps by PBB = PB / 2 threads, so that the partials' loads can be
+// issued early and other work done while they are in flight: consume2_load fetches the partials
+// of two of the PB places (at most K rounds of PB; the caller checks K * PB against the counts),
+// consume2_finish sums them in the order of PB threads (bitwise consume_sum2<PB>'s result).
+template <int K>
 __device__ __forceinline__ void consume2_load(const PcgDev& c, int site_a, int count_a, int site_b, int count_b,
-                                              double (&a)[K], double (&b)[K])
+                                              double (&a)[2][K], double (&b)[2][K])
 {
     const double* pa = c.partials + (size_t)site_a * c.slots;
     const double* pb = c.partials + (size_t)site_b * c.slots;
 #pragma unroll
-    for(int k = 0; k < K; k++)
-    {
-        const int t = threadIdx.x + k * BLOCK;
-        a[k] = t < count_a ? __ldcg(pa + t) : 0.0;
-        b[k] = t < count_b ? __ldcg(pb + t) : 0.0;
-    }
+    for(int h = 0; h < 2; h++)
+#pragma unroll
+        for(int k = 0; k < K; k++)
+        {
+            const int t = threadIdx.x + h * PBB + k * PB;
+            a[h][k] = t < count_a ? __ldcg(pa + t) : 0.0;
+            b[h][k] = t < count_b ? __ldcg(pb + t) : 0.0;
+        }
 }
 
-template <int BLOCK, int K>
-__device__ __forceinline__ void consume2_finish(const double (&a)[K], const double (&b)[K], double& ra, double& rb)
+template <int K>
+__device__ __forceinline__ void consume2_finish(const double (&a)[2][K], const double (&b)[2][K], double& ra, double& rb)
 {
-    __shared__ double red[2][BLOCK / 32];
+    static_assert(PB == 2 * PBB, "each thread stands for two");
+    constexpr int W = PB / 32;
+    __shared__ double red[2][W];
     __shared__ double tot[2];
-    double x = 0, y = 0;
-#pragma unroll
-    for(int k = 0; k < K; k++)
-    {
-        x += a[k];
-        y += b[k];
-    }
-    x = warp_sum(x);
-    y = warp_sum(y);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if(lane == 0)
+#pragma unroll
+    for(int h = 0; h < 2; h++)
     {
-        red[0][warp] = x;
-        red[1][warp] = y;
+        double x = 0, y = 0;
+#pragma unroll
+        for(int k = 0; k < K; k++)
+        {
+            x += a[h][k];
+            y += b[h][k];
+        }
+        x = warp_sum(x);
+        y = warp_sum(y);
+        if(lane == 0)
+        {
+            red[0][warp + h * (W / 2)] = x;
+            red[1][warp + h * (W / 2)] = y;
+        }
     }
     __syncthreads();
     if(warp == 0)
     {
-        double u = lane < BLOCK / 32 ? red[0][lane] : 0.0, v = lane < BLOCK / 32 ? red[1][lane] : 0.0;
+        double u = lane < W ? red[0][lane] : 0.0, v = lane < W ? red[1][lane] : 0.0;
         u = warp_sum(u);
         v = warp_sum(v);
         if(lane == 0)
@@ -235,26 +243,6 @@ __device__ __forceinline__ void consume2_finish(const double (&a)[K], const doub
     rb = tot[1];
 }
 
-// ---------------------------------------------------------------------------------------
-// block loads (16-byte vector loads of the padded layouts)
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void load_block(const float* base, size_t k, float h[9])
-{
-    const float4* p = reinterpret_cast<const float4*>(base) + 3 * k;
-    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w;
-    h[4] = b.x; h[5] = b.y; h[6] = b.z; h[7] = b.w;
-    h[8] = c.x;
-}
-
-__device__ __forceinline__ void load_block(const double* base, size_t k, double h[9])
-{
-    const double2* p = reinterpret_cast<const double2*>(base) + 5 * k;
-    const double2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3), e = __ldg(p + 4);
-    h[0] = a.x; h[1] = a.y; h[2] = b.x; h[3] = b.y; h[4] = c.x; h[5] = c.y; h[6] = d.x; h[7] = d.y;
-    h[8] = e.x;
-}
-
 // acc += H x (trans: H^T x); h column-major
 template <typename T>
 __device__ __forceinline__ void mv3(const T h[9], bool trans, T x0, T x1, T x2, T& a0, T& a1, T& a2)
@@ -265,66 +253,6 @@ __device__ __forceinline__ void mv3(const T h[9], bool trans, T x0, T x1, T x2, 
     a0 += h[0] * x0 + h01 * x1 + h02 * x2;
     a1 += h10 * x0 + h[4] * x1 + h12 * x2;
     a2 += h20 * x0 + h21 * x1 + h[8] * x2;
-}
-
-// Row i of A * v with v_j = z_j + beta p_j gathered from the interleaved zp slots (x_plain:
-// a plain [3n] FP64 vector instead, for the residual replacement).  LPR lanes per row,
-// warp-wide shuffles: every lane of the warp must call it.
-template <typename T, int LPR>
-__device__ __forceinline__ void row_spmv_zp(const PcgDev& c, const T* blk, int i, bool valid, int sub, const T* zp,
-                                            T beta, const double* x_plain, T& a0, T& a1, T& a2)
-{
-    a0 = a1 = a2 = T(0);
-    int u0 = 0, nu = 0, t0 = 0, nt = 0;
-    if(valid)
-    {
-        u0 = __ldg(c.row_ptr + i);
-        nu = __ldg(c.row_ptr + i + 1) - u0;
-        t0 = __ldg(c.t_ptr + i);
-        nt = __ldg(c.t_ptr + i + 1) - t0;
-    }
-    for(int e = sub; e < nu + nt; e += LPR)
-    {
-        int k, j;
-        const bool trans = e >= nu;
-        if(!trans)
-        {
-            k = u0 + e;
-            j = __ldg(c.cols + k);
-        }
-        else
-        {
-            const int2 te = __ldg(c.t_ent + t0 + e - nu);
-            k = te.x;
-            j = te.y;
-        }
-        T h[9];
-        load_block(blk, (size_t)k, h);
-        T x0, x1, x2;
-        if(x_plain)
-        {
-            x0 = (T)x_plain[3 * j];
-            x1 = (T)x_plain[3 * j + 1];
-            x2 = (T)x_plain[3 * j + 2];
-        }
-        else
-        {
-            T p0, p1, p2;
-            ld4(zp + 8 * (size_t)j, x0, x1, x2);
-            ld4(zp + 8 * (size_t)j + 4, p0, p1, p2);
-            x0 += beta * p0;
-            x1 += beta * p1;
-            x2 += beta * p2;
-        }
-        mv3<T>(h, trans, x0, x1, x2, a0, a1, a2);
-    }
-#pragma unroll
-    for(int o = LPR / 2; o > 0; o >>= 1)
-    {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-    }
 }
 
 // Row i of A * (z + beta p) on the full symmetric plane copy (untiled phase A).  LPR lanes
@@ -637,19 +565,62 @@ __device__ __forceinline__ double phase_b_plain(const PcgDev& c, int gt, int gn,
     return acc;
 }
 
+// Row i of A x in FP64 from the upper BCOO and its transpose lists, LPR lanes per row (warp-wide
+// shuffles: every lane of the warp must call it).
+template <int LPR>
+__device__ __forceinline__ void row_spmv_x(const PcgDev& c, int i, bool valid, int sub, const double* x, double& a0,
+                                           double& a1, double& a2)
+{
+    a0 = a1 = a2 = 0.0;
+    int u0 = 0, nu = 0, t0 = 0, nt = 0;
+    if(valid)
+    {
+        u0 = __ldg(c.row_ptr + i);
+        nu = __ldg(c.row_ptr + i + 1) - u0;
+        t0 = __ldg(c.t_ptr + i);
+        nt = __ldg(c.t_ptr + i + 1) - t0;
+    }
+    for(int e = sub; e < nu + nt; e += LPR)
+    {
+        int k, j;
+        const bool trans = e >= nu;
+        if(!trans)
+        {
+            k = u0 + e;
+            j = __ldg(c.cols + k);
+        }
+        else
+        {
+            const int2 te = __ldg(c.t_ent + t0 + e - nu);
+            k = te.x;
+            j = te.y;
+        }
+        double h[9];
+#pragma unroll
+        for(int u = 0; u < 9; u++) h[u] = __ldg(c.blk64 + 9 * (size_t)k + u);
+        mv3<double>(h, trans, x[3 * j], x[3 * j + 1], x[3 * j + 2], a0, a1, a2);
+    }
+#pragma unroll
+    for(int o = LPR / 2; o > 0; o >>= 1)
+    {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+}
+
 // residual replacement: r = b - A x with the FP64 blocks; returns the share of r.r
 __device__ __forceinline__ double phase_replace(const PcgDev& c, int gt, int gn)
 {
     constexpr int LPR = 16, RPW = 32 / LPR;
     const int warp = gt >> 5, nwarps = gn >> 5, lane = gt & 31, sub = lane & (LPR - 1);
-    const double* blk = reinterpret_cast<const double*>(c.blk64);
     double acc = 0;
     for(int base = warp * RPW; base < c.nrows; base += nwarps * RPW)
     {
         const int i = base + lane / LPR;
         const bool valid = i < c.nrows;
         double a0, a1, a2;
-        row_spmv_zp<double, LPR>(c, blk, i, valid, sub, nullptr, 0.0, c.x, a0, a1, a2);
+        row_spmv_x<LPR>(c, i, valid, sub, c.x, a0, a1, a2);
         if(valid && sub < 3)
         {
             const int d = 3 * i + sub;
@@ -2834,10 +2805,10 @@ __global__ void __launch_bounds__(PBB, 8) k_phase_b(PcgDev c, int finish)
     if(B > 0) b_load_vecs<T>(c, zpbuf<T>(c, parity_before(c) ^ 1), reinterpret_cast<const T*>(c.q), first);
     // the p.q and r.z partials, in flight with the slot's loads (a grid too large for the
     // registers sums them in consume_sum2 below)
-    constexpr int PK = 5;
-    const bool early = c.grid_a <= PK * PBB && c.grid_e <= PK * PBB;
-    double pa[PK], pe[PK];
-    if(early) consume2_load<PBB, PK>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pa, pe);
+    constexpr int PK = 3;
+    const bool early = c.grid_a <= PK * PB && c.grid_e <= PK * PB;
+    double pa[2][PK], pe[2][PK];
+    if(early) consume2_load<PK>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pa, pe);
     if(done) return;
     // After the upper SpMV, the spilled products of a warp's 32 consecutive rows (Morton
     // order: consecutive slots are consecutive rows) are one contiguous run of slots: the warp
@@ -2868,7 +2839,7 @@ __global__ void __launch_bounds__(PBB, 8) k_phase_b(PcgDev c, int finish)
     }
     double pq, rz;
     if(early)
-        consume2_finish<PBB, PK>(pa, pe, pq, rz);
+        consume2_finish<PK>(pa, pe, pq, rz);
     else
         consume_sum2<PBB>(c, SITE_A, c.grid_a, SITE_E, c.grid_e, pq, rz);
     if(B > 0 && c.spill && c.identity)
@@ -3301,30 +3272,6 @@ __global__ void __launch_bounds__(PB) k_pcg_persistent(PcgDev c)
 // ---------------------------------------------------------------------------------------
 // layout preparation
 // ---------------------------------------------------------------------------------------
-__global__ void k_pack_blocks(const double* __restrict__ src, int nnzb, float* dst32, double* dst64)
-{
-    for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnzb; k += gridDim.x * blockDim.x)
-    {
-        const double* s = src + 9 * (size_t)k;
-        if(dst32)
-        {
-            float4* d = reinterpret_cast<float4*>(dst32) + 3 * (size_t)k;
-            d[0] = make_float4((float)s[0], (float)s[1], (float)s[2], (float)s[3]);
-            d[1] = make_float4((float)s[4], (float)s[5], (float)s[6], (float)s[7]);
-            d[2] = make_float4((float)s[8], 0.f, 0.f, 0.f);
-        }
-        if(dst64)
-        {
-            double2* d = reinterpret_cast<double2*>(dst64) + 5 * (size_t)k;
-            d[0] = make_double2(s[0], s[1]);
-            d[1] = make_double2(s[2], s[3]);
-            d[2] = make_double2(s[4], s[5]);
-            d[3] = make_double2(s[6], s[7]);
-            d[4] = make_double2(s[8], 0.0);
-        }
-    }
-}
-
 // Builds the full symmetric plane copy (FullPlanes) used by the PCG SpMV (phase A): row i
 // holds its lower blocks (transposes of the upper blocks k with col(k) == i, in transpose-
 // list order) followed by its upper blocks.  16 lanes per row, one entry per lane.
@@ -3413,14 +3360,6 @@ int pack_blocks(Solver& S)
     A.upper_built = false;
     if(nnzb < 1) return 0;
     const bool fp32 = S.cfg.precision == STG_PREC_FP32;
-    if(fp32 && S.cfg.refine_interval > 0)  // read by the residual replacement only
-    {
-        STG_TRY(A.blk64p.resize((size_t)nnzb * 10));
-        k_pack_blocks<<<std::max(1, std::min(div_up(nnzb, 256), kSMs * 16)), 256, 0, S.stream>>>(A.B(), nnzb, nullptr,
-                                                                                               A.blk64p.data());
-        STG_LAUNCH_CHECK();
-        S.launches++;
-    }
     // the autotuner times every kernel: both copies; otherwise the copy the chosen kernel reads
     const bool tuning = S.spmv_tune && S.spmv_rt == 0 && S.cfg.loop_mode != STG_LOOP_PERSISTENT;
     const bool need_upper = tuning || upper_spmv_selected(S);
@@ -4249,7 +4188,7 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     c.cols = bcoo.C();
     c.t_ptr = bcoo.t_ptr.data();
     c.t_ent = bcoo.t_ent.data();
-    c.blk64 = reinterpret_cast<const double2*>(bcoo.blk64p.data());
+    c.blk64 = bcoo.B();
     c.fent = bcoo.fent.data();
     c.frow = bcoo.frow.data();
     c.fstride = bcoo.fstride;

@@ -14,7 +14,7 @@ enum : int
 // Everything a phase needs, passed by value.
 struct PcgDev
 {
-    // SpMV structure (padded blocks: FP32 48 B = 3 x float4, FP64 80 B = 5 x double2)
+    // SpMV structure
     const int* row_ptr;
     const int* cols;
     const int* t_ptr;
@@ -35,7 +35,7 @@ struct PcgDev
     size_t ustride;
     void* spill;
     int upper;
-    const double2* blk64;     // FP64 padded upper blocks (residual replacement)
+    const double* blk64;      // FP64 upper blocks (residual replacement)
     int nrows, n;
     // vectors in the iteration precision T, one 4-wide (16 B FP32 / 32 B FP64) slot per block
     // row; z and p of a row share one 32 / 64-byte slot, so that a neighbour gather is one

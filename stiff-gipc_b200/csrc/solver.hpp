@@ -35,7 +35,6 @@ struct Bcoo
     DBuf<int> t_ptr;             // [nrows+1]
     DBuf<int> t_cnt;             // [nrows+1]
     DBuf<int2> t_ent;            // [offdiag]
-    DBuf<double> blk64p;         // FP64 blocks padded to 80 B (5 x double2), residual replacement
     // full symmetric row-sliced copy for the PCG SpMV in 16-byte planes (FullPlanes in
     // spmv_core.cuh, built by k_build_full in pcg.cu)
     DBuf<unsigned char> fent;
