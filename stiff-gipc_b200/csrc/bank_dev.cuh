@@ -17,22 +17,16 @@
 namespace stg
 {
 
-// z += H x (trans: H^T x), one FMA per element in column order
+// z += H x (trans: H^T x), one FMA per element in column order; element (i, k) is
+// H[i * si + k * sk] with (si, sk) = (1, 3), or (3, 1) transposed: strides instead of a branch,
+// whose two sides a warp with both kinds of lanes runs one after the other
 __device__ __forceinline__ void blk_fma3(const float* H, bool trans, float x0, float x1, float x2, float& z0, float& z1,
                                          float& z2)
 {
-    if(trans)
-    {
-        z0 = __fmaf_rn(H[2], x2, __fmaf_rn(H[1], x1, __fmaf_rn(H[0], x0, z0)));
-        z1 = __fmaf_rn(H[5], x2, __fmaf_rn(H[4], x1, __fmaf_rn(H[3], x0, z1)));
-        z2 = __fmaf_rn(H[8], x2, __fmaf_rn(H[7], x1, __fmaf_rn(H[6], x0, z2)));
-    }
-    else
-    {
-        z0 = __fmaf_rn(H[6], x2, __fmaf_rn(H[3], x1, __fmaf_rn(H[0], x0, z0)));
-        z1 = __fmaf_rn(H[7], x2, __fmaf_rn(H[4], x1, __fmaf_rn(H[1], x0, z1)));
-        z2 = __fmaf_rn(H[8], x2, __fmaf_rn(H[5], x1, __fmaf_rn(H[2], x0, z2)));
-    }
+    const int si = trans ? 3 : 1, sk = trans ? 1 : 3;
+    z0 = __fmaf_rn(H[2 * sk], x2, __fmaf_rn(H[sk], x1, __fmaf_rn(H[0], x0, z0)));
+    z1 = __fmaf_rn(H[si + 2 * sk], x2, __fmaf_rn(H[si + sk], x1, __fmaf_rn(H[si], x0, z1)));
+    z2 = __fmaf_rn(H[2 * si + 2 * sk], x2, __fmaf_rn(H[2 * si + sk], x1, __fmaf_rn(H[2 * si], x0, z2)));
 }
 
 // z = H x (trans: H^T x) as fma(P2, x2, fma(P1, x1, P0 x0)) per element; element (i, k) is
