@@ -624,13 +624,33 @@ __global__ void k_mas_extract(const int* __restrict__ rows, const int* __restric
 
 // The coarse levels' aggregation in one launch, from the triplets of the first level that has
 // at most CHAIN_CAP of them: one CTA sorts a level's triplets by (row, col, index) in shared
-// memory, sums every run in that order (one thread per value), writes the level's operator and
-// bank blocks, and maps it to the next level's triplets.  As separate launches a level costs 10
-// launches and a read-back, about 55 us, for a few thousand triplets; 65 us here for
-// three levels from 2,197 triplets.
+// memory (32-bit keys where the level's nodes fit 10 bits), stages three of the nine values of
+// all blocks at a time there, sums every run in that order (one thread per value), writes the
+// level's operator and bank blocks, and maps it to the next level's triplets.  As separate
+// launches a level costs 10 launches and a read-back, about 55 us, for a few thousand triplets;
+// here all three levels from 2,197 triplets take 57 us (65 with 64-bit keys alone and runs summed
+// from device memory).
 // The sums and their order are those of convert_into.
 constexpr int CHAIN_CAP = 4096, CHAIN_T = 1024;
-constexpr int CHAIN_SMEM = CHAIN_CAP * (8 + 2) + 16;
+constexpr int CHAIN_SMEM = CHAIN_CAP * (8 + 2 + 3 * 8) + 16;
+constexpr int CHAIN_NODES32 = 1023;  // nodes that 10-bit rows and columns of a 32-bit key can name
+
+// bitonic sort of P keys (a power of two) in shared memory
+template <typename K>
+__device__ __forceinline__ void chain_sort(K* key, int P)
+{
+    for(int k = 2; k <= P; k <<= 1)
+        for(int j = k >> 1; j > 0; j >>= 1)
+        {
+            for(int t = threadIdx.x; t < P / 2; t += CHAIN_T)
+            {
+                const int a = 2 * t - (t & (j - 1)), b = a + j;  // pairs (a, a ^ j), a & j == 0
+                const K x = key[a], y = key[b];
+                if((x > y) == ((a & k) == 0)) key[a] = y, key[b] = x;
+            }
+            __syncthreads();
+        }
+}
 
 struct ChainArgs
 {
@@ -638,7 +658,7 @@ struct ChainArgs
     int* tr_cols;
     double* tr_blocks;
     int count, level, L;      // triplets of `level`, levels
-    int begin[kMaxLevels + 1];
+    int begin[kMaxLevels + 1], nodes[kMaxLevels + 1];
     const int* going_next;
     int* rows;                // scratch for one level's operator
     int* cols;
@@ -650,7 +670,8 @@ template <int B>
 __global__ void __launch_bounds__(CHAIN_T) k_mas_chain(ChainArgs A)
 {
     extern __shared__ unsigned long long ckey[];
-    unsigned short* ustart = reinterpret_cast<unsigned short*>(ckey + CHAIN_CAP);  // [CHAIN_CAP + 1]
+    double* stage = reinterpret_cast<double*>(ckey + CHAIN_CAP);  // [3 * CHAIN_CAP], first the 32-bit keys
+    unsigned short* ustart = reinterpret_cast<unsigned short*>(stage + 3 * CHAIN_CAP);  // [CHAIN_CAP + 1]
     __shared__ int wcnt[CHAIN_T / 32];
     __shared__ int live;
     const int NS = nsym(B);
@@ -662,31 +683,34 @@ __global__ void __launch_bounds__(CHAIN_T) k_mas_chain(ChainArgs A)
         int P = 1;
         while(P < n) P <<= 1;
         __syncthreads();
+        const bool small = A.nodes[level] <= CHAIN_NODES32;
+        unsigned* k32 = reinterpret_cast<unsigned*>(stage);
         int kept = 0;
         for(int i = tid; i < P; i += CHAIN_T)
         {
-            unsigned long long k = ~0ull;
             const int r = i < n ? __ldcg(A.tr_rows + i) : -1;
-            if(r >= 0)
-            {
-                k = ((unsigned long long)r << 40) | ((unsigned long long)__ldcg(A.tr_cols + i) << 20) | (unsigned)i;
-                kept++;
-            }
-            ckey[i] = k;
+            const unsigned c = r >= 0 ? (unsigned)__ldcg(A.tr_cols + i) : 0u;
+            kept += r >= 0;
+            if(small)
+                k32[i] = r >= 0 ? ((unsigned)r << 22) | (c << 12) | (unsigned)i : ~0u;
+            else
+                ckey[i] = r >= 0 ? ((unsigned long long)r << 40) | ((unsigned long long)c << 20) | (unsigned)i : ~0ull;
         }
         if(kept) atomicAdd(&live, kept);
         __syncthreads();
-        for(int k = 2; k <= P; k <<= 1)
-            for(int j = k >> 1; j > 0; j >>= 1)
+        if(small)
+        {
+            static_assert(CHAIN_CAP <= 4096, "12-bit indices");
+            chain_sort(k32, P);
+            for(int i = tid; i < P; i += CHAIN_T)
             {
-                for(int t = tid; t < P / 2; t += CHAIN_T)
-                {
-                    const int a = 2 * t - (t & (j - 1)), b = a + j;  // pairs (a, a ^ j), a & j == 0
-                    const unsigned long long x = ckey[a], y = ckey[b];
-                    if((x > y) == ((a & k) == 0)) ckey[a] = y, ckey[b] = x;
-                }
-                __syncthreads();
+                const unsigned k = k32[i];
+                ckey[i] = ((unsigned long long)(k >> 22) << 40) | ((unsigned long long)((k >> 12) & 1023u) << 20) | (k & 4095u);
             }
+            __syncthreads();
+        }
+        else
+            chain_sort(ckey, P);
         // run starts: each thread owns a stretch of PT keys, a block scan numbers the runs
         const int m = live, PT = (m + CHAIN_T - 1) / CHAIN_T, i0 = min(m, tid * PT), i1 = min(m, i0 + PT);
         int heads = 0;
@@ -719,27 +743,30 @@ __global__ void __launch_bounds__(CHAIN_T) k_mas_chain(ChainArgs A)
             }
         __syncthreads();
         const int begin = A.begin[level];
-        for(int t = tid; t < 9 * runs; t += CHAIN_T)
+        for(int p = 0; p < 9; p += 3)
         {
-            const int q = t / 9, e = t - 9 * q;
-            const int s0 = ustart[q], s1 = q + 1 < runs ? ustart[q + 1] : m;
-            double acc = __ldcg(A.tr_blocks + 9 * (size_t)((unsigned)ckey[s0] & 0xfffffu) + e);
-            for(int i = s0 + 1; i < s1; i += 16)  // a diagonal block's run holds up to about 100
+            // values p .. p + 2 of every block in sorted order: independent loads, so that the
+            // runs (a diagonal block's holds up to about 100 blocks) sum from shared memory
+#pragma unroll 4
+            for(int t = tid; t < 3 * m; t += CHAIN_T)
             {
-                double v[16];
-#pragma unroll
-                for(int z = 0; z < 16; z++)
-                    if(i + z < s1) v[z] = __ldcg(A.tr_blocks + 9 * (size_t)((unsigned)ckey[i + z] & 0xfffffu) + e);
-#pragma unroll
-                for(int z = 0; z < 16; z++)
-                    if(i + z < s1) acc += v[z];
+                const int i = t / 3;
+                stage[t] = __ldcg(A.tr_blocks + 9 * (size_t)((unsigned)ckey[i] & 0xfffffu) + p + (t - 3 * i));
             }
-            A.blocks[t] = acc;
-            const int ga = begin + (int)(ckey[s0] >> 40), gb = begin + ((int)(ckey[s0] >> 20) & 0xfffff);
-            if(ga / B == gb / B) A.mat[((size_t)(ga / B) * NS + upper_index(B, ga % B, gb % B)) * 9 + e] = acc;
+            __syncthreads();
+            for(int t = tid; t < 3 * runs; t += CHAIN_T)
+            {
+                const int q = t / 3, e = t - 3 * q;
+                const int s0 = ustart[q], s1 = q + 1 < runs ? ustart[q + 1] : m;
+                double acc = stage[3 * s0 + e];
+                for(int i = s0 + 1; i < s1; i++) acc += stage[3 * i + e];
+                A.blocks[9 * (size_t)q + p + e] = acc;
+                const int ga = begin + (int)(ckey[s0] >> 40), gb = begin + ((int)(ckey[s0] >> 20) & 0xfffff);
+                if(ga / B == gb / B) A.mat[((size_t)(ga / B) * NS + upper_index(B, ga % B, gb % B)) * 9 + p + e] = acc;
+            }
+            __syncthreads();
         }
         if(level + 1 >= A.L || runs == 0) return;
-        __syncthreads();
         const int next = A.begin[level + 1];
         for(int i = tid; i < runs; i += CHAIN_T)
         {
@@ -1366,9 +1393,9 @@ static int mas_assemble_t(Solver& S, int offset)
             STG_TRY(m.ga_rows.resize(std::max<size_t>(m.ga_rows.size, count)));
             STG_TRY(m.ga_cols.resize(std::max<size_t>(m.ga_cols.size, count)));
             STG_TRY(m.ga_blocks.resize(std::max<size_t>(m.ga_blocks.size, 9 * (size_t)count)));
-            ChainArgs A{m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(), count, level, m.L, {}, m.going_next.data(),
+            ChainArgs A{m.tr_rows.data(), m.tr_cols.data(), m.tr_blocks.data(), count, level, m.L, {}, {}, m.going_next.data(),
                         m.ga_rows.data(), m.ga_cols.data(), m.ga_blocks.data(), m.mat.data()};
-            for(int l = 0; l <= m.L; l++) A.begin[l] = m.level_size[2 * l + 1];
+            for(int l = 0; l <= m.L; l++) A.begin[l] = m.level_size[2 * l + 1], A.nodes[l] = m.level_size[2 * l];
             static thread_local unsigned long long seen = 0;
             if(first_on_device(seen))
                 STG_CUDA_TRY(cudaFuncSetAttribute(k_mas_chain<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SMEM));

@@ -200,6 +200,37 @@ def test_mas_matrices_and_inverse(dev, bank):
     assert np.array_equal(gi, ei)
 
 
+@pytest.mark.parametrize("V,count", [(1023, 4096), (1024, 4096), (1024, 4097), (1500, 4095), (17, 40)])
+@pytest.mark.parametrize("bank", [16, 32])
+def test_mas_small_levels_bit_exact(dev, bank, V, count):
+    """Levels whose triplets one CTA aggregates: at most 4,096 triplets, with 32-bit keys up to
+    1,023 nodes.  Couplings across banks only keep every vertex a node of its own at each level;
+    the smallest case couples inside banks too and merges."""
+    from oracle import oracle as orc
+    from stgipc import scenes
+    rng = np.random.default_rng(70 + V + count)
+    iu = np.stack(np.triu_indices(V, 1), 1)
+    far = iu[iu[:, 0] // bank != iu[:, 1] // bank] if V > bank + 1 else iu
+    pick = far[np.sort(rng.choice(len(far), size=min(count - V, len(far)), replace=False))]
+    rows = np.concatenate([np.arange(V), pick[:, 0]]).astype(np.int32)
+    cols = np.concatenate([np.arange(V), pick[:, 1]]).astype(np.int32)
+    bl = rng.standard_normal((rows.size, 3, 3))
+    bl[:V] = np.eye(3) * 20.0 * count / V + 0.5 * (bl[:V] + bl[:V].transpose(0, 2, 1))
+    r, c, bl = orc.convert(rows, cols, bl.reshape(-1, 9))
+    ns, nn, nl = scenes.edge_neighbors(V, pick)
+    pm, rm = scenes.mas_partition_morton(V, bank)
+    om = orc.Mas(bank, V, ns, nn, nl, pm, rm)
+    om.build(None)
+    om.assemble(r, c, bl)
+    solver = _solver(bank_size=bank)
+    solver.mas_init(V, ns, nn, nl, pm, rm)
+    solver.mas_assemble(_t(bl.reshape(-1), dev), _t(r, dev), _t(c, dev), r.size, 0, None)
+    em, ei = om.matrices()
+    gm, gi = solver.export_matrices()
+    assert om.L > 1
+    assert np.array_equal(gm, em) and np.array_equal(gi, ei)
+
+
 @pytest.mark.parametrize("bank", [16, 32])
 def test_mas_apply(dev, bank):
     s = cube_system(16)
