@@ -1149,6 +1149,25 @@ __device__ __forceinline__ void cd_restrict(const PcgDev& c, int rank, const Mem
     }
 }
 
+// One thread's part of a scene's sum, src[i] for i = i0, i0 + PB, ... < r1, in that order from
+// zero; U loads are issued before their adds.  A scene has one CTA, so the round trips of its
+// rows are the launch.  With the loads left to the compiler a solve of 48 scenes of up to 2,197
+// rows took 3.49 ms against 3.23, of 256 scenes of up to 15,625 rows 50.5 ms against 48.9.
+template <int U>
+__device__ __forceinline__ double scene_sum(const double* src, int i0, int r1)
+{
+    double a = 0.0;
+    for(; i0 < r1; i0 += U * PB)
+    {
+        double v[U];
+#pragma unroll
+        for(int u = 0; u < U; u++) v[u] = i0 + u * PB < r1 ? __ldcg(src + i0 + u * PB) : 0.0;
+#pragma unroll
+        for(int u = 0; u < U; u++) a += v[u];
+    }
+    return a;
+}
+
 // Phase B's r.r and the stop test, by one CTA of the last cluster (128 threads, in the order of
 // phase B's finish_reduction); with scenes, one CTA per scene (the last `checkers` clusters)
 // first runs the scene's test as k_seg<SEG_B> does, and the last of them to finish goes on.
@@ -1168,9 +1187,9 @@ __device__ __forceinline__ void cd_check(const PcgDev& c, int grid_b, int checke
         if(id >= c.nseg) return;
         const int r0 = c.seg_row_off[id], r1 = c.seg_row_off[id + 1];
         const double* src = c.seg_row + (size_t)c.nrows;
-        double v0 = 0, v1 = 0;  // threads t and t + 128 of k_seg's 256
-        for(int i = r0 + (int)threadIdx.x; i < r1; i += PB) v0 += __ldcg(src + i);
-        for(int i = r0 + (int)threadIdx.x + PB / 2; i < r1; i += PB) v1 += __ldcg(src + i);
+        // threads t and t + 128 of k_seg's 256
+        double v0 = scene_sum<16>(src, r0 + (int)threadIdx.x, r1);
+        double v1 = scene_sum<16>(src, r0 + (int)threadIdx.x + PB / 2, r1);
         v0 = warp_sum(v0);
         v1 = warp_sum(v1);
         if(lane == 0)
@@ -3070,14 +3089,17 @@ __global__ void __launch_bounds__(PB) k_seg(PcgDev c)
     __shared__ double red[PB / 32];
     __shared__ bool last;
     grid_dep_release();
-    grid_dep_wait();
-    if(MODE != SEG_INIT && __ldcg(c.flags + F_DONE)) return;
     const int sc = blockIdx.x;
-    const int r0 = c.seg_row_off[sc], r1 = c.seg_row_off[sc + 1];
+    const int r0 = __ldg(c.seg_row_off + sc), r1 = __ldg(c.seg_row_off + sc + 1);
     double* S = c.seg + SEG_N * (size_t)sc;
     const double* src = c.seg_row + (size_t)(MODE == SEG_A ? 0 : (MODE == SEG_B ? 1 : 2)) * c.nrows;
-    double v = 0, bb = 0;
-    for(int i = r0 + threadIdx.x; i < r1; i += PB) v += __ldcg(src + i);
+    grid_dep_wait();
+    const int stop = MODE != SEG_INIT ? __ldcg(c.flags + F_DONE) : 0;
+    // what thread 0 needs beside the sum, read in the same round trip
+    const double rz0 = MODE != SEG_INIT ? __ldcg(S + SG_RZ) : 0.0;
+    const double done = MODE != SEG_INIT ? __ldcg(S + SG_DONE) : 0.0;
+    double v = scene_sum<16>(src, r0 + (int)threadIdx.x, r1), bb = 0;
+    if(stop) return;
     if(MODE == SEG_INIT)
         for(int i = 3 * r0 + threadIdx.x; i < 3 * r1; i += PB) bb += c.b[i] * c.b[i];
     v = block_sum<PB>(v, red);
@@ -3098,9 +3120,9 @@ __global__ void __launch_bounds__(PB) k_seg(PcgDev c)
         {
             S[SG_PQ] = v;
             // a scene whose p.q is not positive stops (no update), the others go on
-            const bool go = S[SG_DONE] == 0.0 && v > 0.0 && isfinite(v);
-            S[SG_ALPHA] = go ? S[SG_RZ] / v : 0.0;
-            if(!go && S[SG_DONE] == 0.0)
+            const bool go = done == 0.0 && v > 0.0 && isfinite(v);
+            S[SG_ALPHA] = go ? rz0 / v : 0.0;
+            if(!go && done == 0.0)
             {
                 S[SG_DONE] = 1.0;
                 S[SG_ITER] = __ldcg(c.scal + SS_ITER);
@@ -3108,13 +3130,13 @@ __global__ void __launch_bounds__(PB) k_seg(PcgDev c)
         }
         else if(MODE == SEG_E)
         {
-            if(S[SG_DONE] == 0.0) S[SG_BETA] = S[SG_RZ] != 0.0 ? v / S[SG_RZ] : 0.0;
+            if(done == 0.0) S[SG_BETA] = rz0 != 0.0 ? v / rz0 : 0.0;
             S[SG_RZ] = v;
         }
         else
         {
             S[SG_RR] = v;
-            if(S[SG_DONE] == 0.0 && v <= c.seg_tol2 * S[SG_BB])
+            if(done == 0.0 && v <= c.seg_tol2 * S[SG_BB])
             {
                 S[SG_DONE] = 1.0;
                 S[SG_ITER] = __ldcg(c.scal + SS_ITER);
