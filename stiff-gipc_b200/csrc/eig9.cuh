@@ -1,5 +1,5 @@
-// eig9.cuh -- eigen-decomposition of a symmetric 9x9 matrix on the device (FP64), shared by
-// the PSD projections of the tet Hessian (fem.cu) and the affine-body shape Hessian (abd.cu).
+// eig9.cuh -- eigen-decomposition of a symmetric 9x9 matrix on the device (FP64), for the PSD
+// projection of the affine-body shape Hessian (abd.cu).
 #pragma once
 
 namespace stg

@@ -10,7 +10,6 @@
 // alpha = 1 + mu / lam, whose 9x9 Hessian in F is projected to PSD by clamping negative
 // eigenvalues), and the reference's plane barrier on the squared distance.
 #include "solver.hpp"
-#include "eig9.cuh"
 
 namespace stg
 {

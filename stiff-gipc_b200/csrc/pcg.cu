@@ -16,8 +16,10 @@
 //      (p is double-buffered, so the p update costs no pass), p.q -> alpha
 //   B  x += alpha p; r -= alpha q per MAS level-0 bank, restricting r to level 0 and summing
 //      each level-0 component into level 1 in the same pass; r.r -> stop test
-//   C  restriction of levels >= 2 from level 1 (one CTA, level by level)
+//   C  restriction of levels >= 2 from level 1
 //   D  bank solves z_b = P_b r_b for every bank of every level
+//      (one launch for C, D and B's stop test where the coarse levels fit one cluster:
+//      k_phase_cd16 / cd32; separate launches otherwise and with the learned correction)
 //   E  prolongation z = sum_l P_l z_l (+ ABD 12x12 block-Jacobi), r.z -> beta
 // (non-MAS preconditioners: B is a plain axpy, C/D vanish, E applies block-Jacobi/identity).
 // Every reduction is finished by the last CTA in a fixed order (deterministic).  In FP32 mode
@@ -26,9 +28,10 @@
 //
 // Three drivers share these phases:
 //   LOOP_HOST   one launch per phase, a flag read after every iteration;
-//   LOOP_GRAPH  the iteration is captured once as the body of a device-side WHILE node of a
-//               CUDA graph (the replacement as an IF node); one graph launch runs the whole
-//               solve, the loop condition is set by the stop test on the device;
+//   LOOP_GRAPH  a turn of up to 8 iterations is captured once as the body of a device-side
+//               WHILE node of a CUDA graph (the replacement as an IF node at its end); one
+//               graph launch runs the whole solve, the loop condition is set by the stop test
+//               on the device, and the iterations of a turn after it leave at their first read;
 //   LOOP_PERSISTENT  one cooperative kernel runs all iterations; phases are separated by a
 //               bounded grid barrier that also finishes the reductions.
 #include "solver.hpp"
