@@ -37,7 +37,8 @@ __device__ __forceinline__ double dot3(const double (&a)[3], const double (&b)[3
     return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 
-// c, s of the rotation that diagonalises [[app, apq], [apq, aqq]]
+// c, s of the rotation that diagonalises [[app, apq], [apq, aqq]]; apq * apq > 0 (where it
+// vanishes in 64 bits, d * d may too, and t is no tangent)
 __device__ __forceinline__ void jacobi_cs(double app, double aqq, double apq, double& c, double& s, double& t)
 {
     const double d = aqq - app, w = 2.0 * apq;
@@ -110,9 +111,28 @@ __device__ __forceinline__ void svd3(const double (&F)[3][3], double (&U)[3][3],
             n1 = n2;
         n2 = nn;
     }
+    // A column below 1e-100 of the other counts as zero: it changes nothing, but its direction is
+    // not one of the orthogonal basis (svd_rotate's squares vanish before such a column is
+    // orthogonal, and a lone column may stand in either place).  A rank of one leaves it first.
+    if(n0 < 1e-200 * n1)
+    {
+#pragma unroll
+        for(int i = 0; i < 3; i++)
+        {
+            const double x = A[0][i], v = V[0][i];
+            A[0][i] = A[1][i];
+            A[1][i] = -x;
+            V[0][i] = V[1][i];
+            V[1][i] = -v;
+        }
+        const double nn = n0;
+        n0 = n1;
+        n1 = nn;
+    }
     sv[0] = sqrt(n0);
     sv[1] = sqrt(n1);
-    const double i0 = sv[0] > 0.0 ? 1.0 / sv[0] : 0.0, i1 = sv[1] > 0.0 ? 1.0 / sv[1] : 0.0;
+    const bool has0 = n0 > 0.0, has1 = n1 > 1e-200 * n0;
+    const double i0 = has0 ? 1.0 / sv[0] : 0.0, i1 = has1 ? 1.0 / sv[1] : 0.0;
 #pragma unroll
     for(int i = 0; i < 3; i++)
     {
@@ -120,8 +140,8 @@ __device__ __forceinline__ void svd3(const double (&F)[3][3], double (&U)[3][3],
         U[1][i] = A[1][i] * i1;
     }
     // a rank below two leaves u_0 or u_1 free: any orthonormal completion
-    if(!(sv[0] > 0.0)) U[0][0] = 1.0;
-    if(!(sv[1] > 0.0))
+    if(!has0) U[0][0] = 1.0;
+    if(!has1)
     {
         const bool ax = fabs(U[0][0]) < 0.6;  // an axis away from u_0, made orthogonal to it
         const double e[3] = {ax ? 1.0 : 0.0, ax ? 0.0 : 1.0, 0.0};
@@ -306,7 +326,7 @@ __global__ void __launch_bounds__(FT, 3) k_fem_tet(const double* __restrict__ re
             {
                 const int p = pq == 2 ? 1 : 0, q = pq == 0 ? 1 : 2, o = 3 - p - q;
                 const double apq = M[p][q];
-                if(!(fabs(apq) > 0.0)) continue;
+                if(!(apq * apq > 0.0)) continue;
                 double c, s, tt;
                 jacobi_cs(M[p][p], M[q][q], apq, c, s, tt);
                 M[p][p] -= tt * apq;

@@ -95,3 +95,53 @@ def test_closed_form_projection_on_hard_tets(dev, T):
     scale = np.abs(np.linalg.det(Dm)) / 6.0 * 1e-4 * d2 * h
     assert (np.abs(got - ref).max(axis=1) <= 1e-12 * scale).all()
     np.testing.assert_allclose(b.cpu().numpy(), cpu.b, atol=1e-12 * T * np.abs(cpu.b).max())
+
+
+def _degenerate_gradients():
+    """Deformation gradients of rank zero to two with the non-zero columns in every place, and
+    with columns whose squares vanish in 64 bits."""
+    a, b = np.array([0.6, 0.7, -0.5]), np.array([-0.3, 1.1, 0.4])
+    out = [np.zeros((3, 3))]
+    for c in range(3):
+        for s in (1.0, 2.5):
+            F = np.zeros((3, 3))
+            F[:, c] = s * a
+            out.append(F)                       # rank one, the other columns exactly zero
+            for tiny in (1e-100, 1e-160, 1e-170):
+                G = F.copy()
+                G[:, (c + 1) % 3] = tiny * a    # parallel to the lone column
+                out.append(G)
+                G = G.copy()
+                G[:, (c + 2) % 3] = 0.5 * tiny * b
+                out.append(G)
+        for tiny in (0.0, 1e-120, 1e-168):
+            F = np.stack([a, b, a - 2.0 * b], 1)
+            F[:, c] = tiny
+            out.append(F)                       # rank two
+    out += [np.diag([s, s, q]) for s in (1.0, 2.0) for q in (1e-150, 1e-172, 1e-200)]
+    out += [q * np.eye(3) for q in (1e-60, 1e-150, 1e-200)]
+    return np.stack(out)
+
+
+def test_closed_form_projection_of_degenerate_gradients(dev):
+    """Against numpy's eigh, as above, on unit rest tets (F is exact): 1e-12 of the unprojected
+    Hessian's bound, and no NaN where eigh has none."""
+    from stgipc import fem, scenes
+    F = _degenerate_gradients()
+    T = F.shape[0]
+    rest = np.tile(np.concatenate([np.zeros((1, 3)), np.eye(3)]), (T, 1))
+    tets = np.arange(4 * T).reshape(T, 4)
+    pos = np.zeros_like(rest)
+    for t in range(T):
+        pos[tets[t, 1:]] = F[t].T
+    E = np.full(T, 1e5)
+    cpu = scenes._assemble(name="degenerate", pos_rest=rest, pos=pos, vel=np.zeros_like(pos), tets=tets, E=E, nu=0.45,
+                           rho=1000.0, dt=0.01, barriers=[])
+    _, _, blocks, b = fem.newton_system(rest, pos, np.zeros_like(pos), tets, E, 0.45, 1000.0, 0.01, device=dev)
+    got = blocks.cpu().numpy()[:10 * T].reshape(T, 90)
+    ref = cpu.blocks[:10 * T].reshape(T, 90)
+    mu, lam = 1e5 / 2.9, 1e5 * 0.45 / (1.45 * 0.1)
+    f = np.linalg.norm(F, axis=(1, 2))
+    scale = 1e-4 / 6.0 * 12.0 * (mu + lam * f ** 4 + lam * (f ** 3 + 2.0) * f)
+    assert (np.abs(got - ref).max(axis=1) <= 1e-12 * scale).all()
+    np.testing.assert_allclose(b.cpu().numpy(), cpu.b, atol=1e-12 * T * np.abs(cpu.b).max())
