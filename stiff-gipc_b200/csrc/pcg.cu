@@ -70,7 +70,8 @@ enum Site : int
     SITE_E = 3,
     SITE_INIT = 4,
     SITE_INIT_RZ = 5,
-    SITE_F = 6  // r_(k+1).z_k of phase E (flexible PCG)
+    SITE_F = 6,  // r_(k+1).z_k of phase E (flexible PCG)
+    SITE_SEG = 7 // the scenes' r.r sums (cd_check)
 };
 // last-CTA counters (PcgDev::counters): one per reduction site finished by its producer,
 // plus the scenes' stop test (k_seg<SEG_B>)
@@ -1173,14 +1174,19 @@ __device__ __forceinline__ double scene_sum(const double* src, int i0, int r1)
 
 // Phase B's r.r and the stop test, by one CTA of the last cluster (128 threads, in the order of
 // phase B's finish_reduction); with scenes, one CTA per scene (the last `checkers` clusters)
-// first runs the scene's test as k_seg<SEG_B> does, and the last of them to finish goes on.
+// first forms the scene's sum as k_seg<SEG_B> does, and the last of them to finish goes on.  The
+// scenes' own tests follow the test of the whole system and are left out when that ends the loop
+// (a breakdown, the iteration limit), as with the separate launches: after a breakdown phase B
+// has left no r.r.
 __device__ __forceinline__ void cd_check(const PcgDev& c, int grid_b, int checkers)
 {
     static_assert(PBB == D_WARPS * 32, "the checker sums as phase B's finish_reduction does");
     __shared__ double red[8];
-    __shared__ bool last;
+    __shared__ bool last, go;
+    __shared__ double iter;
     const int id = (int)blockIdx.x - ((int)gridDim.x - checkers * CD_CL);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double* const sums = c.partials + (size_t)SITE_SEG * c.slots;
     if(!c.seg_of_row)
     {
         if(id != 0) return;
@@ -1204,19 +1210,7 @@ __device__ __forceinline__ void cd_check(const PcgDev& c, int grid_b, int checke
         const double v = warp == 0 ? warp_sum(lane < 8 ? red[lane] : 0.0) : 0.0;
         if(threadIdx.x == 0)
         {
-            // the iteration that just ended; at the iteration limit the loop ends before the
-            // scenes' test, as with the separate launches
-            const long k = (long)__ldcg(c.scal + SS_ITER) + 1;
-            double* S = c.seg + SEG_N * (size_t)id;
-            if(k + 1 < c.prm.max_iter)
-            {
-                S[SG_RR] = v;
-                if(S[SG_DONE] == 0.0 && v <= c.seg_tol2 * S[SG_BB])
-                {
-                    S[SG_DONE] = 1.0;
-                    S[SG_ITER] = (double)k;
-                }
-            }
+            sums[id] = v;
             __threadfence();
             last = atomicAdd(c.counters + CNT_SEG, 1u) == (unsigned)(c.nseg - 1);
         }
@@ -1224,23 +1218,48 @@ __device__ __forceinline__ void cd_check(const PcgDev& c, int grid_b, int checke
         if(!last) return;
         __threadfence();
     }
+    // what the tests need beside the sum, read in the same round trip
+    const double pq = __ldcg(c.scal + SS_PQ_B), rz = __ldcg(c.scal + SS_RZ_B);
+    const int done = __ldcg(c.flags + F_DONE);
+    double rr = 0.0, bb = 0.0, closed = 1.0;
+    auto load_scene = [&](int q) {
+        rr = __ldcg(sums + q);
+        bb = __ldcg(c.seg + SEG_N * (size_t)q + SG_BB);
+        closed = __ldcg(c.seg + SEG_N * (size_t)q + SG_DONE);
+    };
+    if(c.seg_of_row && (int)threadIdx.x < c.nseg) load_scene(threadIdx.x);
     const double tot = block_sum<PBB>(strided_sum<PBB>(c.partials + (size_t)SITE_B * c.slots, grid_b), red);
-    double open = 0;
+    if(threadIdx.x == 0)
+    {
+        if(c.seg_of_row) c.counters[CNT_SEG] = 0u;
+        if(!done) post_op(POST_CHECK_PQ, 0, tot, c.scal, c.flags, c.prm, pq, rz);
+        iter = c.scal[SS_ITER];
+        go = !done && !c.flags[F_DONE];
+    }
     if(c.seg_of_row)
     {
-        for(int q = threadIdx.x; q < c.nseg; q += PBB) open += __ldcg(c.seg + SEG_N * (size_t)q + SG_DONE) == 0.0 ? 1.0 : 0.0;
-        open = block_sum<PBB>(open, red);
+        __syncthreads();
+        bool open = !go;
+        for(int q = threadIdx.x; q < c.nseg && go; q += PBB)
+        {
+            if(q != (int)threadIdx.x) load_scene(q);
+            double* S = c.seg + SEG_N * (size_t)q;
+            S[SG_RR] = rr;
+            if(closed == 0.0 && rr <= c.seg_tol2 * bb)
+            {
+                closed = 1.0;
+                S[SG_DONE] = 1.0;
+                S[SG_ITER] = iter;
+            }
+            open = open || closed == 0.0;
+        }
+        if(!__syncthreads_or(open) && threadIdx.x == 0)
+        {
+            c.flags[F_DONE] = 1;
+            c.flags[F_STATUS] = 0;
+        }
     }
-    if(threadIdx.x != 0) return;
-    if(c.seg_of_row) c.counters[CNT_SEG] = 0u;
-    if(__ldcg(c.flags + F_DONE)) return;
-    post_op(POST_CHECK_PQ, 0, tot, c.scal, c.flags, c.prm, __ldcg(c.scal + SS_PQ_B), __ldcg(c.scal + SS_RZ_B));
-    if(c.seg_of_row && open == 0.0 && !c.flags[F_DONE])
-    {
-        c.flags[F_DONE] = 1;
-        c.flags[F_STATUS] = 0;
-    }
-    set_conditionals(c, POST_CHECK);
+    if(threadIdx.x == 0 && !done) set_conditionals(c, POST_CHECK);
 }
 
 // bank bk's inverse into a stage; the barrier expects it plus `extra` bytes

@@ -112,3 +112,35 @@ def test_per_scene_recurrences_match_each_scene_alone(dev):
         tol = 1e-7 if int(its[k]) == se["iterations"] else 1e-5
         assert np.linalg.norm(x - xe) <= tol * np.linalg.norm(xe), (k, np.linalg.norm(x - xe) / np.linalg.norm(xe))
     cb.close()
+
+
+@pytest.mark.parametrize("precision,refine,loop", [("fp64", 32, "graph"), ("fp64", 32, "host"), ("fp32", 0, "graph"),
+                                                   ("fp32", 32, "graph"), ("fp32", 32, "host")])
+def test_breakdown_leaves_every_scene_open(dev, precision, refine, loop):
+    """A NaN in one scene's Hessian ends the whole loop in its first iteration, before any scene
+    was updated: no scene may be reported as converged, also not on a handle whose previous solve
+    left small residuals behind, and with the scenes' tests beside the bank solves or after phase
+    B (the loops with residual replacement).  Then a clean solve again gives the first one's bits."""
+    from stgipc import PCGSolverConfig, StgError, _lib, scenes
+    from stgipc.batch import ConcatenatedBatch
+    sysl = scenes.make_batched_cubes(count=20, seed=1011, n_lo=3, n_hi=6)
+    cb = ConcatenatedBatch(sysl, PCGSolverConfig(precision=precision, refine_interval=refine, loop=loop), device=dev,
+                           spmv_tiles=-1)
+    assert cb.solve()["status"] == 0
+    first = cb.x.cpu().numpy()
+    its, rels = cb.scene_stats()
+    assert (its > 0).all() and (rels <= 1e-4).all()
+    keep = cb.blocks.clone()
+    cb.blocks[9 * (sysl[0].rows.size + 3) + 4] = float("nan")  # a block of the second scene
+    with pytest.raises(StgError) as e:
+        cb.solve()
+    assert e.value.status == _lib.STG_BREAKDOWN
+    bad, rel = cb.scene_stats()
+    assert (bad == 0).all()
+    np.testing.assert_array_equal(rel, 1.0)
+    cb.blocks.copy_(keep)
+    assert cb.solve()["status"] == 0
+    again, _ = cb.scene_stats()
+    assert again.tolist() == its.tolist()
+    np.testing.assert_array_equal(cb.x.cpu().numpy(), first)
+    cb.close()
