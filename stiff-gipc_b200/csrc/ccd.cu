@@ -41,19 +41,23 @@ __device__ inline double det_cols(V3 a, V3 b, V3 c)
 // Parameters of p against edge (a, b) of a triangle with normal n: along = A / D, outward = O / D,
 // with D > 0.  Only their order against 0 and 1 matters, and for D > 0 a rounded quotient is
 // ordered as its operands are (A / D < 1 exactly when A < D: the closest smaller A gives a
-// quotient of at most 1 - 2^-53), so the six divisions of a classification are left out.  A
-// degenerate edge or triangle (D zero, infinite or not a number) divides: along and outward with
-// D = 1.
+// quotient of at most 1 - 2^-53) unless a quotient underflows to zero, so the six divisions of a
+// classification are left out where none can (1e-210 / 1e90).  A degenerate edge or triangle (D
+// zero, infinite or not a number) and numerators next to zero divide: along and outward with D = 1.
 struct EdgeParam
 {
     double A, O, D;
 };
+__device__ inline bool quotient_keeps_sign(double x) { return x == 0.0 || fabs(x) >= 1e-210; }
 __device__ inline EdgeParam edge_param(V3 p, V3 a, V3 b, V3 n)
 {
     const V3 b0 = vsub(b, a), b1 = vcross(b0, n), b2 = vsub(p, a);
     const double D = det_cols(b0, b1, n), A = det_cols(b2, b1, n), O = det_cols(b0, b2, n);
-    if(D > 0.0 && D < 1e300) return {A, O, D};
-    if(D < 0.0 && D > -1e300) return {-A, -O, -D};
+    if(fabs(D) < 1e90 && quotient_keeps_sign(A) && quotient_keeps_sign(O))
+    {
+        if(D > 0.0) return {A, O, D};
+        if(D < 0.0) return {-A, -O, -D};
+    }
     return {A / D, O / D, 1.0};
 }
 

@@ -111,3 +111,45 @@ def test_bound_of_regular_pairs_without_per_pair_times(dev, P):
     a0 = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev))
     want = orc.ccd_step_size(pairs, x, dx, 0.8)
     assert want < 1.0 and float(a0.item()) == want
+
+
+def test_classification_next_to_underflow(dev):
+    """Subnormal and zero coordinates beside large ones: the quotients that place the point in a
+    region of the triangle underflow.  Every time of impact is the oracle's, bit for bit."""
+    from oracle import oracle as orc
+    from stgipc import ccd
+    h = float.fromhex
+    # found by a search on the CPU: the region chosen without dividing gives another last bit
+    found = [
+        ("0x0p+0 0x0p+0 0x1.536119194736ep+26 0x1.d62b5c7f9c398p+26 0x1.12f5cba6da9f4p+26 -0x0.00000001055a4p-1022 "
+         "-0x1.c2522d19258afp+26 -0x1.bf1cd3e951092p+25 0x0p+0 -0x1.1db744f9c0e2ep-1017 -0x1.8f7d4407fc278p-1015 0x0p+0",
+         "0x1.1c5361f67dadp+24 0x1.5accfc352095ap+26 -0x1.be6d88d96e42ap+25 -0x1.e08c3d13edbfp+25 0x1.9871b9d4ce89ap+26 "
+         "0x1.0491bb7f53174p+26 -0x1.a53667fa657a8p+24 -0x1.53015329351f6p+26 -0x1.8f7a6c1772636p+26 "
+         "-0x1.0371156b4b71ap+26 -0x1.4b1368e11cf9ap+26 -0x1.f280d7dc23b1cp+26"),
+        ("-0x1.3745845814d7cp+13 0x0p+0 0x1.ba7f5e2e178cp+10 -0x1.da073ebf869e4p+13 -0x1.feb33c6ce785p+11 0x0p+0 "
+         "-0x1.d8783aa66f839p+14 0x0p+0 -0x0.0000000002ba5p-1022 0x1.e3116e021be88p+14 -0x0.0000000000a3dp-1022 0x0p+0",
+         "0x1.e0d51acdf25f8p+14 -0x1.5f82edbc1e0f4p+14 -0x1.c9e65fa49ebdap+14 -0x1.531534e258a7ep+14 "
+         "-0x1.a9be98639fe7ep+13 -0x1.a7e2d9a6acdp+8 0x1.bb5d2de8785bcp+14 -0x1.df7aa65601c94p+14 "
+         "-0x1.f04f0f5f0be0dp+14 -0x1.ebf75a5675a9ep+13 0x1.a8bebac0b611p+12 0x1.bcae483989e32p+14"),
+        ("0x0p+0 -0x1.5aaa78ee37598p+17 0x1.481f5fdf0300cp+17 0x0p+0 -0x1.6ca2a2186838p+18 0x1.5aea495a6dp+16 "
+         "-0x0.0000000000005p-1022 0x0p+0 0x0p+0 0x1.437e12a9e23bp+17 0x0p+0 0x0p+0",
+         "0x1.4e675605506bcp+18 -0x1.185c601fa23e8p+18 -0x1.1bd37f3fef346p+17 0x1.280fe1bee2b58p+18 "
+         "-0x1.1180049e13b12p+18 -0x1.93dfc7410e808p+18 0x1.812eb28fbeb06p+18 -0x1.11b36b5b9a48p+18 "
+         "0x1.f5d76cc7a3b42p+18 -0x1.1b94e4b443d6p+14 0x1.8fdbd937bba36p+18 0x1.7d318503b5a44p+17"),
+    ]
+    rng = np.random.default_rng(31)
+    P = 2000
+    s = 2.0 ** rng.integers(0, 30, (P, 1, 1))
+    x = rng.uniform(-1, 1, (P, 4, 3)) * s
+    kind = rng.integers(0, 6, x.shape)
+    x = np.where(kind == 0, 0.0, np.where(kind == 1, np.ldexp(rng.uniform(-1, 1, x.shape), -rng.integers(1000, 1074, x.shape)), x))
+    dx = rng.uniform(-1, 1, x.shape) * s
+    for k, (a, b) in enumerate(found):
+        x[k] = np.array([h(v) for v in a.split()]).reshape(4, 3)
+        dx[k] = np.array([h(v) for v in b.split()]).reshape(4, 3)
+    q = np.arange(4 * P).reshape(P, 4)
+    pairs = np.concatenate([-q[:, :1] - 1, q[:, 1:]], 1).astype(np.int32)
+    _, toc = ccd.step_size(_t(pairs, dev), _t(x.reshape(-1, 3), dev), _t(dx.reshape(-1, 3), dev), per_pair=True)
+    want = np.array([orc.accd(0, x[k], dx[k], 0.2) for k in range(P)])
+    assert (want < 1).sum() > 100
+    np.testing.assert_array_equal(toc.cpu().numpy(), want)
