@@ -158,10 +158,11 @@ __device__ inline double ee_floor(V3 a0, V3 a1, V3 b0, V3 b1)
 }
 
 // Time of impact along d: type 0 point-triangle (v = p, t0, t1, t2), 1 edge-edge.
-// bound (may be null): the largest 1 / toc of the pairs so far.  After the first step toc never
-// falls (a step that would shrink it fails the gap test first, as gap > 0), so a pair whose toc
-// has passed 1 / bound cannot change the bound and stops there; its own toc is then not the time
-// of impact, and bound is null when the caller wants those.
+// bound (may be null): the largest 1 / toc of the pairs so far.  From a step that leaves room of
+// at least gap > 0, toc never falls: the next step is positive, and a later one is only added
+// after it has left such room too (the first step is not tested for it).  So a pair whose toc has
+// passed 1 / bound there cannot change the bound and stops; its own toc is then not the time of
+// impact, and bound is null when the caller wants those.
 __device__ double accd(int type, V3* v, V3* d, double eta, double thickness, const unsigned long long* bound)
 {
     const double th2 = thickness * thickness;
@@ -209,10 +210,11 @@ __device__ double accd(int type, V3* v, V3* d, double eta, double thickness, con
         else
             dist2 = pt_dist2(v[0], v[1], v[2], v[3]), dF = dist2 - th2;
         dist = sqrt(dist2);
-        if(toc != 0.0 && (dF / (dist + thickness) < gap)) break;
+        const double room = dF / (dist + thickness);
+        if(toc != 0.0 && room < gap) break;
         toc += lb;
         if(toc > 1.0) return 1.0;
-        if(gap > 0.0 && toc * __longlong_as_double((long long)best) > 1.0 + 1e-15) return 1.0;
+        if(gap > 0.0 && room >= gap && toc * __longlong_as_double((long long)best) > 1.0 + 1e-15) return 1.0;
     }
     return toc;
 }

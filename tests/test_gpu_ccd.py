@@ -153,3 +153,43 @@ def test_classification_next_to_underflow(dev):
     want = np.array([orc.accd(0, x[k], dx[k], 0.2) for k in range(P)])
     assert (want < 1).sum() > 100
     np.testing.assert_array_equal(toc.cpu().numpy(), want)
+
+
+def test_early_stop_keeps_a_time_that_falls(dev):
+    """A slackness next to one and a thickness: the first step ends within a rounding of the
+    thickness, and the second one goes back.  The pair that sets the bound is past the others'
+    time after its first step and below it in the end; it comes after them, so that it meets their
+    bound.  The bound is the oracle's, with the times and without."""
+    from oracle import oracle as orc
+    from stgipc import ccd
+    h = float.fromhex
+    slack, th = 1.0 - 1e-12, 0.5
+    # point and triangle, the point's displacement in the pair that sets the bound and in the others
+    found = [
+        ("0x1.03a5df59f6e6fp-6 -0x1.bfd1f6dccf2e6p-2 0x1.1d11d915932bbp-1 -0x1.e29c51510804ep-1 -0x1.3fef8b51c108cp+0 "
+         "0x1.c63f39c94d5bfp-4 0x1.199e8bc1bc4cdp+0 -0x1.019070fb51829p+0 0x1.c70f9635479ecp-5 -0x1.2540078b74c22p-3 "
+         "0x1.c3bbbe8eea62fp-1 0x1.696bf7f700514p-8",
+         "-0x1.7ce055b124f2bp-26 -0x1.60ba1b06998a8p-25 -0x1.0c249cb28c20bp-20",
+         "-0x1.7ce0559e5baa3p-26 -0x1.60ba1af533b24p-25 -0x1.0c249ca55250cp-20"),
+        ("0x1.bfb3ca553c5a5p-4 -0x1.cfa6ada15f8c6p-2 0x1.867454d9b1ccbp-2 -0x1.94f7edd5177a2p-1 -0x1.47f3005fd4947p+0 "
+         "-0x1.107d9489b7119p-3 0x1.406dc319d65ccp+0 -0x1.a09316ac167a7p-1 -0x1.693d087185b49p-4 -0x1.8c83cf89f68adp-4 "
+         "0x1.721c96f949d1ep-1 -0x1.1327b71e80effp-3",
+         "0x1.9c69d6f5e3846p-26 -0x1.3404365981961p-27 -0x1.0c58e94e25651p-20",
+         "0x1.9c69d6e194047p-26 -0x1.3404364a56454p-27 -0x1.0c58e940ee353p-20"),
+    ]
+    for v, last, others in found:
+        x1 = np.array([h(a) for a in v.split()]).reshape(4, 3)
+        x = np.concatenate([x1, x1])
+        dx = np.zeros((8, 3))
+        dx[0], dx[4] = [h(a) for a in others.split()], [h(a) for a in last.split()]
+        t0, t1 = (orc.accd(0, x[4 * k:4 * k + 4], dx[4 * k:4 * k + 4], 1.0 - slack, th) for k in (0, 1))
+        assert t1 < t0 < 1.0
+        pairs = np.tile(np.array([[-1, 1, 2, 3]], np.int32), (1000000, 1))  # several waves of CTAs
+        pairs[-40:] = [-5, 5, 6, 7]
+        p = _t(pairs, dev)
+        a = ccd.step_size(p, _t(x, dev), _t(dx, dev), slackness=slack, thickness=th)
+        b, toc = ccd.step_size(p, _t(x, dev), _t(dx, dev), slackness=slack, thickness=th, per_pair=True)
+        assert float(toc[0]) == t0 and float(toc[-1]) == t1
+        want = 1.0 / (1.0 / t1)
+        assert float(b.item()) == want
+        assert float(a.item()) == want
