@@ -211,6 +211,13 @@ int stg_profile_spmv(stg_handle h, int reps, float* avg_ms, double* bytes);
  * the device stays usable.  Returns STG_OK when the diagnostic ran. */
 int stg_selftest_wait_timeout(int* status, double* seconds);
 
+/* Diagnostic (no counterpart in the reference): the handle's next solves in the host or graph
+ * loop end in PCG iteration `iteration` (1 to 10000; 0: off) as if a bounded wait had given up
+ * there: in the SpMV phase (site 0) or in the bank solves (site 1).  Nothing waits: a kernel
+ * records the error.  The solve must return STG_ERR_TIMEOUT; if the loop went on past it, the
+ * same kernel ends it after a few more iterations and the solve returns STG_ERR_CUDA. */
+int stg_selftest_fail_iteration(stg_handle h, int iteration, int site);
+
 /* ---- Morton keys ----------------------------------------------------------------------- */
 /* Replaces _calcVertMChash (StiffGIPC/GIPC.cu:453-502) with hash_code type -1 and expand_bits
  * (GIPC.cu:183-208): keys[i] = (code << 32) | i, code the 30-bit interleave (x << 2 | y << 1 | z)

@@ -477,6 +477,19 @@ extern "C" int stg_selftest_wait_timeout(int* status, double* seconds)
     })
 }
 
+extern "C" int stg_selftest_fail_iteration(stg_handle h, int iteration, int site)
+{
+    CHECK_HANDLE(h);
+    if(iteration < 0 || iteration > 10000 || site < 0 || site > 1)
+    {
+        stg::set_error("stg_selftest_fail_iteration: iteration must be 0 to 10000, site 0 or 1");
+        return STG_ERR_INVALID;
+    }
+    h->fail_iter = iteration;
+    h->fail_site = site;
+    return STG_OK;
+}
+
 extern "C" int stg_profile_spmv(stg_handle h, int reps, float* avg_ms, double* bytes)
 {
     CHECK_HANDLE(h);

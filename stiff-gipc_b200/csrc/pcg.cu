@@ -75,7 +75,7 @@ enum Site : int
 };
 // last-CTA counters (PcgDev::counters): one per reduction site finished by its producer,
 // plus the scenes' stop test (k_seg<SEG_B>)
-constexpr int CNT_SEG = 6;
+constexpr int CNT_SEG = 6, CNT_SELFTEST = 8;
 
 // ---------------------------------------------------------------------------------------
 // reductions: last CTA finishes, optionally drives the graph's conditional nodes
@@ -3060,7 +3060,13 @@ __global__ void __launch_bounds__(PB, 4) k_phase_e(PcgDev c, int op)
     const double v = B > 0 ? phase_e_mas<T>(c, GT, GN, maps, done != 0) : phase_e_plain<T>(c, GT, GN, done != 0);
     if(done)
     {
-        if(GT == 0) c.flags[F_STOP] = 1;
+        if(GT == 0)
+        {
+            c.flags[F_STOP] = 1;
+            // also where a bounded wait gave up, before the stop test (which then left the loop's
+            // condition as it was) or after it: every iteration ends here
+            if(c.use_cond) cudaGraphSetConditional(c.h_while, 0u);
+        }
         return;
     }
     if(op == POST_INIT_RZ)
@@ -3523,6 +3529,28 @@ int selftest_wait(int* status, double* seconds)
     return 0;
 }
 
+// stg_selftest_fail_iteration: marks the solve as a bounded wait that gave up does, in place of
+// such a wait, in the given iteration.  iters_done: iterations that the stop test has counted when
+// this runs.  Where the loop went on past that iteration's turn (at most 8 iterations), the run
+// of this kernel that finds it ends the loop with another status, so that it always ends.
+__global__ void k_selftest_fail(PcgDev c, int iters_done)
+{
+    if(c.flags[F_DONE])
+    {
+        if(++c.counters[CNT_SELFTEST] > 16u)
+        {
+            c.flags[F_STATUS] = 2;  // STG_ERR_CUDA
+            if(c.use_cond) cudaGraphSetConditional(c.h_while, 0u);
+        }
+        return;
+    }
+    if((int)c.scal[SS_ITER] == iters_done)
+    {
+        c.flags[F_STATUS] = 6;  // STG_ERR_TIMEOUT
+        c.flags[F_DONE] = 1;
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // host driver
 // ---------------------------------------------------------------------------------------
@@ -3834,6 +3862,7 @@ static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep
     // between depends on it
     const bool finish = !fused_cd<B>(c) || repl != REPL_NONE;
     STG_TRY(launch_phase_a<T>(S, c, dep));
+    if(S.fail_iter > 0 && S.fail_site == 0) STG_TRY(launch_dep(S, false, 1, k_selftest_fail, 1, 1, 0, c, S.fail_iter - 1));
     if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_A>, c.nseg, PB, 0, c));
     STG_TRY(launch_dep(S, true, 1, k_phase_b<T, B>, grid_b, PBB, 0, c, finish ? 1 : 0));
     if(c.seg_of_row && finish) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_B>, c.nseg, PB, 0, c));
@@ -3872,6 +3901,7 @@ static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep
     const bool after_phase = repl == REPL_NONE;
     if(B > 0) STG_TRY(launch_mas_cd<(B > 0 ? B : 16)>(S, c, !finish, grid_b, after_phase));
     if(c.net_mode) STG_TRY(launch_learned(S, c));
+    if(S.fail_iter > 0 && S.fail_site == 1) STG_TRY(launch_dep(S, false, 1, k_selftest_fail, 1, 1, 0, c, S.fail_iter));
     STG_TRY(launch_dep(S, (B > 0 || after_phase) && !c.net_mode, 1, k_phase_e<T, B>, c.grid_e, PB, 0, c, (int)POST_BETA));
     if(c.seg_of_row) STG_TRY(launch_dep(S, true, 1, k_seg<SEG_E>, c.nseg, PB, 0, c));
     return 0;
@@ -3988,7 +4018,7 @@ static int pcg_run(Solver& S, PcgDev& c)
         key.h_while = 0;
         key.h_if = 0;
         key.use_cond = 0;
-        const int variant = (int)sizeof(T) * 1000 + B;
+        const int variant = (int)sizeof(T) * 1000 + B + 10000 * (2 * S.fail_iter + S.fail_site);
         if(P.graph && P.graph_variant == variant && std::memcmp(&key, &P.graph_key, sizeof(key)) == 0)
         {
             c.h_while = P.graph_dev.h_while;
@@ -4418,7 +4448,7 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     const int* h_flags = h.flags;
     const long max_iter = c.prm.max_iter;
     int status = h_flags[F_DONE] ? h_flags[F_STATUS] : STG_MAX_ITER;
-    if(status == STG_ERR_TIMEOUT) set_error("persistent PCG: a grid barrier wait gave up");
+    if(status == STG_ERR_TIMEOUT) set_error("PCG: a bounded device wait gave up");
     const long iters = max_iter <= 1 ? 1 : (long)h_scal[S_ITER];
     if(cfg.loop_mode == STG_LOOP_GRAPH && max_iter > 1)
     {

@@ -203,6 +203,7 @@ struct Solver
     bool spmv_tune = false;
     int tuned_rt = 0, tuned_prec = -1, tuned_nrows = -1, tuned_nnzb = -1;
     float tune_us[4] = {0.f, 0.f, 0.f, 0.f};
+    int fail_iter = 0, fail_site = 0;  // stg_selftest_fail_iteration
 
     ~Solver();
 

@@ -100,6 +100,7 @@ def lib():
     L.stg_spmv_noalloc.argtypes = [cd, vp, vp, vp, ci, vp, cd, vp, ci, vp]
     L.stg_morton_keys.argtypes = [ci, vp, vp, vp]
     L.stg_selftest_wait_timeout.argtypes = [C.POINTER(ci), C.POINTER(cd)]
+    L.stg_selftest_fail_iteration.argtypes = [vp, ci, ci]
     L.stg_spmv_tiles.argtypes = [vp, ci]
     L.stg_set_segments.argtypes = [vp, vp, ci]
     L.stg_segment_stats.argtypes = [vp, vp, vp]
