@@ -1604,13 +1604,14 @@ __device__ __forceinline__ void lds_main(unsigned sb, int f, double h[9])
 
 // a row's whole zp slot {z0 z1 z2 -, p0 p1 p2 -} in one 32-byte load (FP32) or two (FP64)
 // (sm_100 256-bit vector loads; the slots are 32- / 64-byte aligned): a neighbour gather is
-// one L1 wavefront per lane instead of two (FP32) or four (FP64)
+// one L1 wavefront per lane instead of two (FP32) or four (FP64).  Volatile: other kernels write
+// the slots, and nothing else keeps these loads behind grid_dep_wait()
 __device__ __forceinline__ void ld_zp(const float* a, float& z0, float& z1, float& z2, float& p0, float& p1, float& p2)
 {
     float w0, w1;
-    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(z0), "=f"(z1), "=f"(z2), "=f"(w0), "=f"(p0), "=f"(p1), "=f"(p2), "=f"(w1)
-        : "l"(a));
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(z0), "=f"(z1), "=f"(z2), "=f"(w0), "=f"(p0), "=f"(p1), "=f"(p2), "=f"(w1)
+                 : "l"(a));
     (void)w0;
     (void)w1;
 }
@@ -1618,8 +1619,8 @@ __device__ __forceinline__ void ld_zp(const double* a, double& z0, double& z1, d
                                       double& p2)
 {
     double w0, w1;
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(z0), "=d"(z1), "=d"(z2), "=d"(w0) : "l"(a));
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(p0), "=d"(p1), "=d"(p2), "=d"(w1) : "l"(a + 4));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(z0), "=d"(z1), "=d"(z2), "=d"(w0) : "l"(a));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(p0), "=d"(p1), "=d"(p2), "=d"(w1) : "l"(a + 4));
     (void)w0;
     (void)w1;
 }
