@@ -3803,7 +3803,6 @@ static int tune_phase_a(Solver& S, PcgDev c, float* us, int* out)
         float ms = 0.f;
         STG_CUDA_TRY(cudaEventElapsedTime(&ms, S.ev[4], S.ev[5]));
         us[v] = 1e3f * ms / reps;
-        S.launches += 3 + reps;
         if(v == 0 || us[v] < best)
         {
             best = us[v];
@@ -4094,7 +4093,8 @@ static int pcg_run(Solver& S, PcgDev& c)
             }
             if(rc == 0 && S.pending_if_body) rc = record_if_body<T, B>(S, c, grid_rows, S.pending_if_body);
             S.stream = user;
-            S.launches_per_batch = (S.launches - l0) / unroll;
+            S.launches_per_turn = S.launches - l0;
+            S.turn_iters = unroll;
             S.launches = l0;
             if(rc) break;
             cudaError_t ie = cudaGraphInstantiate(&P.graph, g, 0);
@@ -4193,7 +4193,7 @@ int profile_spmv(Solver& S, int reps, float* avg_ms, double* bytes)
         STG_CUDA_TRY(cudaEventElapsedTime(&ms, S.ev[4], S.ev[5]));
         total += ms;
     }
-    S.launches += 2 * reps + 3;
+    S.launches += reps;  // the scrubs; launch_phase_a counts itself
     STG_CUDA_TRY(cudaMemcpyAsync(c.flags, saved, sizeof(saved), cudaMemcpyHostToDevice, s));
     STG_CUDA_TRY(cudaStreamSynchronize(s));
     if(avg_ms) *avg_ms = (float)(total / std::max(reps, 1));
@@ -4453,9 +4453,13 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     const long iters = max_iter <= 1 ? 1 : (long)h_scal[S_ITER];
     if(cfg.loop_mode == STG_LOOP_GRAPH && max_iter > 1)
     {
-        // the graph's body ran once per iteration; its IF node (residual replacement plus
-        // the level-0/1 re-restriction) once per replacement
-        launches += (int)iters * launches_per_batch + h_flags[F_REPL] * (use_mas ? 2 : 1);
+        // the graph's body ran once per turn of turn_iters iterations, whole turns also where the
+        // solve ended within one; its IF node (residual replacement plus the level-0/1
+        // re-restriction) once per replacement.  The iteration limit counts one iteration that
+        // does not run; one that breaks down before its update, or gives up, is not counted.
+        const bool cut = status == STG_ERR_TIMEOUT || (status == STG_BREAKDOWN && !(h_scal[S_PQ] > 0.0 && std::isfinite(h_scal[S_PQ])));
+        const long ran = iters + (cut ? 1 : 0) - (status == STG_MAX_ITER ? 1 : 0);
+        launches += (int)((ran + turn_iters - 1) / turn_iters) * launches_per_turn + h_flags[F_REPL] * (use_mas ? 2 : 1);
     }
     if(st)
     {

@@ -186,7 +186,7 @@ struct Solver
     int mas_fem_offset = 0;       // FEM block offset of the last MAS assembly
     long long generation = 0;     // bumped by every (re)assembly
     bool graph_dirty = true;
-    int launches_per_batch = 0;   // kernels in one captured iteration
+    int launches_per_turn = 0, turn_iters = 1;  // kernels and iterations of the captured loop body
     cudaGraph_t pending_if_body = nullptr;
     PcgDev pcg_dev{};             // parameters of the last solve (measurement hook)
     bool pcg_ready = false;

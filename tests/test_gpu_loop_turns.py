@@ -71,3 +71,38 @@ def test_scene_turns_match_single_iterations(dev, count, precision, refine):
         np.testing.assert_array_equal(got[0][4], got[1][4])
         if ratio == 0.3:
             assert got[0][0] == 0 and max(got[0][3]) <= 1e-4
+
+
+@pytest.mark.parametrize("precond", ["mas", "diag"])
+@pytest.mark.parametrize("precision,refine,turn", [("fp64", 32, 8), ("fp32", 32, 8), ("fp32", 12, 4), ("fp32", 3, 1)])
+def test_reported_launches_count_whole_turns(dev, precond, precision, refine, turn):
+    """kernel_launches of the graph loop: the kernels of every started turn, also past the stop,
+    and two (one without MAS) per replacement; in FP64 a full turn is eight iterations of the host loop."""
+    import torch
+    from stgipc import PCGSolverConfig, Solver, scenes
+    s = scenes.make_cube_drop(n=6, seed=4106)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    rows, cols, blocks, b = t(s.rows), t(s.cols), t(s.blocks.reshape(-1)), t(s.b)
+    x = torch.zeros_like(b)
+
+    def launches(iters, loop):
+        v = Solver(PCGSolverConfig(precision=precision, stop_rule="relative_residual", global_tol_rate=1e-12, loop=loop,
+                                   max_iter_ratio=(iters + 1.5) / s.n, refine_interval=refine, preconditioner=precond))
+        if precond == "mas":
+            v.mas_init(s.num_verts, s.neighbor_start, s.neighbor_num, s.neighbor_list, *s.slot_maps(16))
+        v.solve_linear_system(rows, cols, blocks, b, x)  # loads modules, sizes buffers
+        st = v.solve_linear_system(rows, cols, blocks, b, x)
+        v.close()
+        assert st["iterations"] == iters + 1  # the limit: `iters` ran
+        return st["kernel_launches"] - st["replacements"] * (2 if precond == "mas" else 1)
+
+    one = launches(1, "graph")
+    assert launches(turn, "graph") == one
+    per_turn = launches(turn + 1, "graph") - one
+    assert per_turn > 0
+    assert launches(2 * turn, "graph") == one + per_turn
+    assert launches(2 * turn + 1, "graph") == one + 2 * per_turn
+    if precision == "fp64":
+        h1 = launches(1, "host")
+        assert launches(9, "host") - h1 == per_turn
+        assert launches(8, "host") == one
