@@ -759,14 +759,14 @@ def main():
                                       "accepted": st_l["learned_accepted"], "rejected": st_l["learned_rejected"]}
                 ls.close()
 
-    # the BCOO tile autotuner on this system: both FP32 tile shapes timed in the loop's kernel
+    # the BCOO tile autotuner on this system: whole iterations with each candidate
     tuned = make("fp32")
     tuned.spmv_tiles(0)
     solve(tuned)
     rt_t, us_def, us_alt, us_halo, us_up = tuned.spmv_tiles_info()
     tuned.close()
     tiles = {"tuned": {-2: "halo", -3: "upper"}.get(rt_t, f"{rt_t} rows per tile"),
-             "us_per_launch": {"tiled 64x4": us_def, "tiled 32x8": us_alt, "halo 64x4": us_halo, "upper 64x4": us_up}}
+             "us_per_iteration": {"tiled 64x4": us_def, "tiled 32x8": us_alt, "halo 64x4": us_halo, "upper 64x4": us_up}}
 
     # roofline of the dominant kernel: the PCG SpMV of the FP32 path, timed live
     solve(fast)

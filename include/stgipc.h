@@ -382,14 +382,15 @@ int stg_segment_stats(stg_handle h, int* iterations, double* rel_residual);
  * product spilled to the column's row and added there in a fixed order).  0 = autotune: the
  * next solve of a new shape class (precision, block rows, unique blocks) times every
  * candidate (both tile shapes, the upper kernel, and the halo kernel when its windows fit)
- * on that system; the choice is kept for that shape class by every handle of the process.
+ * on that system in whole iterations; the choice is kept for that shape class by every handle
+ * of the process.
  * -1 = the default kernel.  The persistent loop always runs the full-copy SpMV.  Results
  * differ between candidates in the last bits (summation order); a fixed choice keeps solves
  * bitwise reproducible across processes. */
 int stg_spmv_tiles(stg_handle h, int rows_per_tile);
 /* Kernel of the last solve (rows per tile; -2: the halo kernel; -3: the upper kernel), and
- * the autotuner's mean time per launch of each candidate in microseconds (0 when it has not
- * run or the candidate did not fit). */
+ * the autotuner's mean time of an iteration with each candidate in microseconds (0 when it has
+ * not run or the candidate did not fit). */
 int stg_spmv_tiles_info(stg_handle h, int* rows_per_tile, float* us_default, float* us_alternative,
                         float* us_halo, float* us_upper);
 

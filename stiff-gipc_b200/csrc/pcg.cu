@@ -3775,44 +3775,6 @@ static int launch_phase_a(Solver& S, const PcgDev& c, bool dep)
     return launch_dep(S, dep, 1, k_phase_a_tiled<T, a_rt_default<T>()>, grid, A_THREADS, ATile<T>::SMEM, c);
 }
 
-// BCOO tile autotuner: every candidate of the SpMV phase launched on this system (3 untimed,
-// then `reps` timed with CUDA events): the two tile shapes of the tiled kernel and, when its
-// operand windows fit (halo_ok), the halo kernel.  Returns the fastest (its rows per tile, or
-// SPMV_HALO) and each mean.
-template <typename T>
-static int tune_phase_a(Solver& S, PcgDev c, float* us, int* out)
-{
-    const int cand[4] = {a_rt_default<T>(), a_rt_alt<T>(), SPMV_HALO, SPMV_UPPER};
-    float best = 0.f;
-    int pick = cand[0];
-    for(int v = 0; v < 4; v++)
-    {
-        us[v] = 0.f;
-        if((cand[v] == SPMV_HALO && !S.bcoo.halo_ok) || (cand[v] == SPMV_UPPER && !S.bcoo.upper_built)) continue;
-        c.halo = cand[v] == SPMV_HALO ? 1 : 0;
-        c.upper = cand[v] == SPMV_UPPER ? 1 : 0;
-        c.spill = c.upper ? S.pcg.spill.data() : nullptr;
-        c.a_rt = (c.halo || c.upper) ? a_rt_default<T>() : cand[v];
-        STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0));
-        for(int i = 0; i < 3; i++) STG_TRY(launch_phase_a<T>(S, c, false));
-        const int reps = 10;
-        STG_CUDA_TRY(cudaEventRecord(S.ev[4], S.stream));
-        for(int i = 0; i < reps; i++) STG_TRY(launch_phase_a<T>(S, c, false));
-        STG_CUDA_TRY(cudaEventRecord(S.ev[5], S.stream));
-        STG_CUDA_TRY(cudaEventSynchronize(S.ev[5]));
-        float ms = 0.f;
-        STG_CUDA_TRY(cudaEventElapsedTime(&ms, S.ev[4], S.ev[5]));
-        us[v] = 1e3f * ms / reps;
-        if(v == 0 || us[v] < best)
-        {
-            best = us[v];
-            pick = cand[v];
-        }
-    }
-    *out = pick;
-    return 0;
-}
-
 // learned coarse correction after the bank solves: the sample recorder (the level's r and
 // z before any correction), then the network's forward pass and apply on the level's Z
 static int launch_learned(Solver& S, const PcgDev& c)
@@ -3841,6 +3803,13 @@ static int launch_learned(Solver& S, const PcgDev& c)
 // Grids of the phases that run one thread per block row (E also one per ABD dof)
 static int row_grid(int rows) { return std::max(1, std::min(div_up(rows, PB), kSMs * 4)); }
 
+// Phase B's grid: one CTA per PBB slots (MAS) or block rows
+template <int B>
+static int phase_b_grid(const PcgDev& c)
+{
+    return std::max(1, std::min(div_up(B > 0 ? c.M : c.nrows, PBB), kSMs * 8));
+}
+
 // How one iteration handles the residual replacement
 enum ReplMode : int
 {
@@ -3857,7 +3826,7 @@ static int launch_iteration(Solver& S, const PcgDev& c0, int grid_rows, bool dep
     cudaStream_t s = S.stream;
     PcgDev c = c0;
     c.par = par;
-    const int grid_b = std::max(1, std::min(div_up(B > 0 ? c.M : c.nrows, PBB), kSMs * 8));
+    const int grid_b = phase_b_grid<B>(c);
     // phase B's stop test is finished beside the bank solves when they are fused and nothing in
     // between depends on it
     const bool finish = !fused_cd<B>(c) || repl != REPL_NONE;
@@ -3949,26 +3918,12 @@ static int set_carveouts()
     return 0;
 }
 
+// The loop's start: r = b, x = 0, p = 0, b.b; z = M^-1 r, rz = rz0 = r.z (beta = 0 so p_new = z)
 template <typename T, int B>
-static int pcg_run(Solver& S, PcgDev& c)
+static int pcg_init(Solver& S, const PcgDev& c)
 {
-    STG_TRY((set_carveouts<T, B>()));
-    STG_TRY(phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0));
-    c.grid_e = row_grid(std::max(B > 0 ? c.V : c.nrows, 12 * c.abd_bodies));
-    if(c.grid_a > c.slots || c.grid_e > c.slots)
-    {
-        set_error("SpMV phase grid larger than the reduction slots");
-        return STG_ERR_INVALID;
-    }
     cudaStream_t s = S.stream;
-    PcgState& P = S.pcg;
-    const int grid_vec = std::max(1, std::min(div_up(c.n, PB), kSMs * 4));
-    // the SpMV phase runs as exactly one resident wave (grid-stride over the rows)
-    int per_sm_a = 0;
-    STG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_a, k_phase_a<T>, PB, 0));
-    const int grid_rows = std::max(1, std::min(div_up(c.nrows, PB / 16), std::max(per_sm_a, 1) * kSMs));
-    // init: r = b, x = 0, p = 0, b.b; z = M^-1 r, rz = rz0 = r.z (beta = 0 so p_new = z)
-    k_init<T><<<grid_vec, PB, 0, s>>>(c);
+    k_init<T><<<std::max(1, std::min(div_up(c.n, PB), kSMs * 4)), PB, 0, s>>>(c);
     STG_LAUNCH_CHECK();
     S.launches++;
     if(B > 0)
@@ -3989,6 +3944,101 @@ static int pcg_run(Solver& S, PcgDev& c)
         STG_LAUNCH_CHECK();
         S.launches++;
     }
+    return 0;
+}
+
+// the SpMV kernel `pick` (rows per tile, SPMV_HALO or SPMV_UPPER) into the parameter block
+template <typename T>
+static int set_spmv(Solver& S, PcgDev& c, int pick)
+{
+    c.halo = pick == SPMV_HALO && S.bcoo.halo_ok ? 1 : 0;
+    c.upper = pick == SPMV_UPPER && S.bcoo.upper_built ? 1 : 0;
+    c.a_rt = pick > 0 ? pick : a_rt_default<T>();
+    c.spill = c.upper ? S.pcg.spill.data() : nullptr;
+    return phase_a_grid<T>(c.nrows, c.a_rt, &c.grid_a, c.halo != 0, c.upper != 0);
+}
+
+// BCOO tile autotuner, on this system: the two tile shapes of the tiled kernel, the upper kernel
+// and, when its operand windows fit (halo_ok), the halo kernel, each in whole iterations launched
+// as in the loop, 3 untimed and `reps` timed with CUDA events.  Timed by itself, without what its
+// launch overlaps and without the spilled products that phase B adds, the upper kernel came out
+// within 0.5 % of the 64 x 4 tiles on 48 scenes of up to 2,197 rows, where an iteration takes
+// 35.2 us with it and 31.8 with the tiles.  Returns the fastest (its rows per tile, SPMV_HALO or
+// SPMV_UPPER) and each mean.  The caller runs pcg_init again.
+template <typename T, int B>
+static int tune_phase_a(Solver& S, PcgDev c, int grid_rows, float* us, int* out)
+{
+    const int cand[4] = {a_rt_default<T>(), a_rt_alt<T>(), SPMV_HALO, SPMV_UPPER};
+    float best = 0.f;
+    int pick = cand[0];
+    // no replacement, network pass or recorded sample, and no stop
+    c.net_mode = c.flex = 0;
+    c.prm.refine = c.prm.judge = 0;
+    c.prm.tol = 0.0;
+    c.prm.max_iter = 1L << 40;
+    c.seg_tol2 = -1.0;
+    for(int v = 0; v < 4; v++)
+    {
+        us[v] = 0.f;
+        if((cand[v] == SPMV_HALO && !S.bcoo.halo_ok) || (cand[v] == SPMV_UPPER && !S.bcoo.upper_built)) continue;
+        STG_TRY(set_spmv<T>(S, c, cand[v]));
+        STG_TRY((pcg_init<T, B>(S, c)));
+        int done = 0;
+        auto run = [&](int count) -> int {
+            for(int i = 0; i < count; i++, done++)
+                STG_TRY((launch_iteration<T, B>(S, c, grid_rows, i > 0 && !c.halo, REPL_NONE, done & 1)));
+            return 0;
+        };
+        const int reps = 10;
+        STG_TRY(run(3));
+        STG_CUDA_TRY(cudaEventRecord(S.ev[4], S.stream));
+        STG_TRY(run(reps));
+        STG_CUDA_TRY(cudaEventRecord(S.ev[5], S.stream));
+        STG_CUDA_TRY(cudaEventSynchronize(S.ev[5]));
+        float ms = 0.f;
+        STG_CUDA_TRY(cudaEventElapsedTime(&ms, S.ev[4], S.ev[5]));
+        us[v] = 1e3f * ms / reps;
+        // as a solve starts (pcg_init reads the iteration count): iterations past convergence may
+        // have broken down
+        STG_CUDA_TRY(cudaMemsetAsync(c.scal, 0, sizeof(double) * S_COUNT, S.stream));
+        STG_CUDA_TRY(cudaMemsetAsync(c.flags + F_DONE, 0, 2 * sizeof(int), S.stream));
+        STG_CUDA_TRY(cudaMemsetAsync(c.flags + F_STOP, 0, sizeof(int), S.stream));
+        if(v == 0 || us[v] < best)
+        {
+            best = us[v];
+            pick = cand[v];
+        }
+    }
+    *out = pick;
+    return 0;
+}
+
+// pick: the SpMV kernel; tune: time them all first and take the fastest
+template <typename T, int B>
+static int pcg_run(Solver& S, PcgDev& c, int pick, bool tune)
+{
+    STG_TRY((set_carveouts<T, B>()));
+    STG_TRY(set_spmv<T>(S, c, pick));
+    c.grid_e = row_grid(std::max(B > 0 ? c.V : c.nrows, 12 * c.abd_bodies));
+    if(c.grid_a > c.slots || c.grid_e > c.slots)
+    {
+        set_error("SpMV phase grid larger than the reduction slots");
+        return STG_ERR_INVALID;
+    }
+    cudaStream_t s = S.stream;
+    PcgState& P = S.pcg;
+    // the SpMV phase runs as exactly one resident wave (grid-stride over the rows)
+    int per_sm_a = 0;
+    STG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_a, k_phase_a<T>, PB, 0));
+    const int grid_rows = std::max(1, std::min(div_up(c.nrows, PB / 16), std::max(per_sm_a, 1) * kSMs));
+    if(tune)
+    {
+        STG_TRY((tune_phase_a<T, B>(S, c, grid_rows, S.tune_us, &pick)));
+        S.set_tuned(pick, sizeof(T) == 4 ? 1 : 0);
+        record_choice(S.tuned_prec, S.tuned_nrows, S.tuned_nnzb, pick, S.tune_us);
+        STG_TRY(set_spmv<T>(S, c, pick));
+    }
+    STG_TRY((pcg_init<T, B>(S, c)));
 
     const long max_iter = c.prm.max_iter;
     if(max_iter <= 1) return 0;
@@ -4315,40 +4365,25 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     // SpMV kernel: a fixed tile shape (or the halo kernel), the autotuner's choice for this
     // shape class (precision, block rows, unique blocks; one choice per class and process), or
     // the precision's default shape
-    c.a_rt = fp32 ? a_rt_default<float>() : a_rt_default<double>();
-    c.halo = 0;
-    c.upper = 0;
-    if(spmv_rt == SPMV_HALO)
-        c.halo = bcoo.halo_ok ? 1 : 0;
-    else if(spmv_rt > 0)
-        c.a_rt = spmv_rt;
+    int pick = fp32 ? a_rt_default<float>() : a_rt_default<double>();
+    bool tune = false;
+    if(spmv_rt != 0)
+        pick = spmv_rt;
     else if(spmv_tune && cfg.loop_mode != STG_LOOP_PERSISTENT)
     {
-        if(tuned_prec != (fp32 ? 1 : 0) || tuned_nrows != bcoo.nrows || tuned_nnzb != bcoo.nnzb)
+        const int prec = fp32 ? 1 : 0;
+        if(tuned_prec != prec || tuned_nrows != bcoo.nrows || tuned_nnzb != bcoo.nnzb)
         {
             int r = 0;
-            if(!tuned_choice(fp32 ? 1 : 0, bcoo.nrows, bcoo.nnzb, &r, tune_us))
-            {
-                PcgDev t = c;
-                t.grid_e = std::max(1, std::min(div_up(n, PB), kSMs * 4));
-                STG_TRY(fp32 ? tune_phase_a<float>(*this, t, tune_us, &r) : tune_phase_a<double>(*this, t, tune_us, &r));
-                record_choice(fp32 ? 1 : 0, bcoo.nrows, bcoo.nnzb, r, tune_us);
-            }
-            tuned_rt = r;
-            tuned_prec = fp32 ? 1 : 0;
-            tuned_nrows = bcoo.nrows;
-            tuned_nnzb = bcoo.nnzb;
+            if(tuned_choice(prec, bcoo.nrows, bcoo.nnzb, &r, tune_us))
+                set_tuned(r, prec);
+            else
+                tune = true;
         }
-        if(tuned_rt == SPMV_HALO)
-            c.halo = bcoo.halo_ok ? 1 : 0;
-        else if(tuned_rt == SPMV_UPPER)
-            c.upper = bcoo.upper_built ? 1 : 0;
-        else
-            c.a_rt = tuned_rt;
+        if(!tune) pick = tuned_rt;
     }
     else if(upper_spmv_selected(*this))
-        c.upper = bcoo.upper_built ? 1 : 0;
-    c.spill = c.upper ? pcg.spill.data() : nullptr;
+        pick = SPMV_UPPER;
     if(nseg > 0)
     {
         if(seg_off_host.back() != bcoo.nrows || abd_bodies > 0 || cfg.loop_mode == STG_LOOP_PERSISTENT ||
@@ -4416,20 +4451,20 @@ int Solver::pcg_solve(const double* b, double* x, int n, int abd_bodies, const d
     if(fp32)
     {
         if(!use_mas)
-            STG_TRY((pcg_run<float, 0>(*this, c)));
+            STG_TRY((pcg_run<float, 0>(*this, c, pick, tune)));
         else if(cfg.bank_size == 32)
-            STG_TRY((pcg_run<float, 32>(*this, c)));
+            STG_TRY((pcg_run<float, 32>(*this, c, pick, tune)));
         else
-            STG_TRY((pcg_run<float, 16>(*this, c)));
+            STG_TRY((pcg_run<float, 16>(*this, c, pick, tune)));
     }
     else
     {
         if(!use_mas)
-            STG_TRY((pcg_run<double, 0>(*this, c)));
+            STG_TRY((pcg_run<double, 0>(*this, c, pick, tune)));
         else if(cfg.bank_size == 32)
-            STG_TRY((pcg_run<double, 32>(*this, c)));
+            STG_TRY((pcg_run<double, 32>(*this, c, pick, tune)));
         else
-            STG_TRY((pcg_run<double, 16>(*this, c)));
+            STG_TRY((pcg_run<double, 16>(*this, c, pick, tune)));
     }
     pcg_dev = c;
     pcg_ready = true;

@@ -202,6 +202,13 @@ struct Solver
     int spmv_rt = 0;
     bool spmv_tune = false;
     int tuned_rt = 0, tuned_prec = -1, tuned_nrows = -1, tuned_nnzb = -1;
+    void set_tuned(int pick, int prec)
+    {
+        tuned_rt = pick;
+        tuned_prec = prec;
+        tuned_nrows = bcoo.nrows;
+        tuned_nnzb = bcoo.nnzb;
+    }
     float tune_us[4] = {0.f, 0.f, 0.f, 0.f};
     int fail_iter = 0, fail_site = 0;  // stg_selftest_fail_iteration
 

@@ -65,3 +65,40 @@ def test_unsupported_tile_shape_rejected(dev):
     with pytest.raises(StgError):
         solver.spmv_tiles(16)
     solver.spmv_tiles(-1)
+
+
+@pytest.mark.parametrize("prec,precond", [("fp32", "mas"), ("fp64", "mas"), ("fp64", "diag")])
+def test_timing_the_candidates_leaves_no_trace(dev, prec, precond):
+    """The tuner times the candidates on the solve's own vectors: the solve that tunes gives the
+    bits of one with the chosen kernel fixed, also from an x and a handle that are not fresh."""
+    import torch
+    from stgipc import PCGSolverConfig, Solver
+    s = cube_system(9)  # a shape class of its own
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    rows, cols, blocks, b = t(s.rows), t(s.cols), t(s.blocks.reshape(-1)), t(s.b)
+    # one further triplet per case: a class that no other case has tuned
+    k = {"mas": 0, "diag": 1}[precond]
+    v0 = torch.tensor([0], dtype=torch.int32, device=dev)
+    v1 = torch.tensor([s.num_verts - 1 - k], dtype=torch.int32, device=dev)
+    rows, cols = torch.cat([rows, v0]), torch.cat([cols, v1])
+    blocks = torch.cat([blocks, torch.zeros(9, dtype=torch.float64, device=dev)])
+
+    def make(tiles):
+        v = Solver(PCGSolverConfig(precision=prec, stop_rule="relative_residual", global_tol_rate=1e-7,
+                                   preconditioner=precond))
+        if precond == "mas":
+            v.mas_init(s.num_verts, s.neighbor_start, s.neighbor_num, s.neighbor_list, *s.slot_maps(16))
+        v.spmv_tiles(tiles)
+        return v
+
+    tuned = make(-1)
+    x = torch.full_like(b, 3.0)
+    tuned.solve_linear_system(rows, cols, blocks, 2.0 * b, x)
+    tuned.spmv_tiles(0)
+    st = tuned.solve_linear_system(rows, cols, blocks, b, x)
+    info = tuned.spmv_tiles_info()
+    assert info[1] > 0 and info[2] > 0 and info[4] > 0
+    fixed = make(info[0])
+    y = torch.zeros_like(b)
+    st2 = fixed.solve_linear_system(rows, cols, blocks, b, y)
+    assert st["iterations"] == st2["iterations"] and torch.equal(x, y)
