@@ -69,31 +69,44 @@ def test_stacked_cubes_pushed_together(dev):
         assert d2 > 0
 
 
-@pytest.mark.parametrize("P", [1, 31, 33, 129, 6000])
-@pytest.mark.parametrize("speed", [0.05, 3.0])
-def test_bound_without_per_pair_times(dev, P, speed):
+@pytest.mark.parametrize("P,seed,speed", [(1, 900, 3.0), (31, 902, 0.4), (31, 903, 3.0), (33, 900, 0.4), (33, 901, 3.0),
+                                          (129, 902, 0.05), (129, 900, 3.0), (6000, 902, 0.4), (6000, 900, 3.0)])
+def test_bound_without_per_pair_times(dev, P, seed, speed):
     """The bound alone stops pairs that cannot lower it: it equals the bound of the full run and
     the oracle's, bit for bit, with degenerate pairs (a zero-length edge, a flat triangle, a
-    pair at rest) among them."""
+    pair at rest) among them.  The pair that sets it, below one, stands once where it fell and
+    once last, in a warp that is not full."""
     from oracle import oracle as orc
     from stgipc import ccd
-    rng = np.random.default_rng(900 + P)
+    rng = np.random.default_rng(seed + P)
     V = 4 * P
     x = rng.normal(size=(V, 3))
     dx = rng.normal(size=(V, 3)) * speed
     v = rng.permutation(V).reshape(P, 4)
     pairs = np.where((np.arange(P) % 2 == 0)[:, None], np.stack([-v[:, 0] - 1, v[:, 1], v[:, 2], v[:, 3]], 1), v).astype(np.int32)
+    if P == 1:  # a point on its way through a triangle
+        x[v[0]] = [[0.1, 0.5, 0.2], [-1.0, 0.0, -1.0], [1.0, 0.1, -1.0], [0.0, -0.1, 1.0]]
+        dx[v[0]] = [[0.0, -0.9, 0.1], [0.0, 0.1, 0.0], [0.1, 0.0, 0.0], [0.0, 0.2, 0.0]]
     for k in range(5, P, 17):
         x[v[k, 3]] = 0.5 * (x[v[k, 1]] + x[v[k, 2]])  # collinear triangle / nearby edge
     for k in range(7, P, 19):
         dx[v[k]] = 0.0
-    a0 = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev))
-    a1, _ = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev), per_pair=True)
+    toc = np.array([orc.accd(0 if q[0] < 0 else 1, x[np.abs(q + (q < 0))], dx[np.abs(q + (q < 0))], 0.2) for q in pairs])
+    ok = np.isfinite(toc)
+    if not ok.all():
+        # the time of a pair that is flat to the last bit is no number: then the bound is none
+        for per_pair in (False, True):
+            a = ccd.step_size(_t(pairs, dev), _t(x, dev), _t(dx, dev), per_pair=per_pair)
+            assert np.isnan(float((a[0] if per_pair else a).item()))
+        pairs, toc = pairs[ok], toc[ok]
     want = orc.ccd_step_size(pairs, x, dx, 0.8)
-    # a degenerate pair's time may be no number: the bound then is none either, in both modes
-    np.testing.assert_array_equal(float(a0.item()), float(a1.item()))
-    if np.isfinite(float(a1.item())):
-        assert float(a0.item()) == want
+    assert want < 1.0 and want == 1.0 / (1.0 / toc).max()
+    k = np.argmin(toc)
+    last = np.concatenate([np.delete(pairs, k, 0), pairs[[k]]])
+    for p in (pairs, last):
+        a0 = ccd.step_size(_t(p, dev), _t(x, dev), _t(dx, dev))
+        a1, _ = ccd.step_size(_t(p, dev), _t(x, dev), _t(dx, dev), per_pair=True)
+        assert float(a0.item()) == want and float(a1.item()) == want
 
 
 @pytest.mark.parametrize("P", [33, 6000])
