@@ -2,7 +2,8 @@
 restriction and the stop test in one launch.  The host loop runs the same phases one iteration
 at a time (and, with residual replacement, finishes the stop test in phase B): same sums in the
 same order, so both loops must give the same bits for any iteration count (a turn's middle and
-end), replacement interval (turns of 8, 4, 2 and 1 iterations) and level count (2 to 5 levels)."""
+end), replacement interval (turns of 8, 4, 2 and 1 iterations) and level count (2 to 6 levels), as must
+the separate launches of restriction, bank solves and stop test that the fused one replaces."""
 import numpy as np
 import pytest
 
@@ -106,3 +107,39 @@ def test_reported_launches_count_whole_turns(dev, precond, precision, refine, tu
         h1 = launches(1, "host")
         assert launches(9, "host") - h1 == per_turn
         assert launches(8, "host") == one
+
+
+@pytest.mark.parametrize("n,bank,levels", [(6, 16, 4), (16, 16, 5), (40, 16, 6), (6, 32, 3), (16, 32, 4), (40, 32, 5)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_separate_launches_match_the_fused_one(dev, n, bank, levels, precision):
+    """Recording samples for the learned correction takes the separate launches (restriction of
+    level 2, of the levels above, bank solves, stop test in phase B), which very large systems and
+    many scenes take too: the same bits as the fused launch, in both loops, for up to six levels
+    of 16-vertex banks and five of 32-vertex ones."""
+    import torch
+    from stgipc import PCGSolverConfig, Solver, fem, scenes
+    st = scenes.make_heterogeneous_cube(n=n, seed=4500 + n, state_only=True)
+    V = st["pos"].shape[0]
+    nb = scenes.vert_neighbors(V, st["tets"])
+    maps = scenes.mas_partition_morton(V, bank)
+    rows, cols, blocks, b = fem.newton_system(st["pos_rest"], st["pos"], st["vel"], st["tets"], st["E"], st["nu"], st["rho"],
+                                              st["dt"], st["barriers"], device=dev)
+    samples = torch.zeros(2, 4 * V, dtype=torch.float32, device=dev)
+    for iters in (2, 17):
+        got = []
+        for loop, record in (("graph", False), ("host", False), ("graph", True), ("host", True)):
+            v = Solver(PCGSolverConfig(precision=precision, stop_rule="relative_residual", global_tol_rate=1e-12, loop=loop,
+                                       max_iter_ratio=(iters + 0.5) / (3 * V), bank_size=bank))
+            v.mas_init(V, *nb, *maps)
+            if record:
+                v.net_configure(1)
+                v.net_record(samples[0], samples[1], 1, 1000)
+            x = torch.zeros_like(b)
+            stats = v.solve_linear_system(rows, cols, blocks.reshape(-1), b, x)
+            assert v.mas_info()[0] == levels
+            assert (v.net_recorded() == 1) == record
+            got.append((stats["iterations"], stats["rz_final"], stats["rel_residual_recursive"], x))
+            v.close()
+        for g in got[1:]:
+            assert g[:3] == got[0][:3]
+            assert torch.equal(g[3], got[0][3])
