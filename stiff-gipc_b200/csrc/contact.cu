@@ -13,7 +13,7 @@
 // and the Hessian the rank-one E''(s) ds/dx ds/dx^T (GIPC.cu:3187-3403: PFPx's last column is
 // ds/dx), with E''(s) evaluated at s^2 = 1e-6 below that (the reference's gassThreshold,
 // GIPC.cu:3171); E'' >= 0 on s < 1, so the Hessian is positive semi-definite as it stands.
-// ds/dx is the forward-mode derivative of the distance formula.  The mollified near-parallel
+// ds/dx is the forward derivative of the distance formula.  The mollified near-parallel
 // edge-edge encodings (x >= 0 with w < 0; x < 0 with y < 0 and z < 0 or w < 0) are not
 // produced here: such a pair gets zero blocks and counts in *skipped.
 //
@@ -25,100 +25,31 @@
 namespace stg
 {
 
-// a value with its derivatives with respect to the 12 coordinates of the pair
-struct Dual12
+__device__ __forceinline__ void v_cross(const double* a, const double* b, double* r)
 {
-    double v;
-    double g[12];
-};
-
-__device__ __forceinline__ Dual12 dconst(double v)
-{
-    Dual12 r;
-    r.v = v;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = 0.0;
-    return r;
+    r[0] = a[1] * b[2] - a[2] * b[1];
+    r[1] = a[2] * b[0] - a[0] * b[2];
+    r[2] = a[0] * b[1] - a[1] * b[0];
 }
-__device__ __forceinline__ Dual12 dvar(double v, int k)
-{
-    Dual12 r = dconst(v);
-    r.g[k] = 1.0;
-    return r;
-}
-__device__ __forceinline__ Dual12 operator+(const Dual12& a, const Dual12& b)
-{
-    Dual12 r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = a.g[k] + b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual12 operator-(const Dual12& a, const Dual12& b)
-{
-    Dual12 r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = a.g[k] - b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual12 operator*(const Dual12& a, const Dual12& b)
-{
-    Dual12 r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = a.g[k] * b.v + a.v * b.g[k];
-    return r;
-}
-__device__ __forceinline__ Dual12 operator/(const Dual12& a, const Dual12& b)
-{
-    Dual12 r;
-    r.v = a.v / b.v;
-    const double ib = 1.0 / b.v;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = (a.g[k] - r.v * b.g[k]) * ib;
-    return r;
-}
-__device__ __forceinline__ Dual12 dsqrt(const Dual12& a)
-{
-    Dual12 r;
-    r.v = sqrt(a.v);
-    const double h = r.v > 0.0 ? 0.5 / r.v : 0.0;
-#pragma unroll
-    for(int k = 0; k < 12; k++) r.g[k] = a.g[k] * h;
-    return r;
-}
-
-struct DVec
-{
-    Dual12 x, y, z;
-};
-__device__ __forceinline__ DVec dsub(const DVec& a, const DVec& b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ Dual12 ddot(const DVec& a, const DVec& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ DVec dcross(const DVec& a, const DVec& b)
-{
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
+__device__ __forceinline__ double v_dot(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
 // squared distance of the pair's type (_d_PP / _d_PE / _d_PT / _d_EE, mlbvh.cu:229-257)
-__device__ Dual12 squared_distance(int type, const DVec* v)
+__device__ __forceinline__ double squared_distance(int type, const double (&x)[4][3])
 {
-    if(type == 0) return ddot(dsub(v[0], v[1]), dsub(v[0], v[1]));
-    if(type == 1)
+    // type 0: u; 1: |u x v|^2 / |w|^2; 2 and 3: (w . (u x v))^2 / |u x v|^2
+    double u[3], v[3], w[3], n[3];
+#pragma unroll
+    for(int k = 0; k < 3; k++)
     {
-        const DVec c = dcross(dsub(v[1], v[0]), dsub(v[2], v[0]));
-        const DVec e = dsub(v[2], v[1]);
-        return ddot(c, c) / ddot(e, e);
+        u[k] = type == 0 ? x[0][k] - x[1][k] : (type == 2 ? x[2][k] - x[1][k] : x[1][k] - x[0][k]);
+        v[k] = type == 1 ? x[2][k] - x[0][k] : (type == 2 ? x[3][k] - x[1][k] : x[3][k] - x[2][k]);
+        w[k] = type == 1 ? x[2][k] - x[1][k] : (type == 2 ? x[0][k] - x[1][k] : x[2][k] - x[0][k]);
     }
-    if(type == 2)
-    {
-        const DVec b = dcross(dsub(v[2], v[1]), dsub(v[3], v[1]));
-        const Dual12 a = ddot(dsub(v[0], v[1]), b);
-        return a * a / ddot(b, b);
-    }
-    const DVec b = dcross(dsub(v[1], v[0]), dsub(v[3], v[2]));
-    const Dual12 a = ddot(dsub(v[2], v[0]), b);
-    return a * a / ddot(b, b);
+    if(type == 0) return v_dot(u, u);
+    v_cross(u, v, n);
+    if(type == 1) return v_dot(n, n) / v_dot(w, w);
+    const double a = v_dot(w, n);
+    return a * a / v_dot(n, n);
 }
 
 // E'(s) and E''(s) of kappa dHat^2 (s^2 - 1)^2 ln^2(s^2) (RANK 2, GIPC.cu:3226-3230, 3285-3303)
@@ -137,13 +68,6 @@ __device__ __forceinline__ void barrier_derivs(double s, double dhat, double kap
 // +-1) times a unit vector e_k, so of n = u x v only the two components beside k change.  Every
 // term and sum is the one that differentiating with all 12 partials forms, in its order, with
 // p2 for the derivative of a square (x' x + x x').
-__device__ __forceinline__ void v_cross(const double* a, const double* b, double* r)
-{
-    r[0] = a[1] * b[2] - a[2] * b[1];
-    r[1] = a[2] * b[0] - a[0] * b[2];
-    r[2] = a[0] * b[1] - a[1] * b[0];
-}
-__device__ __forceinline__ double v_dot(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 __device__ __forceinline__ double p2(double dx, double x) { return fma(dx, x, dx * x); }
 
 // derivative of the components k + 1 and k + 2 of u x v
@@ -379,13 +303,12 @@ __global__ void k_contact_energy(int ncp, const int4* __restrict__ pairs, const 
     double e = 0.0;
     if(ok)
     {
-        DVec v[4];
+        double v[4][3];
+#pragma unroll
         for(int i = 0; i < 4; i++)
-        {
-            const int g = vid[i < cnt ? i : 0];
-            v[i] = {dconst(x[3 * (size_t)g]), dconst(x[3 * (size_t)g + 1]), dconst(x[3 * (size_t)g + 2])};
-        }
-        const double I = squared_distance(type, v).v / dhat;
+#pragma unroll
+            for(int k = 0; k < 3; k++) v[i][k] = x[3 * (size_t)vid[i < cnt ? i : 0] + k];
+        const double I = squared_distance(type, v) / dhat;
         if(I < 1.0)
         {
             const double l = log(I);
