@@ -64,7 +64,8 @@ typedef struct stg_config
     double max_iter_ratio;  /* PCGSolverConfig::max_iter_ratio (0.3): max_iter = ratio*n */
     int refine_interval;    /* FP32 mode: recompute r = b - A x in FP64 every k iters    */
     int loop_mode;          /* STG_LOOP_HOST / STG_LOOP_GRAPH / STG_LOOP_PERSISTENT      */
-    int graph_batch;        /* iterations per captured graph launch (STG_LOOP_GRAPH)     */
+    int graph_batch;        /* not read: a turn of the captured loop (STG_LOOP_GRAPH) holds 8
+                               iterations, or fewer so as to divide refine_interval     */
     int learned;            /* 1: apply the learned coarse correction (stg_net_*) inside a
                                flexible PCG, MAS only, host or graph loop; 0: off        */
     void* stream;           /* cudaStream_t (NULL = legacy default stream)               */

@@ -1,4 +1,4 @@
-// common.cu -- error state and the single-CTA exclusive scan used by the build stages.
+// common.cu -- error state and the exclusive scan used by the build stages.
 #include "common.cuh"
 
 #include <cooperative_groups.h>

@@ -250,7 +250,7 @@ class Solver:
 
     def spmv_tiles_info(self):
         """(rows per tile of the last solve (-2: halo kernel, -3: upper kernel), tuner us per
-        launch: default shape, alternative shape, halo kernel, upper kernel)."""
+        iteration: default shape, alternative shape, halo kernel, upper kernel)."""
         rt, a, b, h, u = C.c_int(), C.c_float(), C.c_float(), C.c_float(), C.c_float()
         check(_L.lib().stg_spmv_tiles_info(self.h, C.byref(rt), C.byref(a), C.byref(b), C.byref(h), C.byref(u)),
               "stg_spmv_tiles_info")

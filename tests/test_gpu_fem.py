@@ -54,8 +54,7 @@ def test_gpu_built_system_solves_like_cpu_built(dev):
 def test_closed_form_projection_on_hard_tets(dev, T):
     """The closed-form PSD projection against numpy's eigh, per tet: strongly compressed,
     inverted, flattened, collapsed and rank-one deformations, a negative modulus, warps that are
-    not full, and one vertex shared by every tet (more incident tets than the shared-memory sort
-    holds).  Both projections are backward stable, so they agree to a few hundred eps of the
+    not full, and one vertex shared by every tet (more incident tets than are sorted in registers).  Both projections are backward stable, so they agree to a few hundred eps of the
     unprojected Hessian's norm in x (kinetic scale max d^2): 1e-12."""
     from stgipc import fem, scenes
     rng = np.random.default_rng(77 + T)

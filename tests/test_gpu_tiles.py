@@ -1,7 +1,7 @@
 """GPU: the kernels of the in-loop SpMV and their autotuner (stg_spmv_tiles): every tile shape
 of the full-copy kernel, the halo kernel and the upper kernel give the same solve up to
-summation order, the tuner picks the fastest of the timed candidates and keeps it, and
-unsupported shapes are rejected."""
+summation order, the tuner picks the fastest of the timed candidates and keeps it, its timing
+leaves no trace in the solve, and unsupported shapes are rejected."""
 import numpy as np
 import pytest
 
